@@ -15,6 +15,7 @@
 
 #include "../../include/pgm_b200.h"
 #include "pgm_kernels.cuh"
+#include "pgm_fft.cuh"
 
 namespace pgmmp_engine {  // the message-passing model of the learned guess (pgm_mpnn.cu)
 size_t work_bytes(int n);
@@ -90,17 +91,6 @@ std::vector<double> host_moduli(int K, int order) {
   return mod;
 }
 
-// Radices of a length-K FFT (4s first, then 2, 3, 5); empty if K has another factor.
-std::vector<int> radices(int K) {
-  std::vector<int> r;
-  while (K % 4 == 0) { r.push_back(4); K /= 4; }
-  while (K % 2 == 0) { r.push_back(2); K /= 2; }
-  while (K % 3 == 0) { r.push_back(3); K /= 3; }
-  while (K % 5 == 0) { r.push_back(5); K /= 5; }
-  if (K != 1) r.clear();
-  return r;
-}
-
 struct EngineBase {
   virtual ~EngineBase() {
     if (host_scratch) cudaFree(host_scratch);
@@ -144,26 +134,10 @@ struct EngineBase {
   long long generation = 0;  // bumped when device buffers are reallocated (captured graphs go stale)
 };
 
-// Mesh lengths with a compiled FFT plan (others run the runtime-length kernels).
-template <typename F>
-void with_fft_len(int L, F &&f) {
-  switch (L) {
-    case 32: f(std::integral_constant<int, 32>{}); break;
-    case 48: f(std::integral_constant<int, 48>{}); break;
-    case 64: f(std::integral_constant<int, 64>{}); break;
-    case 72: f(std::integral_constant<int, 72>{}); break;
-    case 96: f(std::integral_constant<int, 96>{}); break;
-    case 128: f(std::integral_constant<int, 128>{}); break;
-    case 192: f(std::integral_constant<int, 192>{}); break;
-    default: f(std::integral_constant<int, 0>{}); break;
-  }
-}
-
-// The systems of one FFT pass launch: same mesh length along the pass's axis.
+// The tiles of one FFT pass launch: the systems with the same mesh length along the pass's axis.
 struct FftGroup {
-  int K = 0, ng = 0, ntiles = 0;
-  size_t smem = 0;
-  DBuf<int> sys, tile0;
+  int K = 0;
+  DBuf<pgmfft::Tile> tiles;
 };
 
 // Autotuner choices, shared by the handles of one process with the same precision, spline
@@ -370,9 +344,6 @@ struct Engine : EngineBase {
       rg += (long long)S.K[0] * S.K[1] * S.K[2];
       cg += (long long)S.K[0] * S.K[1] * S.K3h;
       for (int a = 0; a < 3; ++a) {
-        std::vector<int> r = radices(S.K[a]);
-        S.nst[a] = (int)r.size();
-        for (size_t k = 0; k < r.size(); ++k) S.rad[a][k] = r[k];
         S.tw[a] = tw_for(S.K[a]);
         S.mod0[a] = (int)h_bmod.size();
         std::vector<double> mm = host_moduli(S.K[a], P);
@@ -484,69 +455,60 @@ struct Engine : EngineBase {
     nwblk = (int)wbs.size();
     ntblk = (int)tbs.size();
     wb_sys.upload(wbs); wb_atom0.upload(wba); tb_sys.upload(tbs); tb_atom0.upload(tba);
-    // plane passes for the systems whose K2 = K3 mesh has a compiled plan and whose plane (two
-    // regions + the twiddles) fits in a CTA's shared memory; the others run the k3 and k2 passes
+    // plane passes for the systems whose K2 = K3 plane fits in a CTA's shared memory; the others run
+    // the k3 and k2 passes
     int cur_dev = 0, smem_optin = 0;
     CK(cudaGetDevice(&cur_dev));
     CK(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, cur_dev));
     auto plane_ok = [&](const pgm::SysInfo &S) {
-      const int L = S.K[1];
-      if (L != S.K[2] || L > 128 || L % 8 != 0) return false;
-      bool compiled = false;
-      with_fft_len(L, [&](auto Lc) { compiled = decltype(Lc)::value != 0; });
-      return compiled && plane_smem(L) <= (size_t)smem_optin;
+      const size_t b = S.K[1] == S.K[2] && S.K[1] <= pgmfft::PLANE_MAX ? pgmfft::plane_smem(S.K[1], sizeof(T)) : 0;
+      return b > 0 && b <= (size_t)smem_optin;
     };
-    // FFT launch groups per axis: systems with the same mesh length share one launch
-    auto groups = [&](int axis, std::vector<std::unique_ptr<FftGroup>> &out) {
-      std::vector<int> Ks;
-      for (auto &S : hsys)
-        if ((axis == 0 || !plane_ok(S)) && std::find(Ks.begin(), Ks.end(), S.K[axis]) == Ks.end()) Ks.push_back(S.K[axis]);
-      for (int K : Ks) {
-        std::unique_ptr<FftGroup> g(new FftGroup());
-        g->K = K;
-        std::vector<int> gs, gt{0};
-        for (int si = 0; si < n; ++si) {
-          const pgm::SysInfo &S = hsys[si];
-          if (S.K[axis] != K || (axis != 0 && plane_ok(S))) continue;
-          int tiles = axis == 2 ? (S.K[0] * S.K[1] + 2 * pgm::FFT_PAIRS - 1) / (2 * pgm::FFT_PAIRS)
-                    : axis == 1 ? (S.K[0] * S.K3h + pgm::FFT_TILE - 1) / pgm::FFT_TILE
-                                : (S.K[1] * S.K3h + pgm::FFT_TILE - 1) / pgm::FFT_TILE;
-          gs.push_back(si);
-          gt.push_back(gt.back() + tiles);
+    // FFT launches per pass: systems with the same mesh length along its axis share one
+    auto groups = [&](int axis, bool planes, std::vector<std::unique_ptr<FftGroup>> &out) {
+      std::map<int, std::vector<pgmfft::Tile>> by;
+      const int tc = pgmfft::tile_width<T>();
+      for (int si = 0; si < n; ++si) {
+        const pgm::SysInfo &S = hsys[si];
+        if (axis != 0 && planes != plane_ok(S)) continue;
+        std::vector<pgmfft::Tile> &v = by[S.K[axis]];
+        pgmfft::Tile t{};
+        t.s = si; t.K3h = S.K3h; t.K2 = S.K[1]; t.K3 = S.K[2]; t.tw = S.tw[axis]; t.rg = S.rgrid0; t.cg = S.cgrid0;
+        if (planes) {
+          for (int k1 = 0; k1 < S.K[0]; ++k1) {
+            t.rg = S.rgrid0 + (long long)k1 * S.K[1] * S.K[2];
+            t.cg = S.cgrid0 + (long long)k1 * S.K[1] * S.K3h;
+            v.push_back(t);
+          }
+        } else if (axis == 2) {
+          const int lines = S.K[0] * S.K[1];
+          for (t.c0 = 0; t.c0 < lines; t.c0 += 2 * tc) {
+            t.n = std::min(tc, (lines - t.c0) / 2);
+            v.push_back(t);
+          }
+        } else {
+          t.n = (axis == 1 ? S.K[0] : S.K[1]) * S.K3h;
+          const int tiles = (t.n + tc - 1) / tc;
+          const long long nq = (long long)S.K[0] * S.K[1] * S.K[2], per = (nq / 4 + tiles - 1) / tiles * 4;
+          for (int k = 0; k < tiles; ++k) {
+            t.c0 = k * tc;
+            t.q0 = std::min(nq, k * per);
+            t.q1 = std::min(nq, (k + 1) * per);
+            v.push_back(t);
+          }
         }
-        g->ng = (int)gs.size();
-        g->ntiles = gt.back();
-        g->smem = (axis == 2 ? (size_t)2 * pgm::FFT_PAIRS * K : (size_t)2 * pgm::FFT_TILE * (K + 1)) * sizeof(pgm::c2<T>) +
-                  (size_t)K * sizeof(pgm::c2<T>);  // + the twiddle table
-        g->sys.upload(gs);
-        g->tile0.upload(gt);
+      }
+      for (auto &kv : by) {
+        std::unique_ptr<FftGroup> g(new FftGroup());
+        g->K = kv.first;
+        g->tiles.upload(kv.second);
         out.push_back(std::move(g));
       }
     };
-    groups(2, gx);
-    groups(1, gy);
-    groups(0, gz);
-    {
-      std::vector<int> Ls;
-      for (auto &S : hsys)
-        if (plane_ok(S) && std::find(Ls.begin(), Ls.end(), S.K[1]) == Ls.end()) Ls.push_back(S.K[1]);
-      for (int L : Ls) {
-        std::unique_ptr<FftGroup> g(new FftGroup());
-        g->K = L;
-        std::vector<int> gs, gt{0};
-        for (int si = 0; si < n; ++si) {
-          if (!plane_ok(hsys[si]) || hsys[si].K[1] != L) continue;
-          gs.push_back(si);
-          gt.push_back(gt.back() + hsys[si].K[0]);  // one CTA per k1 plane
-        }
-        g->ng = (int)gs.size();
-        g->ntiles = gt.back();
-        g->smem = plane_smem(L);
-        g->sys.upload(gs);
-        g->tile0.upload(gt);
-        gp.push_back(std::move(g));
-      }
-    }
+    groups(2, false, gx);
+    groups(1, false, gy);
+    groups(0, false, gz);
+    groups(2, true, gp);
     d_sys.upload(hsys);
     d_box.alloc(n);
     CK(cudaMemset(d_box.p, 0, sizeof(pgm::BoxInfo) * n));
@@ -642,7 +604,10 @@ struct Engine : EngineBase {
     CK(cudaStreamCreateWithPriority(&nn_st, cudaStreamNonBlocking, prio_hi));
     CK(cudaEventCreateWithFlags(&ev_nn_fork, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&ev_nn_join, cudaEventDisableTiming));
-    set_smem();
+    for (auto &g : gp) {
+      CK(pgmfft::prepare<T>(pgmfft::PLANE_FWD, g->K));
+      CK(pgmfft::prepare<T>(pgmfft::PLANE_INV, g->K));
+    }
   }
 
   void alloc_rows() {
@@ -651,95 +616,26 @@ struct Engine : EngineBase {
     rk.alloc(m); rx.alloc(m); ry.alloc(m); rz.alloc(m); rg0.alloc(m); rg1.alloc(m); rg2.alloc(m); rg3.alloc(m);
   }
 
-  static size_t plane_smem(int L) { return (size_t)(2 * pgm::plane_region(L) + L) * sizeof(pgm::c2<T>); }
-
-  // Plane-pass lengths: the compiled plans up to 128 (a 192 plane does not fit in shared memory).
-  template <typename F>
-  static void with_plane_len(int L, F &&f) {
-    with_fft_len(L, [&](auto Lc) {
-      constexpr int Lv = decltype(Lc)::value;
-      if constexpr (Lv > 0 && Lv <= 128) f(Lc);
-    });
-  }
-
-  template <typename K>
-  void smem_attr(K kern, size_t bytes) {
-    if (bytes > 48 * 1024) CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  }
-
-  void set_smem() {
-    for (auto &g : gp)
-      with_plane_len(g->K, [&](auto Lc) {
-        constexpr int L = decltype(Lc)::value;
-        smem_attr(pgm::k_fft_plane_fwd<T, L>, g->smem);
-        smem_attr(pgm::k_fft_plane_inv<T, L>, g->smem);
-      });
-    for (auto &g : gx)
-      with_fft_len(g->K, [&](auto Lc) {
-        constexpr int L = decltype(Lc)::value;
-        smem_attr(pgm::k_fft_x_fwd<T, L>, g->smem);
-        smem_attr(pgm::k_fft_x_inv<T, L>, g->smem);
-      });
-    for (auto &g : gy)
-      with_fft_len(g->K, [&](auto Lc) {
-        constexpr int L = decltype(Lc)::value;
-        smem_attr(pgm::k_fft_y<T, L>, g->smem);
-      });
-    for (auto &g : gz)
-      with_fft_len(g->K, [&](auto Lc) {
-        constexpr int L = decltype(Lc)::value;
-        smem_attr(pgm::k_fft_z_conv<T, L, false>, g->smem);
-        smem_attr(pgm::k_fft_z_conv<T, L, true>, g->smem);
-      });
-  }
-
-  // The forward plane passes (k3 + k2 per k1 plane) of the systems that have them.
-  void plane_fwd(cudaStream_t st, pgm::Dev<T> &a, int act) {
-    for (auto &g : gp)
-      with_plane_len(g->K, [&](auto Lc) {
-        launch_pdl(pgm::k_fft_plane_fwd<T, decltype(Lc)::value>, g->ntiles, pgm::PLANE_THREADS, g->smem, st, a,
-                   (const int *)g->sys.p, (const int *)g->tile0.p, g->ng, act);
-      });
+  // One pass of the FFTs over its groups of systems.
+  void fft_pass(cudaStream_t st, const pgm::Dev<T> &a, pgmfft::Pass p, std::vector<std::unique_ptr<FftGroup>> &groups, int act,
+                int sign = 0) {
+    const pgmfft::Args<T> f{a.Q, a.Phi, a.Ginf, a.C, a.tw, a.cg, a.box, a.eacc, a.beta};
+    for (auto &g : groups) {
+      CK(pgmfft::launch<T>(p, g->K, f, g->tiles.p, (int)g->tiles.n, act, sign, st, true));
+      ++launches;
+    }
   }
 
   // The passes of one reciprocal-space convolution: r2c (k3) and k2 -- one plane pass where the
   // mesh has it --, k1 with G, k2 and c2r (k3).
   void fft_chain(cudaStream_t st, pgm::Dev<T> &a, int act, bool energy) {
-    plane_fwd(st, a, act);
-    for (auto &g : gx)
-      with_fft_len(g->K, [&](auto Lc) {
-        launch_pdl(pgm::k_fft_x_fwd<T, decltype(Lc)::value>, g->ntiles, pgm::FFT_THREADS, g->smem, st, a, (const int *)g->sys.p,
-                   (const int *)g->tile0.p, g->ng, act);
-      });
-    for (auto &g : gy)
-      with_fft_len(g->K, [&](auto Lc) {
-        launch_pdl(pgm::k_fft_y<T, decltype(Lc)::value>, g->ntiles, pgm::FFT_THREADS, g->smem, st, a, (const int *)g->sys.p,
-                   (const int *)g->tile0.p, g->ng, act, -1);
-      });
-    for (auto &g : gz)
-      with_fft_len(g->K, [&](auto Lc) {
-        if (energy)
-          launch_pdl(pgm::k_fft_z_conv<T, decltype(Lc)::value, true>, g->ntiles, pgm::FFT_THREADS, g->smem, st, a,
-                     (const int *)g->sys.p, (const int *)g->tile0.p, g->ng, act);
-        else
-          launch_pdl(pgm::k_fft_z_conv<T, decltype(Lc)::value, false>, g->ntiles, pgm::FFT_THREADS, g->smem, st, a,
-                     (const int *)g->sys.p, (const int *)g->tile0.p, g->ng, act);
-      });
-    for (auto &g : gy)
-      with_fft_len(g->K, [&](auto Lc) {
-        launch_pdl(pgm::k_fft_y<T, decltype(Lc)::value>, g->ntiles, pgm::FFT_THREADS, g->smem, st, a, (const int *)g->sys.p,
-                   (const int *)g->tile0.p, g->ng, act, +1);
-      });
-    for (auto &g : gx)
-      with_fft_len(g->K, [&](auto Lc) {
-        launch_pdl(pgm::k_fft_x_inv<T, decltype(Lc)::value>, g->ntiles, pgm::FFT_THREADS, g->smem, st, a, (const int *)g->sys.p,
-                   (const int *)g->tile0.p, g->ng, act);
-      });
-    for (auto &g : gp)
-      with_plane_len(g->K, [&](auto Lc) {
-        launch_pdl(pgm::k_fft_plane_inv<T, decltype(Lc)::value>, g->ntiles, pgm::PLANE_THREADS, g->smem, st, a,
-                   (const int *)g->sys.p, (const int *)g->tile0.p, g->ng, act);
-      });
+    fft_pass(st, a, pgmfft::PLANE_FWD, gp, act);
+    fft_pass(st, a, pgmfft::X_FWD, gx, act);
+    fft_pass(st, a, pgmfft::Y_PASS, gy, act, -1);
+    fft_pass(st, a, energy ? pgmfft::Z_ENERGY : pgmfft::Z_CONV, gz, act);
+    fft_pass(st, a, pgmfft::Y_PASS, gy, act, +1);
+    fft_pass(st, a, pgmfft::X_INV, gx, act);
+    fft_pass(st, a, pgmfft::PLANE_INV, gp, act);
   }
 
   // ---------------------------------------------------------------- autotuner
@@ -998,11 +894,8 @@ struct Engine : EngineBase {
       }
       else if (which == 5 || which == 6) {  // the first FFT pass (plane or k3), after the spread with 6
         if (which == 6) pgm::k_spread<T, P, false, false, 0, SPREAD_LPA><<<nwblk, 8 * SPREAD_LPA, 0, st>>>(a, Pv.p);
-        plane_fwd(st, a, 0);
-        for (auto &g : gx)
-          with_fft_len(g->K, [&](auto Lc) {
-            pgm::k_fft_x_fwd<T, decltype(Lc)::value><<<g->ntiles, pgm::FFT_THREADS, g->smem, st>>>(a, g->sys.p, g->tile0.p, g->ng, 0);
-          });
+        fft_pass(st, a, pgmfft::PLANE_FWD, gp, 0);
+        fft_pass(st, a, pgmfft::X_FWD, gx, 0);
       } else if (which == 7) rowfield<false, 0>(st, a, Pv.p, Fv.p, false);
       else if (which == 8) pgm::k_rowmat<T, P, false, 1, 0, false, false, GATHER_LPA><<<nwblk, 8 * GATHER_LPA, 0, st>>>(a, Pv.p, AP.p);
       else if (which == 9) {  // a whole operator sweep with the row/PME overlap
@@ -1613,7 +1506,7 @@ PgmStatus pgm_create(const PgmSettings *s, const PgmSystemDesc *systems, int n, 
         return fail(PGM_ERR_INVALID, "covalent dipole index out of range");
     for (int a = 0; a < 3; ++a) {
       int K = d.pme_grid[a];
-      if (K < 2 * s->pme_order || K > 256 || K % 2 || radices(K).empty())
+      if (K < 2 * s->pme_order || !pgmfft::supported<float>(K))
         return fail(PGM_ERR_UNSUPPORTED, "PME grid sizes must be even, 2, 3, 5-smooth, >= 2 order and <= 256");
     }
   }

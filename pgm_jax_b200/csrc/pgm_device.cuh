@@ -11,10 +11,6 @@ constexpr double SQRT_PI = 1.7724538509055160273;
 constexpr double PI = 3.14159265358979323846;
 constexpr int WARPS_PER_BLOCK = 8;       // warp-per-atom kernels: 8 atoms per block
 constexpr int THREADS_PER_BLOCK = 256;   // thread-per-atom kernels: 256 atoms per block
-constexpr int MAX_STAGES = 10;           // FFT stages per axis
-constexpr int FFT_TILE = 16;             // lines per CTA in the strided FFT passes
-constexpr int FFT_PAIRS = 8;             // complex lines (= 2x real lines) per CTA in the k3 pass
-constexpr int FFT_THREADS = 256;         // threads per CTA of the FFT passes (<= the passes' launch bounds)
 
 template <typename T> struct Vec4;
 template <> struct Vec4<float> { using type = float4; };
@@ -45,8 +41,6 @@ struct SysInfo {
   int nc[3];            // cell grid
   int cell0;            // offset of the cells
   int tw[3];            // offsets of the twiddle tables of K1, K2, K3
-  int nst[3];           // FFT stages per axis
-  int rad[3][MAX_STAGES];
   int mod0[3];          // offsets of the B-spline moduli of each axis
   double tail_sb;       // 2 sum_k C(6,k) M_k M_(6-k) of the LJ tail (lj.py:87-114)
   double sum_q, sum_q2; // charges

@@ -796,594 +796,6 @@ __global__ void __launch_bounds__(8 * LPA) k_spread(Dev<T> a, const v4<T> *__res
   }
 }
 
-// ------------------------------------------------------------------ FFT (shared memory, Stockham)
-template <typename T>
-__device__ __forceinline__ c2<T> cmul(c2<T> a, c2<T> b) {
-  c2<T> r;
-  r.x = a.x * b.x - a.y * b.y;
-  r.y = a.x * b.y + a.y * b.x;
-  return r;
-}
-
-// Compile-time radix plan of a length-L transform: radix 8 first, then 4, 2, 3, 5 (the runtime
-// plans of the host use 4, 2, 3, 5).
-__host__ __device__ constexpr int fft_nst(int L) {
-  int n = 0;
-  while (L % 8 == 0) { L /= 8; ++n; }
-  while (L % 4 == 0) { L /= 4; ++n; }
-  while (L % 2 == 0) { L /= 2; ++n; }
-  while (L % 3 == 0) { L /= 3; ++n; }
-  while (L % 5 == 0) { L /= 5; ++n; }
-  return n;
-}
-__host__ __device__ constexpr int fft_radix(int L, int st) {
-  int n = 0;
-  while (L % 8 == 0) { if (n == st) return 8; L /= 8; ++n; }
-  while (L % 4 == 0) { if (n == st) return 4; L /= 4; ++n; }
-  while (L % 2 == 0) { if (n == st) return 2; L /= 2; ++n; }
-  while (L % 3 == 0) { if (n == st) return 3; L /= 3; ++n; }
-  while (L % 5 == 0) { if (n == st) return 5; L /= 5; ++n; }
-  return 1;
-}
-
-// R-point DFT in registers, sign -1 forward / +1 inverse: X_k = sum_n v_n w^(n k), w = exp(sign 2 pi i / R).
-template <typename T, int R>
-__device__ __forceinline__ void butterfly(c2<T> *v, T sg) {
-  c2<T> o[R];
-  if constexpr (R == 8) {
-    // two 4-point DFTs of the even and odd points, X_k = E_k + w^k O_k, X_(k+4) = E_k - w^k O_k
-    c2<T> e[4] = {v[0], v[2], v[4], v[6]}, d[4] = {v[1], v[3], v[5], v[7]};
-    butterfly<T, 4>(e, sg);
-    butterfly<T, 4>(d, sg);
-    const T h = T(0.70710678118654752440);
-    c2<T> t[4];
-    t[0] = d[0];
-    t[1].x = h * (d[1].x - sg * d[1].y); t[1].y = h * (d[1].y + sg * d[1].x);
-    t[2].x = -sg * d[2].y; t[2].y = sg * d[2].x;
-    t[3].x = -h * (d[3].x + sg * d[3].y); t[3].y = h * (sg * d[3].x - d[3].y);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      o[k].x = e[k].x + t[k].x; o[k].y = e[k].y + t[k].y;
-      o[k + 4].x = e[k].x - t[k].x; o[k + 4].y = e[k].y - t[k].y;
-    }
-  } else if constexpr (R == 2) {
-    o[0].x = v[0].x + v[1].x; o[0].y = v[0].y + v[1].y;
-    o[1].x = v[0].x - v[1].x; o[1].y = v[0].y - v[1].y;
-  } else if constexpr (R == 4) {
-    c2<T> a0, a1, b0, b1, ib1;
-    a0.x = v[0].x + v[2].x; a0.y = v[0].y + v[2].y;
-    a1.x = v[0].x - v[2].x; a1.y = v[0].y - v[2].y;
-    b0.x = v[1].x + v[3].x; b0.y = v[1].y + v[3].y;
-    b1.x = v[1].x - v[3].x; b1.y = v[1].y - v[3].y;
-    ib1.x = -sg * b1.y; ib1.y = sg * b1.x;  // sign * i * b1
-    o[0].x = a0.x + b0.x; o[0].y = a0.y + b0.y;
-    o[2].x = a0.x - b0.x; o[2].y = a0.y - b0.y;
-    o[1].x = a1.x + ib1.x; o[1].y = a1.y + ib1.y;
-    o[3].x = a1.x - ib1.x; o[3].y = a1.y - ib1.y;
-  } else if constexpr (R == 3) {
-    const T c = T(-0.5), sn = sg * T(0.86602540378443864676);
-    c2<T> t1, t2, m;
-    t1.x = v[1].x + v[2].x; t1.y = v[1].y + v[2].y;
-    t2.x = v[1].x - v[2].x; t2.y = v[1].y - v[2].y;
-    o[0].x = v[0].x + t1.x; o[0].y = v[0].y + t1.y;
-    m.x = v[0].x + c * t1.x; m.y = v[0].y + c * t1.y;
-    o[1].x = m.x - sn * t2.y; o[1].y = m.y + sn * t2.x;
-    o[2].x = m.x + sn * t2.y; o[2].y = m.y - sn * t2.x;
-  } else {
-    static_assert(R == 5, "radix");
-    const T c1 = T(0.30901699437494742410), c2v = T(-0.80901699437494742410);
-    const T s1 = sg * T(0.95105651629515357212), s2 = sg * T(0.58778525229247312917);
-    c2<T> a1, a2, b1, b2, m1, m2, n1, n2;
-    a1.x = v[1].x + v[4].x; a1.y = v[1].y + v[4].y;
-    b1.x = v[1].x - v[4].x; b1.y = v[1].y - v[4].y;
-    a2.x = v[2].x + v[3].x; a2.y = v[2].y + v[3].y;
-    b2.x = v[2].x - v[3].x; b2.y = v[2].y - v[3].y;
-    o[0].x = v[0].x + a1.x + a2.x; o[0].y = v[0].y + a1.y + a2.y;
-    m1.x = v[0].x + c1 * a1.x + c2v * a2.x; m1.y = v[0].y + c1 * a1.y + c2v * a2.y;
-    m2.x = v[0].x + c2v * a1.x + c1 * a2.x; m2.y = v[0].y + c2v * a1.y + c1 * a2.y;
-    n1.x = s1 * b1.x + s2 * b2.x; n1.y = s1 * b1.y + s2 * b2.y;
-    n2.x = s2 * b1.x - s1 * b2.x; n2.y = s2 * b1.y - s1 * b2.y;
-    o[1].x = m1.x - n1.y; o[1].y = m1.y + n1.x;
-    o[4].x = m1.x + n1.y; o[4].y = m1.y - n1.x;
-    o[2].x = m2.x - n2.y; o[2].y = m2.y + n2.x;
-    o[3].x = m2.x + n2.y; o[3].y = m2.y - n2.x;
-  }
-#pragma unroll
-  for (int r = 0; r < R; ++r) v[r] = o[r];
-}
-
-// One Stockham stage (radix R, NS points already combined) of nl lines of length L in shared
-// memory: v_r = x[j + r L/R] w^(r k), k = j mod NS, DFT_R, y[(j / NS) NS R + k + r NS].  LF (lines
-// fastest): consecutive threads take the same j of consecutive lines, for line strides ld that are
-// odd in 8-byte words, where the stride-R writes of the first stage would otherwise hit the same
-// shared-memory banks; otherwise consecutive threads take consecutive j of one line.
-template <typename T, int R, bool LF = false>
-__device__ __forceinline__ void fft_stage(const c2<T> *x, c2<T> *y, int L, int NS, int nl, int ld, const c2<T> *tw, int sign) {
-  const int LR = L / R, stride = L / (NS * R);
-  const T sg = T(sign);
-  for (int w = threadIdx.x; w < LR * nl; w += blockDim.x) {
-    int line, j;
-    if (LF) { j = w / nl; line = w - j * nl; }
-    else { line = w / LR; j = w - line * LR; }
-    int k = j % NS;
-    const c2<T> *in = x + line * ld;
-    c2<T> *out = y + line * ld;
-    c2<T> v[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      c2<T> u = in[j + r * LR];
-      if (r > 0) {
-        c2<T> t = tw[r * k * stride];
-        if (sign > 0) t.y = -t.y;
-        u = cmul<T>(u, t);
-      }
-      v[r] = u;
-    }
-    butterfly<T, R>(v, sg);
-    int dst = (j / NS) * NS * R + k;
-#pragma unroll
-    for (int r = 0; r < R; ++r) out[dst + r * NS] = v[r];
-  }
-  __syncthreads();
-}
-
-// Compile-time length: every index constant folds (L, R, NS template-known).
-template <typename T, int L, int ST, int NS, bool LF = false>
-__device__ __forceinline__ c2<T> *fft_run_ct(c2<T> *x, c2<T> *y, int nl, int ld, const c2<T> *tw, int sign) {
-  if constexpr (ST == fft_nst(L)) {
-    return x;
-  } else {
-    constexpr int R = fft_radix(L, ST);
-    fft_stage<T, R, LF>(x, y, L, NS, nl, ld, tw, sign);
-    return fft_run_ct<T, L, ST + 1, NS * R, LF>(y, x, nl, ld, tw, sign);
-  }
-}
-
-// Runtime length (fallback for meshes without a compiled plan).
-template <typename T>
-__device__ c2<T> *fft_run_rt(c2<T> *x, c2<T> *y, int L, int nl, int ld, const int *rad, int nst, const c2<T> *tw, int sign) {
-  int NS = 1;
-  for (int st = 0; st < nst; ++st) {
-    const int R = rad[st];
-    if (R == 4) fft_stage<T, 4>(x, y, L, NS, nl, ld, tw, sign);
-    else if (R == 2) fft_stage<T, 2>(x, y, L, NS, nl, ld, tw, sign);
-    else if (R == 3) fft_stage<T, 3>(x, y, L, NS, nl, ld, tw, sign);
-    else fft_stage<T, 5>(x, y, L, NS, nl, ld, tw, sign);
-    c2<T> *t = x; x = y; y = t;
-    NS *= R;
-  }
-  return x;
-}
-
-template <typename T, int L, bool LF = false>
-__device__ __forceinline__ c2<T> *fft_lines(c2<T> *x, c2<T> *y, int Lrt, int nl, int ld, const int *rad, int nst, const c2<T> *tw,
-                                            int sign) {
-  if constexpr (L == 0) return fft_run_rt<T>(x, y, Lrt, nl, ld, rad, nst, tw, sign);
-  else return fft_run_ct<T, L, 0, 1, LF>(x, y, nl, ld, tw, sign);
-}
-
-// Global -> shared staging of `total` elements by the FFT_THREADS threads of a pass: with a
-// compile-time bound N every load of a thread is issued before its first store (the passes are
-// latency-bound; one L2 round trip instead of one per element); N = 0: a plain loop.
-template <int N, typename Get, typename Put>
-__device__ __forceinline__ void staged_copy(int total, Get &&get, Put &&put) {
-  if constexpr (N > 0) {
-    constexpr int PER = (N + FFT_THREADS - 1) / FFT_THREADS;
-    using V = decltype(get(0));
-    V v[PER];
-#pragma unroll
-    for (int j = 0; j < PER; ++j) {
-      int t = threadIdx.x + j * FFT_THREADS;
-      if (t < total) v[j] = get(t);
-    }
-#pragma unroll
-    for (int j = 0; j < PER; ++j) {
-      int t = threadIdx.x + j * FFT_THREADS;
-      if (t < total) put(t, v[j]);
-    }
-  } else {
-    for (int t = threadIdx.x; t < total; t += blockDim.x) put(t, get(t));
-  }
-}
-
-template <typename T>
-struct c2pair {
-  c2<T> a, b;
-};
-
-static_assert(FFT_THREADS <= 256, "the FFT passes are compiled for at most 256 threads per CTA");
-
-// A launch of an FFT pass covers a group of systems with the same mesh length along the pass's
-// axis: block -> (group member g, tile) by the tile prefix gtile0 (ng + 1 entries).
-__device__ __forceinline__ int group_member(const int *gtile0, int ng, int b) {
-  int g = 0;
-  while (g + 1 < ng && gtile0[g + 1] <= b) ++g;
-  return g;
-}
-
-template <typename T>
-__device__ __forceinline__ bool pass_active(const Dev<T> &a, int s, int act) {
-  return act == 0 || (act == 1 && a.cg[s].active) || (act == 2 && a.cg[s].sweep2) || (act == 3 && a.cg[s].fallback);
-}
-
-// k3 pass, real -> half complex: two real lines packed as one complex line (z = a + i b), one
-// length-K3 FFT, untangled.
-template <typename T, int L>
-__global__ void __launch_bounds__(256) k_fft_x_fwd(Dev<T> a, const int *gsys, const int *gtile0, int ng, int act) {
-  pdl_enter();
-  extern __shared__ unsigned char smem_raw[];
-  int g = group_member(gtile0, ng, blockIdx.x);
-  int s = gsys[g];
-  if (!pass_active(a, s, act)) return;
-  const SysInfo &S = a.sys[s];
-  const int K3 = L ? L : S.K[2], K3h = K3 / 2 + 1, nlines = S.K[0] * S.K[1];
-  int tile = blockIdx.x - gtile0[g];
-  int l0 = tile * 2 * FFT_PAIRS;  // first real line
-  int np = min(FFT_PAIRS, (nlines - l0) / 2);
-  c2<T> *x = reinterpret_cast<c2<T> *>(smem_raw), *y = x + FFT_PAIRS * K3, *tws = y + FFT_PAIRS * K3;
-  T *Q = a.Q + S.rgrid0 + (size_t)l0 * K3;
-  for (int t = threadIdx.x; t < K3; t += blockDim.x) tws[t] = a.tw[S.tw[2] + t];  // twiddles in shared memory
-  staged_copy<2 * FFT_PAIRS * L>(
-      2 * np * K3, [&](int t) { return Q[t]; },
-      [&](int t, T v) {
-        int rl = t / K3, k = t - rl * K3;
-        reinterpret_cast<T *>(&x[(rl >> 1) * K3 + k])[rl & 1] = v;
-      });
-  __syncthreads();
-  c2<T> *res = fft_lines<T, L>(x, y, K3, np, K3, S.rad[2], S.nst[2], tws, -1);
-  c2<T> *C = a.C + S.cgrid0 + (size_t)l0 * K3h;
-  for (int t = threadIdx.x; t < np * K3h; t += blockDim.x) {
-    int cl = t / K3h, m = t - cl * K3h;
-    c2<T> Z = res[cl * K3 + m], W = res[cl * K3 + (m == 0 ? 0 : K3 - m)];
-    c2<T> A, Bv;
-    A.x = T(0.5) * (Z.x + W.x); A.y = T(0.5) * (Z.y - W.y);
-    T dx = Z.x - W.x, dy = Z.y + W.y;  // (Z - conj W) / (2 i)
-    Bv.x = T(0.5) * dy; Bv.y = -T(0.5) * dx;
-    C[(size_t)(2 * cl) * K3h + m] = A;
-    C[(size_t)(2 * cl + 1) * K3h + m] = Bv;
-  }
-}
-
-// k3 pass, half complex -> real (the inverse of k_fft_x_fwd, unnormalised): writes phi.
-template <typename T, int L>
-__global__ void __launch_bounds__(256) k_fft_x_inv(Dev<T> a, const int *gsys, const int *gtile0, int ng, int act) {
-  pdl_enter();
-  extern __shared__ unsigned char smem_raw[];
-  int g = group_member(gtile0, ng, blockIdx.x);
-  int s = gsys[g];
-  if (!pass_active(a, s, act)) return;
-  const SysInfo &S = a.sys[s];
-  const int K3 = L ? L : S.K[2], K3h = K3 / 2 + 1, nlines = S.K[0] * S.K[1];
-  int tile = blockIdx.x - gtile0[g];
-  int l0 = tile * 2 * FFT_PAIRS;
-  int np = min(FFT_PAIRS, (nlines - l0) / 2);
-  c2<T> *x = reinterpret_cast<c2<T> *>(smem_raw), *y = x + FFT_PAIRS * K3, *tws = y + FFT_PAIRS * K3;
-  const c2<T> *C = a.C + S.cgrid0 + (size_t)l0 * K3h;
-  for (int t = threadIdx.x; t < K3; t += blockDim.x) tws[t] = a.tw[S.tw[2] + t];
-  staged_copy<FFT_PAIRS * L>(
-      np * K3,
-      [&](int t) {
-        int cl = t / K3, m = t - cl * K3;
-        int mm = m > K3 / 2 ? K3 - m : m;
-        return c2pair<T>{C[(size_t)(2 * cl) * K3h + mm], C[(size_t)(2 * cl + 1) * K3h + mm]};
-      },
-      [&](int t, c2pair<T> p) {
-        int cl = t / K3, m = t - cl * K3;
-        bool up = m > K3 / 2;
-        int mm = up ? K3 - m : m;
-        c2<T> A = p.a, Bv = p.b;
-        if (mm == 0 || 2 * mm == K3) { A.y = T(0); Bv.y = T(0); }
-        if (up) { A.y = -A.y; Bv.y = -Bv.y; }
-        c2<T> Z;
-        Z.x = A.x - Bv.y; Z.y = A.y + Bv.x;
-        x[cl * K3 + m] = Z;
-      });
-  __syncthreads();
-  c2<T> *res = fft_lines<T, L>(x, y, K3, np, K3, S.rad[2], S.nst[2], tws, +1);
-  T *Phi = a.Phi + S.rgrid0 + (size_t)l0 * K3;
-  for (int t = threadIdx.x; t < 2 * np * K3; t += blockDim.x) {
-    int rl = t / K3, k = t - rl * K3;
-    c2<T> z = res[(rl >> 1) * K3 + k];
-    Phi[t] = (rl & 1) ? z.y : z.x;
-  }
-}
-
-// k2 pass (both directions): FFT_TILE consecutive columns (k1, m3) of the flattened K1 x K3h
-// column index, each a line over k2 with stride K3h.
-template <typename T, int L>
-__global__ void __launch_bounds__(256) k_fft_y(Dev<T> a, const int *gsys, const int *gtile0, int ng, int act, int sign) {
-  pdl_enter();
-  extern __shared__ unsigned char smem_raw[];
-  int g = group_member(gtile0, ng, blockIdx.x);
-  int s = gsys[g];
-  if (!pass_active(a, s, act)) return;
-  const SysInfo &S = a.sys[s];
-  const int K2 = L ? L : S.K[1], K3h = S.K3h, ncol = S.K[0] * K3h;
-  int c0 = (blockIdx.x - gtile0[g]) * FFT_TILE;
-  const int ld = K2 + 1;
-  c2<T> *x = reinterpret_cast<c2<T> *>(smem_raw), *y = x + FFT_TILE * ld, *tws = y + FFT_TILE * ld;
-  c2<T> *C = a.C + S.cgrid0;
-  for (int t = threadIdx.x; t < K2; t += blockDim.x) tws[t] = a.tw[S.tw[1] + t];
-  staged_copy<L * FFT_TILE>(
-      K2 * FFT_TILE,
-      [&](int t) {
-        int k2 = t / FFT_TILE, c = t - k2 * FFT_TILE;
-        int col = c0 + c;
-        c2<T> v;
-        v.x = T(0); v.y = T(0);
-        if (col < ncol) {
-          int k1 = col / K3h, m3 = col - k1 * K3h;
-          v = C[((size_t)k1 * K2 + k2) * K3h + m3];
-        }
-        return v;
-      },
-      [&](int t, c2<T> v) {
-        int k2 = t / FFT_TILE, c = t - k2 * FFT_TILE;
-        x[c * ld + k2] = v;
-      });
-  __syncthreads();
-  if (sign < 0) {
-    // the real grid of this system was consumed by the k3 pass: clear this CTA's share of it for
-    // the next spread (no separate memset between the sweeps)
-    const size_t nq = (size_t)S.K[0] * S.K[1] * S.K[2];
-    const int ntile = gtile0[g + 1] - gtile0[g];
-    const size_t per = (nq + ntile - 1) / ntile, q0 = (size_t)(blockIdx.x - gtile0[g]) * per;
-    const size_t q1 = q0 + per < nq ? q0 + per : nq;
-    T *Qs = a.Q + S.rgrid0;
-    for (size_t t = q0 + threadIdx.x; t < q1; t += blockDim.x) Qs[t] = T(0);
-  }
-  c2<T> *res = fft_lines<T, L, true>(x, y, K2, FFT_TILE, ld, S.rad[1], S.nst[1], tws, sign);
-  for (int t = threadIdx.x; t < K2 * FFT_TILE; t += blockDim.x) {
-    int k2 = t / FFT_TILE, c = t - k2 * FFT_TILE;
-    int col = c0 + c;
-    if (col < ncol) {
-      int k1 = col / K3h, m3 = col - k1 * K3h;
-      C[((size_t)k1 * K2 + k2) * K3h + m3] = res[c * ld + k2];
-    }
-  }
-}
-
-// ---- plane passes (meshes with K2 = K3 = L): one CTA per k1 plane runs the k3 and k2 passes in
-// shared memory, in two regions of plane_region(L) complex elements each (the L/2 packed k3-lines
-// of the real plane, or the L/2 + 1 k2-columns padded to L + 1).  The same arithmetic as
-// k_fft_x_fwd followed by k_fft_y(-1), and as k_fft_y(+1) followed by k_fft_x_inv, with one grid
-// round trip and one launch instead of two.
-constexpr int PLANE_THREADS = 512;
-__host__ __device__ constexpr int plane_region(int L) { return (L / 2 + 1) * (L + 1); }
-
-template <typename T, int L>
-__global__ void __launch_bounds__(PLANE_THREADS) k_fft_plane_fwd(Dev<T> a, const int *gsys, const int *gtile0, int ng, int act) {
-  static_assert(L > 0 && L % 8 == 0, "compile-time plane length");
-  pdl_enter();
-  extern __shared__ unsigned char smem_raw[];
-  const int g = group_member(gtile0, ng, blockIdx.x);
-  const int s = gsys[g];
-  if (!pass_active(a, s, act)) return;
-  const SysInfo &S = a.sys[s];
-  constexpr int K = L, Kh = L / 2 + 1, NP = L / 2, LD = L + 1, REG = plane_region(L), Q4 = L / 4;
-  const int k1 = blockIdx.x - gtile0[g];
-  c2<T> *A = reinterpret_cast<c2<T> *>(smem_raw), *B = A + REG, *tws = B + REG;
-  for (int t = threadIdx.x; t < K; t += PLANE_THREADS) tws[t] = a.tw[S.tw[2] + t];  // K2 = K3: one table
-  // rows 2cl and 2cl + 1 of the plane (K x K reals, rows k2) packed as complex line cl, four
-  // columns per thread and load; each thread clears what it read (Q is zero for the next spread)
-  using V = v4<T>;
-  V *Qp = reinterpret_cast<V *>(a.Q + S.rgrid0 + (size_t)k1 * K * K);
-  constexpr int NV = NP * Q4, PER = (NV + PLANE_THREADS - 1) / PLANE_THREADS;
-  V lo[PER], hi[PER];
-#pragma unroll
-  for (int j = 0; j < PER; ++j) {
-    const int t = threadIdx.x + j * PLANE_THREADS;
-    if (t < NV) {
-      const int cl = t / Q4, q = t - cl * Q4;
-      lo[j] = Qp[(2 * cl) * Q4 + q];
-      hi[j] = Qp[(2 * cl + 1) * Q4 + q];
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < PER; ++j) {
-    const int t = threadIdx.x + j * PLANE_THREADS;
-    if (t < NV) {
-      const int cl = t / Q4, q = t - cl * Q4;
-      c2<T> *d = A + cl * LD + 4 * q;  // line stride LD: odd in 8-byte words
-      d[0].x = lo[j].x; d[0].y = hi[j].x;
-      d[1].x = lo[j].y; d[1].y = hi[j].y;
-      d[2].x = lo[j].z; d[2].y = hi[j].z;
-      d[3].x = lo[j].w; d[3].y = hi[j].w;
-      V z;
-      z.x = T(0); z.y = T(0); z.z = T(0); z.w = T(0);
-      Qp[(2 * cl) * Q4 + q] = z;
-      Qp[(2 * cl + 1) * Q4 + q] = z;
-    }
-  }
-  __syncthreads();
-  c2<T> *res = fft_lines<T, L, true>(A, B, K, NP, LD, S.rad[2], S.nst[2], tws, -1);
-  c2<T> *col = res == A ? B : A;
-  // untangle line cl into rows 2cl, 2cl + 1 (m3 = 0..K/2), stored as k2-columns
-  for (int t = threadIdx.x; t < NP * Kh; t += PLANE_THREADS) {
-    const int cl = t / Kh, m = t - cl * Kh;
-    const c2<T> Z = res[cl * LD + m], W = res[cl * LD + (m == 0 ? 0 : K - m)];
-    c2<T> X0, X1;
-    X0.x = T(0.5) * (Z.x + W.x); X0.y = T(0.5) * (Z.y - W.y);
-    const T dx = Z.x - W.x, dy = Z.y + W.y;  // (Z - conj W) / (2 i)
-    X1.x = T(0.5) * dy; X1.y = -T(0.5) * dx;
-    col[m * LD + 2 * cl] = X0;
-    col[m * LD + 2 * cl + 1] = X1;
-  }
-  __syncthreads();
-  c2<T> *res2 = fft_lines<T, L, true>(col, res, K, Kh, LD, S.rad[1], S.nst[1], tws, -1);
-  c2<T> *C = a.C + S.cgrid0 + (size_t)k1 * K * Kh;
-  for (int t = threadIdx.x; t < K * Kh; t += PLANE_THREADS) {
-    const int k2 = t / Kh, m3 = t - k2 * Kh;
-    C[t] = res2[m3 * LD + k2];
-  }
-}
-
-template <typename T, int L>
-__global__ void __launch_bounds__(PLANE_THREADS) k_fft_plane_inv(Dev<T> a, const int *gsys, const int *gtile0, int ng, int act) {
-  static_assert(L > 0 && L % 8 == 0, "compile-time plane length");
-  pdl_enter();
-  extern __shared__ unsigned char smem_raw[];
-  const int g = group_member(gtile0, ng, blockIdx.x);
-  const int s = gsys[g];
-  if (!pass_active(a, s, act)) return;
-  const SysInfo &S = a.sys[s];
-  constexpr int K = L, Kh = L / 2 + 1, NP = L / 2, LD = L + 1, REG = plane_region(L), Q4 = L / 4;
-  const int k1 = blockIdx.x - gtile0[g];
-  c2<T> *A = reinterpret_cast<c2<T> *>(smem_raw), *B = A + REG, *tws = B + REG;
-  for (int t = threadIdx.x; t < K; t += PLANE_THREADS) tws[t] = a.tw[S.tw[2] + t];
-  const c2<T> *C = a.C + S.cgrid0 + (size_t)k1 * K * Kh;
-  constexpr int NC = K * Kh, PER = (NC + PLANE_THREADS - 1) / PLANE_THREADS;
-  c2<T> v[PER];
-#pragma unroll
-  for (int j = 0; j < PER; ++j) {
-    const int t = threadIdx.x + j * PLANE_THREADS;
-    if (t < NC) v[j] = C[t];
-  }
-#pragma unroll
-  for (int j = 0; j < PER; ++j) {
-    const int t = threadIdx.x + j * PLANE_THREADS;
-    if (t < NC) {
-      const int k2 = t / Kh, m3 = t - k2 * Kh;
-      A[m3 * LD + k2] = v[j];
-    }
-  }
-  __syncthreads();
-  c2<T> *res = fft_lines<T, L, true>(A, B, K, Kh, LD, S.rad[1], S.nst[1], tws, +1);
-  c2<T> *lin = res == A ? B : A;
-  // rows 2cl, 2cl + 1 back into complex line cl (z = a + i b) over the full k3 range (Hermitian)
-  for (int t = threadIdx.x; t < NP * K; t += PLANE_THREADS) {
-    const int cl = t / K, m = t - cl * K;
-    const bool up = m > K / 2;
-    const int mm = up ? K - m : m;
-    c2<T> X0 = res[mm * LD + 2 * cl], X1 = res[mm * LD + 2 * cl + 1];
-    if (mm == 0 || 2 * mm == K) { X0.y = T(0); X1.y = T(0); }
-    if (up) { X0.y = -X0.y; X1.y = -X1.y; }
-    c2<T> Z;
-    Z.x = X0.x - X1.y; Z.y = X0.y + X1.x;
-    lin[cl * LD + m] = Z;  // line stride LD: odd in 8-byte words
-  }
-  __syncthreads();
-  c2<T> *res2 = fft_lines<T, L, true>(lin, res, K, NP, LD, S.rad[2], S.nst[2], tws, +1);
-  using V = v4<T>;
-  V *Pp = reinterpret_cast<V *>(a.Phi + S.rgrid0 + (size_t)k1 * K * K);
-  for (int t = threadIdx.x; t < NP * Q4; t += PLANE_THREADS) {
-    const int cl = t / Q4, q = t - cl * Q4;
-    const c2<T> *z = res2 + cl * LD + 4 * q;
-    V r0, r1;
-    r0.x = z[0].x; r0.y = z[1].x; r0.z = z[2].x; r0.w = z[3].x;
-    r1.x = z[0].y; r1.y = z[1].y; r1.z = z[2].y; r1.w = z[3].y;
-    Pp[(2 * cl) * Q4 + q] = r0;
-    Pp[(2 * cl + 1) * Q4 + q] = r1;
-  }
-}
-
-// k1 pass with the convolution: FFT_TILE consecutive columns c = k2 K3h + m3 (contiguous in
-// memory), forward FFT along k1, multiply by 2 G(m) (phi = dE/dQ = 2 K^3 irfft(G F[Q]),
-// pme.py:370-376), inverse FFT.  With ENERGY the reciprocal energy sum w3 G |F|^2
-// (pme.py:390-411) and the influence part of the virial are accumulated.
-template <typename T, int L, bool ENERGY>
-__global__ void __launch_bounds__(256) k_fft_z_conv(Dev<T> a, const int *gsys, const int *gtile0, int ng, int act) {
-  pdl_enter();
-  extern __shared__ unsigned char smem_raw[];
-  __shared__ double red[7][8];
-  int g = group_member(gtile0, ng, blockIdx.x);
-  int s = gsys[g];
-  if (!pass_active(a, s, act)) return;
-  const SysInfo &S = a.sys[s];
-  const int K1 = L ? L : S.K[0], K2 = S.K[1], K3 = S.K[2], K3h = S.K3h, ncol = K2 * K3h;
-  int c0 = (blockIdx.x - gtile0[g]) * FFT_TILE;
-  const int ld = K1 + 1;
-  c2<T> *x = reinterpret_cast<c2<T> *>(smem_raw), *y = x + FFT_TILE * ld, *tws = y + FFT_TILE * ld;
-  c2<T> *C = a.C + S.cgrid0;
-  const size_t rs = (size_t)ncol;
-  for (int t = threadIdx.x; t < K1; t += blockDim.x) tws[t] = a.tw[S.tw[0] + t];
-  const T *G = a.Ginf + S.cgrid0;
-  // the influence values of this tile are staged beside the grid columns (their loads in flight
-  // with the grid's); y holds them until the first transform overwrites it
-  T *gst = reinterpret_cast<T *>(y);
-  staged_copy<L * FFT_TILE>(
-      K1 * FFT_TILE,
-      [&](int t) {
-        int k1 = t / FFT_TILE, c = t - k1 * FFT_TILE;
-        int col = c0 + c;
-        c2pair<T> v;
-        v.a.x = T(0); v.a.y = T(0); v.b.x = T(0); v.b.y = T(0);
-        if (col < ncol) { v.a = C[k1 * rs + col]; v.b.x = G[k1 * rs + col]; }
-        return v;
-      },
-      [&](int t, c2pair<T> v) {
-        int k1 = t / FFT_TILE, c = t - k1 * FFT_TILE;
-        x[c * ld + k1] = v.a;
-        gst[t] = v.b.x;
-      });
-  __syncthreads();
-  T gvr[(L * FFT_TILE + FFT_THREADS - 1) / FFT_THREADS > 0 ? (L * FFT_TILE + FFT_THREADS - 1) / FFT_THREADS : 1];
-  if constexpr (L > 0) {
-#pragma unroll
-    for (int j = 0; j < (L * FFT_TILE + FFT_THREADS - 1) / FFT_THREADS; ++j) {
-      int t = threadIdx.x + j * FFT_THREADS;
-      gvr[j] = t < K1 * FFT_TILE ? gst[t] : T(0);
-    }
-    __syncthreads();  // y is the transform's scratch from here
-  }
-  c2<T> *res = fft_lines<T, L, true>(x, y, K1, FFT_TILE, ld, S.rad[0], S.nst[0], tws, -1);
-  c2<T> *oth = res == x ? y : x;
-  double acc[7] = {0, 0, 0, 0, 0, 0, 0};
-  const BoxInfo &B = a.box[s];
-#pragma unroll
-  for (int j = 0; j < (L > 0 ? (L * FFT_TILE + FFT_THREADS - 1) / FFT_THREADS : 1); ++j) {
-   for (int t = threadIdx.x + j * FFT_THREADS; t < K1 * FFT_TILE; t += (L > 0 ? K1 * FFT_TILE : (int)blockDim.x)) {
-    int k1 = t / FFT_TILE, c = t - k1 * FFT_TILE;
-    int col = c0 + c;
-    if (col >= ncol) continue;
-    T gv = L > 0 ? gvr[j] : G[k1 * rs + col];
-    c2<T> F = res[c * ld + k1];
-    if (ENERGY && gv != T(0)) {
-      int k2 = col / K3h, m3 = col - k2 * K3h;
-      double w3 = (m3 == 0 || 2 * m3 == K3) ? 1.0 : 2.0;
-      double e = w3 * double(gv) * (double(F.x) * double(F.x) + double(F.y) * double(F.y));
-      int m1 = k1 <= (K1 - 1) / 2 ? k1 : k1 - K1;
-      int m2 = k2 <= (K2 - 1) / 2 ? k2 : k2 - K2;
-      if (K1 % 2 == 0 && k1 == K1 / 2) m1 = -K1 / 2;
-      if (K2 % 2 == 0 && k2 == K2 / 2) m2 = -K2 / 2;
-      double mv[3];
-      for (int cc = 0; cc < 3; ++cc) mv[cc] = m1 * B.Hinv[cc * 3 + 0] + m2 * B.Hinv[cc * 3 + 1] + m3 * B.Hinv[cc * 3 + 2];
-      double msq = mv[0] * mv[0] + mv[1] * mv[1] + mv[2] * mv[2];
-      double fac = 2.0 * (PI * PI / (a.beta * a.beta) + 1.0 / msq);
-      acc[0] += e;
-      acc[1] += e * (fac * mv[0] * mv[0] - 1.0);
-      acc[2] += e * (fac * mv[1] * mv[1] - 1.0);
-      acc[3] += e * (fac * mv[2] * mv[2] - 1.0);
-      acc[4] += e * fac * mv[0] * mv[1];
-      acc[5] += e * fac * mv[0] * mv[2];
-      acc[6] += e * fac * mv[1] * mv[2];
-    }
-    T g2 = T(2) * gv;
-    F.x *= g2; F.y *= g2;
-    res[c * ld + k1] = F;
-   }
-  }
-  if (ENERGY) {
-    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int k = 0; k < 7; ++k) {
-      double v = warp_sum<double>(acc[k]);
-      if (lane == 0) red[k][warp] = v;
-    }
-  }
-  __syncthreads();
-  if (ENERGY && threadIdx.x < 7) {
-    double v = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v += red[threadIdx.x][w];
-    atomicAdd(&a.eacc[s].vinf[threadIdx.x], v);
-  }
-  c2<T> *res2 = fft_lines<T, L, true>(res, oth, K1, FFT_TILE, ld, S.rad[0], S.nst[0], tws, +1);
-  for (int t = threadIdx.x; t < K1 * FFT_TILE; t += blockDim.x) {
-    int k1 = t / FFT_TILE, c = t - k1 * FFT_TILE;
-    int col = c0 + c;
-    if (col < ncol) C[k1 * rs + col] = res2[c * ld + k1];
-  }
-}
-
 // ------------------------------------------------------------------ row field + PME gather
 // One warp (or group of LPA lanes) per atom.  s_i = sum_k de_ik/dd_i (forcefield.py:1395-1402) + dU_rec/dd_i
 // (pme.py:378-388), then by MODE:

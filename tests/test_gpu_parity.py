@@ -425,6 +425,28 @@ def test_field_on_the_workload_meshes(grid, prec):
     assert np.abs(got - ref).max() <= tol * np.abs(ref).max(), np.abs(got - ref).max() / np.abs(ref).max()
 
 
+MESH_LENGTHS = [K for K in range(8, 257, 2) if 2**8 * 3**5 * 5**3 % K == 0]
+
+
+@pytest.mark.parametrize("L", MESH_LENGTHS)
+@pytest.mark.parametrize("prec", ["double", "mixed"])
+def test_field_on_every_mesh_length(L, prec):
+    """Every mesh length the engine takes, along each axis in turn (the last tiles of lines and columns
+    are ragged) and as a plane (K2 = K3), on 64 waters in a cubic box with order 4, against the oracle.
+    Tolerances as on the workload meshes."""
+    from pgm_jax_b200.forcefield import MDSettings, PGMForceField
+    from pgm_jax_b200.systems import water_box
+
+    s, pos, H = water_box(4, 1.2416, seed=3)
+    d = np.random.default_rng(11).normal(scale=0.01, size=(s.n, 3))
+    tol = 1e-9 if prec == "double" else 2e-6
+    for grid in [(L, 8, 10), (10, L, 8), (8, 10, L), (8, L, L)]:
+        st = dict(cutoff=0.6, ewald_beta=6.0, pme_grid=grid, pme_order=4)
+        ref = O.Oracle(s, st).field(pos, H, s.q, d)
+        got = PGMForceField(s, H, MDSettings(precision=prec, **st)).field(pos, H, d, charges=True).cpu().numpy()
+        assert np.abs(got - ref).max() <= tol * np.abs(ref).max(), (grid, np.abs(got - ref).max() / np.abs(ref).max())
+
+
 def test_water4096_frame_matches_oracle():
     """The 4,096-water benchmark frame (12,288 atoms, 4.966 nm box, PME 96^3, cutoff 0.9 nm,
     Ewald 4.0/nm) as a single point at tol 1e-8: the FP64 engine against the oracle (energy 1e-9,
