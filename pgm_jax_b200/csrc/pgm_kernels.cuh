@@ -381,11 +381,10 @@ __global__ void k_nb_lower(int *flag, long long *builds) {
 // ------------------------------------------------------------------ pair rows
 // k_rows: one warp per atom finds the row -- the molecule partners (always kept inside the cutoff;
 // the rigid special table of md/topology.py:161-178), then the candidates of the Verlet list (or
-// the caller's rows), masked to r < rc (forcefield.py:1140-1195) -- and writes k, x, y, z compacted
-// by ballot; then the same warp evaluates the radial kernels G_n = B_n[erf(a r)/r] -
-// B_n[erf(beta r)/r] (forcefield.py:1314-1338, kernels.py:76-118) of its row's entries from the
-// rounded displacements it stored, every lane busy, and writes with them the local
-// preconditioner's short entries and the learned guess's graph edges.
+// the caller's rows), masked to r < rc (forcefield.py:1140-1195).  Kept entries go through a queue of
+// the warp in shared memory; whenever 32 are waiting the warp evaluates their radial kernels
+// (pair_kernels), every lane busy, and writes k, x, y, z, G0..G3 with them, contiguous over the lanes,
+// and the local preconditioner's short entries and the learned guess's graph edges.
 
 // An atom's group of LPA lanes (32: the warp; 16, 8: a half, a quarter warp): its shuffle mask, and the sum over
 // it (the warp's own reduction for a whole warp).
@@ -415,14 +414,13 @@ __device__ __forceinline__ void min_image_fast_f(float &x, float &y, float &z, c
   x -= n * H[0];
 }
 
-// The row scan of atom i by its group of LPA lanes: the molecule partners (special = true), then the
+// The row scan of atom i by its warp: the molecule partners (special = true), then the
 // candidates, one entry per lane and round, the next round's candidate loaded before the current one
-// is tested.  visit(keep, j, x, y, z, special) runs on all LPA lanes every round (it may use the
-// group's collectives);
-// keep is r < rc for an entry of another atom, false on lanes without one; the displacement comes
-// as T, as the rows store it.  Mixed precision: the candidates' FP32 displacements from the wrapped
+// is tested.  visit(keep, j, x, y, z, special) runs on all lanes every round (it may use the warp's
+// collectives); keep is r < rc for an entry of another atom, false on lanes without one; the displacement
+// comes as T, as the rows store it.  Mixed precision: the candidates' FP32 displacements from the wrapped
 // FP32 positions (16-byte gathers), the molecule partners' rounded from FP64.
-template <typename T, int LPA, typename Visit>
+template <typename T, typename Visit>
 __device__ __forceinline__ void row_scan(const Dev<T> &a, const SysInfo &S, const BoxInfo &B, int i, int lane, Visit &&visit) {
   double H[9], id[3];
 #pragma unroll
@@ -431,7 +429,7 @@ __device__ __forceinline__ void row_scan(const Dev<T> &a, const SysInfo &S, cons
   const double4 pi = a.pos4[i];
   const double rc2 = a.cutoff * a.cutoff;
   const int mf = a.molfirst[i], me = a.molend[i];
-  for (int j0 = mf; j0 < me; j0 += LPA) {
+  for (int j0 = mf; j0 < me; j0 += 32) {
     int j = j0 + lane;
     bool keep = false;
     double x = 0, y = 0, z = 0;
@@ -462,7 +460,7 @@ __device__ __forceinline__ void row_scan(const Dev<T> &a, const SysInfo &S, cons
     }
     return j;
   };
-  if (sizeof(T) == 4 && a.pos4f) {
+  if constexpr (sizeof(T) == 4) {
     float Hf[9], idf[3];
 #pragma unroll
     for (int k = 0; k < 9; ++k) Hf[k] = float(H[k]);
@@ -471,10 +469,10 @@ __device__ __forceinline__ void row_scan(const Dev<T> &a, const SysInfo &S, cons
     const float rc2f = float(rc2);
     int jn = partner(lane);
     float4 pn = jn >= 0 ? a.pos4f[jn] : make_float4(0.f, 0.f, 0.f, -1.f);
-    for (int c0 = 0; c0 < nc; c0 += LPA) {
+    for (int c0 = 0; c0 < nc; c0 += 32) {
       const int j = jn;
       const float4 pj = pn;
-      jn = partner(c0 + LPA + lane);  // prefetch the next round
+      jn = partner(c0 + 32 + lane);  // prefetch the next round
       if (jn >= 0) pn = a.pos4f[jn];
       bool keep = false;
       float x = 0.f, y = 0.f, z = 0.f;
@@ -488,10 +486,10 @@ __device__ __forceinline__ void row_scan(const Dev<T> &a, const SysInfo &S, cons
   } else {
     int jn = partner(lane);
     double4 pn = jn >= 0 ? a.pos4[jn] : make_double4(0, 0, 0, -1);
-    for (int c0 = 0; c0 < nc; c0 += LPA) {
+    for (int c0 = 0; c0 < nc; c0 += 32) {
       const int j = jn;
       const double4 pj = pn;
-      jn = partner(c0 + LPA + lane);  // prefetch the next round
+      jn = partner(c0 + 32 + lane);  // prefetch the next round
       if (jn >= 0) pn = a.pos4[jn];
       bool keep = false;
       double x = 0, y = 0, z = 0;
@@ -500,180 +498,122 @@ __device__ __forceinline__ void row_scan(const Dev<T> &a, const SysInfo &S, cons
         min_image_fast(x, y, z, H, id);
         keep = x * x + y * y + z * z < rc2;
       }
-      visit(keep, j, T(x), T(y), T(z), false);
+      visit(keep, j, x, y, z, false);
     }
   }
 }
 
-template <typename T, bool EVAL>
-__device__ __forceinline__ void row_keep(const Dev<T> &a, bool keep, int j, T x, T y, T z, size_t base, int &count, unsigned gm,
-                                         int i, T Ri, int &ecount, int &vcount, int &scount, bool special) {
-  const unsigned lt = (1u << (threadIdx.x & 31)) - 1u;  // the lanes below this one (the group's bits only
-                                                          // are set in its ballots)
-  const T r2 = x * x + y * y + z * z;  // the tests below in the rows' precision
-  bool kv = false;
-  if (a.rnv && keep && !(r2 < T(a.rce2))) {  // split rows: beyond elec_cutoff only pairs with an LJ term stay
-    kv = !special && j >= 0 && a.seps[i] * a.seps[j] != T(0);  // molecule partners have LJ weight 0
-    keep = false;
-  }
-  // the slots first (all lanes take part in the ballots), then one branch for an entry's stores
-  const unsigned bal = __ballot_sync(gm, keep);
-  const int slot = count + __popc(bal & lt);
-  count += __popc(bal);
-  const bool kept = keep && slot < a.mce;
-  if constexpr (!EVAL) {  // the entry alone; its kernels, short entry and edge follow the scan
-    if (kept) {
-      const size_t o = base + slot;
-      a.rk[o] = j;
-      a.rx[o] = x; a.ry[o] = y; a.rz[o] = z;
-    }
-  } else {
-  bool sh = false, ed = false;
-  int at_s = 0, at_e = 0;
-  if (a.sh_n) {  // the local preconditioner's entries: partner, displacement, G1, G2, entry-major
-    sh = kept && r2 < T(a.lc2);
-    const unsigned sb = __ballot_sync(gm, sh);
-    at_s = scount + __popc(sb & lt);
-    scount += __popc(sb);
-    sh = sh && at_s < a.sh_max;
-  }
-  if (a.nn_e4) {  // the learned guess's graph edges: the entries closer than rg, with G1, G2
-    ed = kept && float(r2) < a.nn_rg2;
-    const unsigned eb = __ballot_sync(gm, ed);
-    at_e = ecount + __popc(eb & lt);
-    ecount += __popc(eb);
-    ed = ed && at_e < a.nn_emax;
-  }
-  if (kept) {
-    const size_t o = base + slot;
-    a.rk[o] = j;
-    a.rx[o] = x; a.ry[o] = y; a.rz[o] = z;
-    const T r = t_sqrt(r2), Rk = a.radius[j];
-    const T aik = t_rsqrt(T(2) * (Ri * Ri + Rk * Rk));
-    T A[4], Bb[4];
-    erf_kernels<T>(aik, r, A);
-    erf_kernels<T>(T(a.beta), r, Bb);
-    const T g1 = A[1] - Bb[1], g2 = A[2] - Bb[2];
-    a.rg0[o] = A[0] - Bb[0]; a.rg1[o] = g1; a.rg2[o] = g2; a.rg3[o] = A[3] - Bb[3];
-    if (sh) {
-      const size_t c = (size_t)at_s * a.nt + i;
-      a.c_k[c] = j;
-      a.c_x[c] = x; a.c_y[c] = y; a.c_z[c] = z;
-      a.c_g1[c] = g1; a.c_g2[c] = g2;
-    }
-    if (ed) {
-      const size_t e = (size_t)i * a.nn_emax + at_e;
-      a.nn_e4[e] = make_float4(float(x), float(y), float(z), __int_as_float(j));
-      a.nn_g[e] = make_float2(float(g1), float(g2));
-    }
-  }
-  }
-  if (a.rnv) {
-    const unsigned bv = __ballot_sync(gm, kv);
-    const int sv = vcount + __popc(bv & lt);
-    if (kv && sv < a.mc - a.mce) {
-      const size_t o = base + a.mce + sv;
-      a.rk[o] = j;
-      a.rx[o] = x; a.ry[o] = y; a.rz[o] = z;
-    }
-    vcount += __popc(bv);
-  }
-}
+// Kept entries waiting for their evaluation (ring; at most 63 at a time).
+template <typename T>
+struct RowQueue {
+  int j[64];
+  T x[64], y[64], z[64];
+};
 
-// TWO_PHASE: the scan stores the entries only; then the group evaluates the kernels of its row
-// (read back from L2) with every lane busy, and assigns the short entries and graph edges in row order.
-template <typename T, int LPA = 32, bool TWO_PHASE = false>
-__global__ void __launch_bounds__(8 * LPA, 6 * 32 / LPA) k_rows(Dev<T> a) {
-  static_assert(LPA == 32 || LPA == 16 || LPA == 8, "lanes per atom");
+template <typename T>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_rows(Dev<T> a) {
+  __shared__ RowQueue<T> queues[WARPS_PER_BLOCK];
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
-  const int warp = threadIdx.x / LPA, lane = threadIdx.x % LPA;  // the atom's group of LPA lanes
-  const unsigned gm = group_mask<LPA>();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int s = a.wb_sys[blockIdx.x];
   const int i = a.wb_atom0[blockIdx.x] + warp;
   const SysInfo &S = a.sys[s];
   if (i >= S.atom0 + S.natom) return;
-  const T Ri = a.radius[i];
+  RowQueue<T> &q = queues[warp];
+  const unsigned lt = (1u << lane) - 1u;
+  const T Ri2 = T(2) * a.radius[i] * a.radius[i], beta = T(a.beta);
   const size_t base = (size_t)i * a.mc;
-  int count = 0, ecount = 0, vcount = 0, scount = 0, nsp = 0;
-  row_scan<T, LPA>(a, S, a.box[s], i, lane, [&](bool keep, int j, T x, T y, T z, bool special) {
-    row_keep<T, !TWO_PHASE>(a, keep, j, x, y, z, base, count, gm, i, Ri, ecount, vcount, scount, special);
-    if (special) nsp = count;
-  });
-  if constexpr (TWO_PHASE) {
-    __syncwarp(gm);  // the row, stored by the group's lanes, visible to all of them
-    const unsigned lt = (1u << (threadIdx.x & 31)) - 1u;
-    const int n = min(count, a.mce);
-    const T beta = T(a.beta), lc2 = T(a.lc2);
-    // the next round's entry is loaded before the current one is evaluated
-    auto load = [&](int t, int &j, T &x, T &y, T &z) {
-      const bool in = t < n;
-      const size_t o = base + (in ? t : 0);
-      j = in ? a.rk[o] : 0;
-      x = in ? a.rx[o] : T(0); y = in ? a.ry[o] : T(0); z = in ? a.rz[o] : T(0);
-    };
-    int jn;
-    T xn, yn, zn;
-    load(lane, jn, xn, yn, zn);
-    for (int t0 = 0; t0 < n; t0 += LPA) {
-      const int t = t0 + lane;
-      const bool in = t < n;
-      const size_t o = base + (in ? t : 0);
-      const int j = jn;
-      const T x = xn, y = yn, z = zn;
-      load(t + LPA, jn, xn, yn, zn);
-      const T r2 = x * x + y * y + z * z;
-      bool sh = false, ed = false;
-      int at_s = 0, at_e = 0;
-      if (a.sh_n) {  // the local preconditioner's entries: partner, displacement, G1, G2, entry-major
-        sh = in && r2 < lc2;
-        const unsigned sb = __ballot_sync(gm, sh);
-        at_s = scount + __popc(sb & lt);
-        scount += __popc(sb);
-        sh = sh && at_s < a.sh_max;
+  int head = 0, tail = 0, ecount = 0, vcount = 0, scount = 0, nsp = 0;  // head: evaluated, tail: found
+  auto evaluate = [&](int n) {  // the next n <= 32 entries of the queue, to row slots head .. head + n - 1
+    const int w = (head + lane) & 63, slot = head + lane;
+    const bool in = lane < n && slot < a.mce;
+    const int j = in ? q.j[w] : i;
+    const T x = q.x[w], y = q.y[w], z = q.z[w];
+    const T Rk = a.radius[j];
+    const T r2 = x * x + y * y + z * z;
+    bool sh = false, ed = false;
+    int at_s = 0, at_e = 0;
+    if (a.sh_n) {  // the local preconditioner's entries: partner, displacement, G1, G2, entry-major
+      sh = in && r2 < T(a.lc2);
+      const unsigned sb = __ballot_sync(0xffffffffu, sh);
+      at_s = scount + __popc(sb & lt);
+      scount += __popc(sb);
+      sh = sh && at_s < a.sh_max;
+    }
+    if (a.nn_e4) {  // the learned guess's graph edges: the entries closer than rg, with G1, G2
+      ed = in && float(r2) < a.nn_rg2;
+      const unsigned eb = __ballot_sync(0xffffffffu, ed);
+      at_e = ecount + __popc(eb & lt);
+      ecount += __popc(eb);
+      ed = ed && at_e < a.nn_emax;
+    }
+    if (in) {
+      const size_t o = base + slot;
+      a.rk[o] = j;
+      a.rx[o] = x; a.ry[o] = y; a.rz[o] = z;
+      T g[4];
+      pair_kernels<T>(Ri2 + T(2) * Rk * Rk, beta, r2, g);
+      a.rg0[o] = g[0]; a.rg1[o] = g[1]; a.rg2[o] = g[2]; a.rg3[o] = g[3];
+      if (sh) {
+        const size_t c = (size_t)at_s * a.nt + i;
+        a.c_k[c] = j;
+        a.c_x[c] = x; a.c_y[c] = y; a.c_z[c] = z;
+        a.c_g1[c] = g[1]; a.c_g2[c] = g[2];
       }
-      if (a.nn_e4) {  // the learned guess's graph edges: the entries closer than rg, with G1, G2
-        ed = in && float(r2) < a.nn_rg2;
-        const unsigned eb = __ballot_sync(gm, ed);
-        at_e = ecount + __popc(eb & lt);
-        ecount += __popc(eb);
-        ed = ed && at_e < a.nn_emax;
-      }
-      if (in) {
-        const T r = t_sqrt(r2), Rk = a.radius[j];
-        const T aik = t_rsqrt(T(2) * (Ri * Ri + Rk * Rk));
-        T A[4], Bb[4];
-        erf_kernels<T>(aik, r, A);
-        erf_kernels<T>(beta, r, Bb);
-        const T g1 = A[1] - Bb[1], g2 = A[2] - Bb[2];
-        a.rg0[o] = A[0] - Bb[0]; a.rg1[o] = g1; a.rg2[o] = g2; a.rg3[o] = A[3] - Bb[3];
-        if (sh) {
-          const size_t c = (size_t)at_s * a.nt + i;
-          a.c_k[c] = j;
-          a.c_x[c] = x; a.c_y[c] = y; a.c_z[c] = z;
-          a.c_g1[c] = g1; a.c_g2[c] = g2;
-        }
-        if (ed) {
-          const size_t e = (size_t)i * a.nn_emax + at_e;
-          a.nn_e4[e] = make_float4(float(x), float(y), float(z), __int_as_float(j));
-          a.nn_g[e] = make_float2(float(g1), float(g2));
-        }
+      if (ed) {
+        const size_t e = (size_t)i * a.nn_emax + at_e;
+        a.nn_e4[e] = make_float4(float(x), float(y), float(z), __int_as_float(j));
+        a.nn_g[e] = make_float2(float(g[1]), float(g[2]));
       }
     }
-  }
+    head += n;
+  };
+  row_scan<T>(a, S, a.box[s], i, lane, [&](bool keep, int j, T x, T y, T z, bool special) {
+    if (a.rnv) {  // split rows: beyond elec_cutoff only pairs with an LJ term stay, in the row's second part
+      bool kv = false;
+      if (keep && !(x * x + y * y + z * z < T(a.rce2))) {
+        kv = !special && j >= 0 && a.seps[i] * a.seps[j] != T(0);  // molecule partners have LJ weight 0
+        keep = false;
+      }
+      const unsigned bv = __ballot_sync(0xffffffffu, kv);
+      const int sv = vcount + __popc(bv & lt);
+      if (kv && sv < a.mc - a.mce) {
+        const size_t o = base + a.mce + sv;
+        a.rk[o] = j;
+        a.rx[o] = x; a.ry[o] = y; a.rz[o] = z;
+      }
+      vcount += __popc(bv);
+    }
+    const unsigned bal = __ballot_sync(0xffffffffu, keep);
+    if (keep) {
+      const int w = (tail + __popc(bal & lt)) & 63;
+      q.j[w] = j;
+      q.x[w] = x; q.y[w] = y; q.z[w] = z;
+    }
+    tail += __popc(bal);
+    if (special) nsp = tail;
+    if (tail - head >= 32) {
+      __syncwarp();  // the queue's entries, stored by other lanes
+      evaluate(32);
+      __syncwarp();  // read before their slots are filled again
+    }
+  });
+  __syncwarp();
+  if (tail > head) evaluate(tail - head);
   if (lane == 0) {
-    a.rn[i] = count;
+    a.rn[i] = tail;
     a.rnsp[i] = nsp;
     if (a.nn_e4) a.nn_ne[i] = ecount;
     if (a.sh_n) {
       a.sh_n[i] = min(scount, a.sh_max);
       if (scount > a.sh_max) atomicOr(&a.status[s], 0x20u);  // the preconditioner kept the first sh_max
     }
-    if (count > a.mce) atomicOr(&a.status[s], 0x1u);
-    atomicMax(a.max_count, count);
+    if (tail > a.mce) atomicOr(&a.status[s], 0x1u);
+    if (tail > __ldca(a.max_count)) atomicMax(a.max_count, tail);  // a stale count only costs an atomic
     if (a.rnv) {
       a.rnv[i] = vcount;
       if (vcount > a.mc - a.mce) atomicOr(&a.status[s], 0x1u);
-      atomicMax(a.max_count + 1, vcount);
+      if (vcount > __ldca(a.max_count + 1)) atomicMax(a.max_count + 1, vcount);
     }
   }
 }

@@ -425,6 +425,31 @@ def test_field_on_the_workload_meshes(grid, prec):
     assert np.abs(got - ref).max() <= tol * np.abs(ref).max(), np.abs(got - ref).max() / np.abs(ref).max()
 
 
+@pytest.mark.parametrize("prec,beta", [("double", b) for b in (1.0, 4.0, 8.0, 14.0)] + [("mixed", b) for b in (1.0, 4.0, 8.0)])
+def test_pair_kernels_over_their_ranges(prec, beta):
+    """The field of charges and dipoles of single atoms at all distances from 0.02 nm (both arguments of the
+    pair kernels small) to the cutoff (the Gaussians screened out), with widths on both sides of beta,
+    against the oracle.  Tolerances as for the field of the small box.  At beta 14 / nm the field is a small
+    difference of the row, mesh and self parts (137, 155 and 52 of 80 e/nm^2), whose FP32 mesh part alone is
+    above the mixed tolerance: FP64 only."""
+    from pgm_jax_b200.forcefield import MDSettings, PGMForceField
+    from pgm_jax_b200.systems import Molecule, System
+
+    rng = np.random.default_rng(17)
+    n, edge = 80, 1.3
+    mols = [Molecule("X", ["O"], [q], [r], [1e-3]) for q, r in zip(rng.normal(size=n), rng.uniform(0.03, 0.12, size=n))]
+    s, H = System(mols), np.eye(3) * edge
+    pos = rng.uniform(0, edge, size=(n, 3))
+    u = rng.normal(size=(n // 2, 3))  # every second atom beside its neighbour, 0.02 .. 0.3 nm away
+    pos[1::2] = pos[::2] + u / np.linalg.norm(u, axis=1)[:, None] * np.linspace(0.02, 0.3, n // 2)[:, None]
+    d = rng.normal(scale=0.01, size=(n, 3))
+    st = dict(cutoff=0.6, ewald_beta=beta, pme_grid=(24, 24, 24), pme_order=6)
+    ref = O.Oracle(s, st).field(pos, H, s.q, d)
+    got = PGMForceField(s, H, MDSettings(precision=prec, **st)).field(pos, H, d, charges=True).cpu().numpy()
+    tol = 1e-10 if prec == "double" else 2e-6
+    assert np.abs(got - ref).max() <= tol * np.abs(ref).max(), np.abs(got - ref).max() / np.abs(ref).max()
+
+
 MESH_LENGTHS = [K for K in range(8, 257, 2) if 2**8 * 3**5 * 5**3 % K == 0]
 
 
