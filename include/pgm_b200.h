@@ -221,8 +221,8 @@ long long pgm_launches_per_iteration(const PgmHandle *h);
 int pgm_unrolled_iterations(const PgmHandle *h);
 
 /* Average duration [ms] of one launch of a kernel of the last pgm_compute, re-run `reps` times on
- * `stream` between CUDA events on the state that step left: 0 the CG matvec (row field + PME
- * gather in one kernel), 1 the PME spread, 2 the five FFT/convolution passes, 3 the energy/force
+ * `stream` between CUDA events on the state that step left: 0 the CG matvec (row field, then the
+ * PME gather), 1 the PME spread, 2 the five FFT/convolution passes, 3 the energy/force
  * pass, 4 the row build, 5 the first FFT pass alone, 6 a spread followed by the first FFT pass,
  * 7 the row field alone, 8 the PME gather + operator assembly alone, 9 a whole operator sweep as
  * the solver runs it (spread, row field beside the FFT chain, gather), 10 the learned guess's

@@ -165,7 +165,7 @@ struct Engine : EngineBase {
   double skin = 0.0;
   long long rgrid = 0, cgrid = 0;
   std::vector<std::unique_ptr<FftGroup>> gx, gy, gz, gp;  // k3, k2, k1 passes; plane passes (k3 + k2)
-  int nwblk = 0, ntblk = 0;
+  int nwblk = 0, nqblk = 0, ntblk = 0;
   std::vector<int> natoms;
 
   DBuf<pgm::SysInfo> d_sys;
@@ -173,7 +173,7 @@ struct Engine : EngineBase {
   DBuf<pgm::CGSys> d_cg;
   DBuf<pgm::EnergyAcc> d_eacc;
   DBuf<unsigned> d_status;
-  DBuf<int> wb_sys, wb_atom0, tb_sys, tb_atom0;
+  DBuf<int> wb_sys, wb_atom0, qb_sys, qb_atom0, tb_sys, tb_atom0;
   DBuf<int> sysid, molid, molfirst, molend, mol_start, cov_start, cov_j, cov_i_flat, cov_j_flat;
   DBuf<T> q, radius, alpha, ialpha, rminh, seps;
   DBuf<pgm::v4<T>> qls;
@@ -224,8 +224,9 @@ struct Engine : EngineBase {
   DBuf<T> c_x, c_y, c_z, c_g1, c_g2;
   DBuf<pgm::v4<T>> LRR, LZZ, LP0, LP1, DRv;
   static constexpr int NN_EMAX = 128;
-  // lanes per atom of the spread, the PME gather, the force pass and the learned guess's channel pass (32: a warp per atom; 16, 8: two, four atoms per warp)
-  static constexpr int SPREAD_LPA = 8, GATHER_LPA = 8, FORCES_LPA = 8, CHAN_LPA = 32;
+  static constexpr int QT = pgm::ATOMS_PER_BLOCK * pgm::QL;  // threads of the spread and the PME gather
+  // lanes per atom of the force pass and the learned guess's channel pass (32: a warp per atom; 16, 8: two, four atoms per warp)
+  static constexpr int FORCES_LPA = 8, CHAN_LPA = 32;
   float nn_sigma = 2e-4f, nn_rg = 0.5f;  // until pgm_set_nn_model
   int *h_any = nullptr;
   const double *last_pos = nullptr;
@@ -266,7 +267,7 @@ struct Engine : EngineBase {
     a.c_self = 4.0 * std::pow(set.ewald_beta, 3) / (3.0 * pgm::SQRT_PI);
     a.tol = set.dipole_tol; a.peek = set.peek; a.max_iter = set.max_iter;
     a.sys = d_sys.p; a.box = d_box.p; a.cg = d_cg.p; a.eacc = d_eacc.p; a.status = status;
-    a.wb_sys = wb_sys.p; a.wb_atom0 = wb_atom0.p; a.tb_sys = tb_sys.p; a.tb_atom0 = tb_atom0.p;
+    a.wb_sys = wb_sys.p; a.wb_atom0 = wb_atom0.p; a.qb_sys = qb_sys.p; a.qb_atom0 = qb_atom0.p; a.tb_sys = tb_sys.p; a.tb_atom0 = tb_atom0.p;
     a.sysid = sysid.p; a.molid = molid.p; a.molfirst = molfirst.p; a.molend = molend.p; a.mol_start = mol_start.p;
     a.q = q.p; a.radius = radius.p; a.alpha = alpha.p; a.ialpha = ialpha.p; a.rminh = rminh.p; a.seps = seps.p;
     a.qls = qls.p;
@@ -443,15 +444,17 @@ struct Engine : EngineBase {
     cc_auto = std::max(32, (int)std::ceil((shell * 1.25 + 32.0) / 32.0) * 32);
     cc = set.list_capacity > 0 ? ((set.list_capacity + 31) / 32) * 32 : cc_auto;
     // block maps
-    std::vector<int> wbs, wba, tbs, tba;
+    std::vector<int> wbs, wba, qbs, qba, tbs, tba;
     for (int si = 0; si < n; ++si) {
       const pgm::SysInfo &S = hsys[si];
       for (int a = 0; a < S.natom; a += pgm::WARPS_PER_BLOCK) { wbs.push_back(si); wba.push_back(S.atom0 + a); }
+      for (int a = 0; a < S.natom; a += pgm::ATOMS_PER_BLOCK) { qbs.push_back(si); qba.push_back(S.atom0 + a); }
       for (int a = 0; a < S.natom; a += pgm::THREADS_PER_BLOCK) { tbs.push_back(si); tba.push_back(S.atom0 + a); }
     }
     nwblk = (int)wbs.size();
+    nqblk = (int)qbs.size();
     ntblk = (int)tbs.size();
-    wb_sys.upload(wbs); wb_atom0.upload(wba); tb_sys.upload(tbs); tb_atom0.upload(tba);
+    wb_sys.upload(wbs); wb_atom0.upload(wba); qb_sys.upload(qbs); qb_atom0.upload(qba); tb_sys.upload(tbs); tb_atom0.upload(tba);
     // plane passes for the systems whose K2 = K3 plane fits in a CTA's shared memory; the others run
     // the k3 and k2 passes
     int cur_dev = 0, smem_optin = 0;
@@ -881,8 +884,11 @@ struct Engine : EngineBase {
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
     auto one = [&]() {
-      if (which == 0) pgm::k_rowmat<T, P, false, 1, 0><<<nwblk, 256, 0, st>>>(a, Pv.p, AP.p);
-      else if (which == 1) pgm::k_spread<T, P, false, false, 0, SPREAD_LPA><<<nwblk, 8 * SPREAD_LPA, 0, st>>>(a, Pv.p);
+      if (which == 0) {
+        rowfield<false, 0>(st, a, Pv.p, Fv.p, false);
+        pgm::k_gather<T, P, 1, 0><<<nqblk, QT, 0, st>>>(a, Pv.p, AP.p);
+      }
+      else if (which == 1) pgm::k_spread<T, P, false, false, 0><<<nqblk, QT, 0, st>>>(a, Pv.p);
       else if (which == 2) {
         fft_chain(st, a, 0, false);
       } else if (which == 3) forces_pass(st, a, nullptr, false);
@@ -890,11 +896,11 @@ struct Engine : EngineBase {
         pgm::k_rows<T><<<nwblk, 256, 0, st>>>(a);
       }
       else if (which == 5 || which == 6) {  // the first FFT pass (plane or k3), after the spread with 6
-        if (which == 6) pgm::k_spread<T, P, false, false, 0, SPREAD_LPA><<<nwblk, 8 * SPREAD_LPA, 0, st>>>(a, Pv.p);
+        if (which == 6) pgm::k_spread<T, P, false, false, 0><<<nqblk, QT, 0, st>>>(a, Pv.p);
         fft_pass(st, a, pgmfft::PLANE_FWD, gp, 0);
         fft_pass(st, a, pgmfft::X_FWD, gx, 0);
       } else if (which == 7) rowfield<false, 0>(st, a, Pv.p, Fv.p, false);
-      else if (which == 8) pgm::k_rowmat<T, P, false, 1, 0, false, false, GATHER_LPA><<<nwblk, 8 * GATHER_LPA, 0, st>>>(a, Pv.p, AP.p);
+      else if (which == 8) pgm::k_gather<T, P, 1, 0><<<nqblk, QT, 0, st>>>(a, Pv.p, AP.p);
       else if (which == 9) {  // a whole operator sweep with the row/PME overlap
         sweep<false, false, 0, 1>(st, a, Pv.p, AP.p);
       } else if (which == 10) {  // the learned guess's channel pass (rewrites the same graph field)
@@ -1039,7 +1045,7 @@ struct Engine : EngineBase {
   template <bool WITH_Q, bool UPDATE_P, int ACT, bool ENERGY>
   void pme(cudaStream_t st, pgm::Dev<T> &a, const pgm::v4<T> *vin) {
     // Q is zero here: cleared at creation and, after every spread, by the forward k2 FFT pass
-    launch_pdl(pgm::k_spread<T, P, WITH_Q, UPDATE_P, ACT, SPREAD_LPA>, nwblk, 8 * SPREAD_LPA, 0, st, a, vin);
+    launch_pdl(pgm::k_spread<T, P, WITH_Q, UPDATE_P, ACT>, nqblk, QT, 0, st, a, vin);
     fft_chain(st, a, ACT, ENERGY);
   }
 
@@ -1052,11 +1058,11 @@ struct Engine : EngineBase {
       // one stream: the row field runs between the spread and the first FFT pass, while the L2
       // still processes the spread's atomic adds, then the FFTs and the PME gather
       // Q is zero here: cleared at creation and, after every spread, by the forward k2 FFT pass
-      pgm::k_spread<T, P, WITH_Q, UPDATE_P, ACT, SPREAD_LPA><<<nwblk, 8 * SPREAD_LPA, 0, st>>>(a, vin); check_launch();
+      pgm::k_spread<T, P, WITH_Q, UPDATE_P, ACT><<<nqblk, QT, 0, st>>>(a, vin); check_launch();
       const pgm::v4<T> *dv = UPDATE_P ? Pv.p : vin;
       rowfield<WITH_Q, ACT>(st, a, dv, Fv.p, true);
       fft_chain(st, a, ACT, false);
-      launch_pdl(pgm::k_rowmat<T, P, WITH_Q, MODE, ACT, false, false, GATHER_LPA>, nwblk, 8 * GATHER_LPA, 0, st, a, dv, out);
+      launch_pdl(pgm::k_gather<T, P, MODE, ACT>, nqblk, QT, 0, st, a, dv, out);
       return;
     }
     // the loop body is captured as a sequence of its own: it forks to its own stream
@@ -1069,13 +1075,13 @@ struct Engine : EngineBase {
       CK(cudaStreamWaitEvent(ax, ef, 0));
       rowfield<WITH_Q, ACT>(ax, a, UPDATE_P ? Z.p : vin, Fv.p, false, 0, true);
       CK(cudaEventRecord(ej, ax));
-      launch_pdl(pgm::k_spread<T, P, WITH_Q, UPDATE_P, ACT, SPREAD_LPA>, nwblk, 8 * SPREAD_LPA, 0, st, a, vin);
+      launch_pdl(pgm::k_spread<T, P, WITH_Q, UPDATE_P, ACT>, nqblk, QT, 0, st, a, vin);
       fft_chain(st, a, ACT, false);
       CK(cudaStreamWaitEvent(st, ej, 0));
-      launch_pdl(pgm::k_rowmat<T, P, WITH_Q, MODE, ACT, false, UPDATE_P, GATHER_LPA>, nwblk, 8 * GATHER_LPA, 0, st, a, vin, out);
+      launch_pdl(pgm::k_gather<T, P, MODE, ACT, UPDATE_P>, nqblk, QT, 0, st, a, vin, out);
       return;
     }
-    launch_pdl(pgm::k_spread<T, P, WITH_Q, UPDATE_P, ACT, SPREAD_LPA>, nwblk, 8 * SPREAD_LPA, 0, st, a, vin);
+    launch_pdl(pgm::k_spread<T, P, WITH_Q, UPDATE_P, ACT>, nqblk, QT, 0, st, a, vin);
     CK(cudaEventRecord(ef, st));
     CK(cudaStreamWaitEvent(ax, ef, 0));
     rowfield<WITH_Q, ACT>(ax, a, vin, Fv.p, false, 0, true);
@@ -1083,7 +1089,7 @@ struct Engine : EngineBase {
     fft_chain(st, a, ACT, false);
     CK(cudaStreamWaitEvent(st, ej, 0));
     // a programmatic dependent of the last FFT pass; griddepcontrol.wait also covers the joined row field
-    launch_pdl(pgm::k_rowmat<T, P, WITH_Q, MODE, ACT, false, false, GATHER_LPA>, nwblk, 8 * GATHER_LPA, 0, st, a, vin, out);
+    launch_pdl(pgm::k_gather<T, P, MODE, ACT>, nqblk, QT, 0, st, a, vin, out);
   }
 
   // The local preconditioner's chain z = M^-1 r (k_lp_start, then per inner iteration k_lp_ap and

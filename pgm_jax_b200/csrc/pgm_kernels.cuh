@@ -13,6 +13,8 @@
 // pme.py:243-411, CG forcefield.py:1714-1821, start forcefield.py:1917-2008, energy and forces
 // forcefield.py:2011-2045,2294-2430, strain derivative forcefield.py:608-662,2628-2695.
 #pragma once
+#include <type_traits>
+
 #include "pgm_device.cuh"
 #include "pgm_nn.cuh"
 
@@ -39,7 +41,7 @@ struct Dev {
   EnergyAcc *eacc;
   unsigned *status;
   // block maps (warp-per-atom and thread-per-atom kernels)
-  const int *wb_sys, *wb_atom0, *tb_sys, *tb_atom0;
+  const int *wb_sys, *wb_atom0, *qb_sys, *qb_atom0, *tb_sys, *tb_atom0;  // 8, 32, 256 atoms per block
   // atoms
   const int *sysid, *molid, *molfirst, *molend, *mol_start;
   const T *q, *radius, *alpha, *ialpha, *rminh, *seps;
@@ -651,25 +653,112 @@ __global__ void k_influence(Dev<T> a, long long total) {
   }
 }
 
+// ------------------------------------------------------------------ spline stencils
+// The PME kernels give an atom QL = 8 lanes (four atoms per warp, 32 per block).  The P x P stencil rows along
+// k3 are taken SLOTS at a time, a row's points as GPL aligned vectors of VW (16 bytes where K3 allows it, else
+// two points), one lane each: the vectors of a row sit side by side, so a warp's request touches 16 rows in whole
+// sectors, and a lane's k3 weights stay in registers for all rows.  What bounds them is latency and the L1's line
+// rate: with one point or vector per lane and the k3 weights read from shared memory for every
+// point, a row cost three times the instructions.
+constexpr int QL = 8, ATOMS_PER_BLOCK = 32;
+template <typename T, int VW> struct VecOf;
+template <> struct VecOf<float, 4> { using type = float4; };
+template <> struct VecOf<float, 2> { using type = float2; };
+template <> struct VecOf<double, 2> { using type = double2; };
+
+template <int P, int VW>
+struct Stencil {
+  static constexpr int GPL = VW == 4 ? 2 : 4, SLOTS = QL / GPL, ROUNDS = P * P / SLOTS;
+  static constexpr int NG = (VW + P - 2) / VW + 1;    // most vectors of a row
+  static constexpr int NQ = (NG + GPL - 1) / GPL;     // per lane
+  static_assert(P * P % SLOTS == 0 && SLOTS <= P, "rows in whole rounds");
+};
+
+// A lane's vectors of a row: their k3 weights (0 outside the stencil), places along k3 and whether they are needed.
+template <typename T, int P, int VW, int NW>
+struct RowVectors {
+  static constexpr int NQ = Stencil<P, VW>::NQ;
+  T w[NW][NQ][VW];
+  int at[NQ];
+  bool on[NQ];
+  // wk[n] (P values each): the weights along k3 and their derivatives, in shared memory
+  __device__ __forceinline__ void set(int lane, int bz, int K3, const T *(&wk)[NW], int stride) {
+    const int o = bz % VW, g0 = bz / VW, ng = (o + P - 1) / VW + 1, KV = K3 / VW;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+      const int g = lane % Stencil<P, VW>::GPL + q * Stencil<P, VW>::GPL;
+      on[q] = g < ng;
+      at[q] = g0 + g < KV ? g0 + g : g0 + g - KV;
+#pragma unroll
+      for (int e = 0; e < VW; ++e) {
+        const int j = VW * g + e - o;
+#pragma unroll
+        for (int n = 0; n < NW; ++n) w[n][q][e] = j >= 0 && j < P ? wk[n][j * stride] : T(0);
+      }
+    }
+  }
+};
+
+// f(j1, j2, row) for the rows of a lane's slot; row = index of the row's first vector.
+template <int P, int VW, typename F>
+__device__ __forceinline__ void for_rows(int lane, int4 b, int K1, int K2, int K3, F &&f) {
+  using S = Stencil<P, VW>;
+  int j1 = 0, j2 = lane / S::GPL;
+  const int KV = K3 / VW;
+#pragma unroll(S::ROUNDS <= 9 ? S::ROUNDS : 4)
+  for (int r = 0; r < S::ROUNDS; ++r) {
+    int i1 = b.x + j1; if (i1 >= K1) i1 -= K1;
+    int i2 = b.y + j2; if (i2 >= K2) i2 -= K2;
+    f(j1, j2, (size_t)(i1 * K2 + i2) * KV);
+    j2 += S::SLOTS;
+    if (j2 >= P) { j2 -= P; ++j1; }
+  }
+}
+
+__device__ __forceinline__ void add_vec(float *p, const float (&v)[4]) {
+  atomicAdd(reinterpret_cast<float4 *>(p), make_float4(v[0], v[1], v[2], v[3]));
+}
+__device__ __forceinline__ void add_vec(float *p, const float (&v)[2]) {
+  atomicAdd(reinterpret_cast<float2 *>(p), make_float2(v[0], v[1]));
+}
+__device__ __forceinline__ void add_vec(double *p, const double (&v)[2]) {
+  if (v[0] != 0.0) atomicAdd(p, v[0]);
+  if (v[1] != 0.0) atomicAdd(p + 1, v[1]);
+}
+template <typename T, int VW>
+__device__ __forceinline__ void load_vec(const T *p, T (&v)[VW]) {
+  const auto u = *reinterpret_cast<const typename VecOf<T, VW>::type *>(p);
+  v[0] = u.x; v[1] = u.y;
+  if constexpr (VW == 4) { v[2] = u.z; v[3] = u.w; }
+}
+// f(integral_constant VW) with the widest vector that the mesh allows (K3 is even; grids start 256-byte aligned)
+template <typename T, typename F>
+__device__ __forceinline__ void with_vec(int K3, F &&f) {
+  if constexpr (sizeof(T) == 4) {
+    if ((K3 & 3) == 0) { f(std::integral_constant<int, 4>{}); return; }
+  }
+  f(std::integral_constant<int, 2>{});
+}
+
 // ------------------------------------------------------------------ spread (pme.py:306-337)
-// A group of LPA lanes per atom (a warp, or 16 / 8 lanes: two or four atoms per warp, whose B-spline
-// weights, stencil rounds and tails proceed together), the P^3 stencil over the group's lanes, atomic
-// adds into the system's grid.  With UPDATE_P the CG direction is first advanced, p = z + beta p
-// (forcefield.py:1812), and spread.
-template <typename T, int P, bool WITH_Q, bool UPDATE_P, int ACT, int LPA = 32>
-__global__ void __launch_bounds__(8 * LPA) k_spread(Dev<T> a, const v4<T> *__restrict__ vin) {
-  static_assert(LPA == 32 || LPA == 16 || LPA == 8 || LPA == 4, "lanes per atom");
+// Vector atomic adds into the system's grid: the weight of a point is A(j1, j2) t3 + B(j1, j2) u3 with
+// A = (q t1 + e1 u1) t2 + e2 t1 u2, B = e3 t1 t2.  With UPDATE_P the CG direction is first advanced,
+// p = z + beta p (forcefield.py:1812), and spread.
+template <typename T, int P, bool WITH_Q, bool UPDATE_P, int ACT>
+__global__ void __launch_bounds__(ATOMS_PER_BLOCK * QL) k_spread(Dev<T> a, const v4<T> *__restrict__ vin) {
   pdl_enter();
-  __shared__ T sh[WARPS_PER_BLOCK][2][3][P];  // per atom of the block
-  const int warp = threadIdx.x / LPA, lane = threadIdx.x % LPA;  // the atom's group of LPA lanes
-  const unsigned gm = group_mask<LPA>();
-  int s = a.wb_sys[blockIdx.x];
-  int i = a.wb_atom0[blockIdx.x] + warp;
+  __shared__ c2<T> sh[ATOMS_PER_BLOCK][3][P];  // per atom of the block: weight and derivative
+  const int sub = threadIdx.x / QL, lane = threadIdx.x % QL;  // the atom's group of lanes
+  const unsigned gm = group_mask<QL>();
+  const int s = a.qb_sys[blockIdx.x];
+  const int i = a.qb_atom0[blockIdx.x] + sub;
   const SysInfo &S = a.sys[s];
   if (i >= S.atom0 + S.natom) return;
   if (ACT == 1 && !a.cg[s].active) return;
   if (ACT == 2 && !a.cg[s].sweep2) return;
   if (ACT == 3 && !a.cg[s].fallback) return;
+  const int4 b = a.base[i];
+  const v4<T> f = a.frac[i];
   v4<T> d;
   if (UPDATE_P) {
     v4<T> z = a.Z[i], p = a.P[i];
@@ -681,64 +770,42 @@ __global__ void __launch_bounds__(8 * LPA) k_spread(Dev<T> a, const v4<T> *__res
     d = vin[i];
   }
   const BoxInfo &B = a.box[s];
-  int4 b = a.base[i];
-  v4<T> f = a.frac[i];
+  const int K1 = S.K[0], K2 = S.K[1], K3 = S.K[2];
+  T e = 0;
   if (lane < 3) {
     T th[P], dth[P];
     bspline<T, P, false>(lane == 0 ? f.x : (lane == 1 ? f.y : f.z), th, dth, nullptr);
 #pragma unroll
-    for (int k = 0; k < P; ++k) { sh[warp][0][lane][k] = th[k]; sh[warp][1][lane][k] = dth[k]; }
+    for (int k = 0; k < P; ++k) { sh[sub][lane][k].x = th[k]; sh[sub][lane][k].y = dth[k]; }
+    e = T((double(d.x) * B.Hinv[lane] + double(d.y) * B.Hinv[3 + lane] + double(d.z) * B.Hinv[6 + lane]) * S.K[lane]);
   }
+  const int l0 = (threadIdx.x & 31) & ~(QL - 1);
+  const T e0 = __shfl_sync(gm, e, l0), e1 = __shfl_sync(gm, e, l0 + 1), e2 = __shfl_sync(gm, e, l0 + 2);
   __syncwarp(gm);
-  T e[3];
-#pragma unroll
-  for (int ax = 0; ax < 3; ++ax)
-    e[ax] = T((double(d.x) * B.Hinv[0 * 3 + ax] + double(d.y) * B.Hinv[1 * 3 + ax] + double(d.z) * B.Hinv[2 * 3 + ax]) * S.K[ax]);
-  T qi = WITH_Q ? a.q[i] : T(0);
+  const T qi = WITH_Q ? a.q[i] : T(0);
   T *grid = a.Q + S.rgrid0;
-  const int K1 = S.K[0], K2 = S.K[1], K3 = S.K[2];
-  if constexpr (sizeof(T) == 4) {
-    if ((K3 & 3) == 0 && (S.rgrid0 & 3) == 0) {
-      // 16-byte vector reductions: along k3 the P points of a stencil row fall into ng aligned
-      // groups of 4 (2.4x fewer L2 atomic operations than one per point); the weight of a point is
-      // A(j1, j2) t3 + B(j1, j2) u3 with A = (q t1 + e1 u1) t2 + e2 t1 u2, B = e3 t1 t2.
-      const int g0 = b.z >> 2, ng = ((b.z + P - 1) >> 2) - g0 + 1, K34 = K3 >> 2;
-      for (int sl = lane; sl < P * P * ng; sl += LPA) {
-        int r = ng == 2 ? (sl >> 1) : (ng == 3 ? sl / 3 : sl / ng), gi = sl - r * ng;  // no runtime division for 2, 3
-        int j1 = r / P, j2 = r - j1 * P;
-        T t1 = sh[warp][0][0][j1], t2 = sh[warp][0][1][j2];
-        T u1 = sh[warp][1][0][j1], u2 = sh[warp][1][1][j2];
-        T A = (qi * t1 + e[0] * u1) * t2 + e[1] * t1 * u2, Bw = e[2] * t1 * t2;
-        int g = g0 + gi;
-        float vv[4];
+  with_vec<T>(K3, [&](auto vw) {
+    constexpr int VW = decltype(vw)::value;
+    RowVectors<T, P, VW, 2> rv;
+    const T *wk[2] = {&sh[sub][2][0].x, &sh[sub][2][0].y};
+    rv.set(lane, b.z, K3, wk, 2);
+    for_rows<P, VW>(lane, b, K1, K2, K3, [&](int j1, int j2, size_t row) {
+      const c2<T> w1 = sh[sub][0][j1], w2 = sh[sub][1][j2];
+      const T A = (qi * w1.x + e0 * w1.y) * w2.x + e1 * w1.x * w2.y, Bw = e2 * w1.x * w2.x;
 #pragma unroll
-        for (int el = 0; el < 4; ++el) {
-          int j3 = 4 * g + el - b.z;
-          vv[el] = (j3 >= 0 && j3 < P) ? A * sh[warp][0][2][j3] + Bw * sh[warp][1][2][j3] : 0.0f;
-        }
-        int i1 = b.x + j1; if (i1 >= K1) i1 -= K1;
-        int i2 = b.y + j2; if (i2 >= K2) i2 -= K2;
-        int gp = g >= K34 ? g - K34 : g;
-        atomicAdd(reinterpret_cast<float4 *>(grid + ((size_t)i1 * K2 + i2) * K3) + gp, make_float4(vv[0], vv[1], vv[2], vv[3]));
+      for (int q = 0; q < rv.NQ; ++q) {
+        if (!rv.on[q]) continue;
+        T v[VW];
+#pragma unroll
+        for (int k = 0; k < VW; ++k) v[k] = A * rv.w[0][q][k] + Bw * rv.w[1][q][k];
+        add_vec(grid + (row + rv.at[q]) * VW, v);
       }
-      return;
-    }
-  }
-  for (int p = lane; p < P * P * P; p += LPA) {
-    int j1 = p / (P * P), j2 = (p / P) % P, j3 = p % P;
-    T t1 = sh[warp][0][0][j1], t2 = sh[warp][0][1][j2], t3 = sh[warp][0][2][j3];
-    T u1 = sh[warp][1][0][j1], u2 = sh[warp][1][1][j2], u3 = sh[warp][1][2][j3];
-    T v = (qi * t1 + e[0] * u1) * t2 * t3 + e[1] * t1 * u2 * t3 + e[2] * t1 * t2 * u3;
-    int i1 = b.x + j1; if (i1 >= K1) i1 -= K1;
-    int i2 = b.y + j2; if (i2 >= K2) i2 -= K2;
-    int i3 = b.z + j3; if (i3 >= K3) i3 -= K3;
-    atomicAdd(grid + ((size_t)i1 * K2 + i2) * K3 + i3, v);
-  }
+    });
+  });
 }
 
 // ------------------------------------------------------------------ row field + PME gather
-// One warp (or group of LPA lanes) per atom.  s_i = sum_k de_ik/dd_i (forcefield.py:1395-1402) + dU_rec/dd_i
-// (pme.py:378-388), then by MODE:
+// s_i = sum_k de_ik/dd_i (forcefield.py:1395-1402) + dU_rec/dd_i (pme.py:378-388), then by MODE:
 //   0 FIELD  out = -(s - c_self d)                       (forcefield.py:1428-1433)
 //   1 OPER   out = d / alpha + s - c_self d, and p.Ap    (forcefield.py:1694-1712, 1806-1807)
 // The row part alone: F_i = sum_k de_ik/dd_i (runs beside the PME chain).  LPR lanes per row
@@ -824,118 +891,65 @@ __global__ void __launch_bounds__(8 * LPR) k_rowfield(Dev<T> a, const v4<T> *__r
   }
 }
 
-// ROWS: the row sum is computed here; otherwise it is read from a.F (k_rowfield).  COMBINE (the
-// CG direction's sweep with the row field started before the spread): a.F holds the rows of
-// z, and the rows of p = z + beta p_prev are a.F + beta a.Fp (a.Fp: those of p_prev, rewritten).
-template <typename T, int P, bool WITH_Q, int MODE, int ACT, bool ROWS = true, bool COMBINE = false, int LPA = 32>
-__global__ void __launch_bounds__(8 * LPA) k_rowmat(Dev<T> a, const v4<T> *__restrict__ D, v4<T> *__restrict__ out) {
-  static_assert(LPA == 32 || LPA == 16 || LPA == 8 || LPA == 4, "lanes per atom");
+// The PME gather of the system's potential at every atom, with the row field a.F: assembles the field (MODE 0) or
+// the operator and p.Ap (MODE 1).  COMBINE (the CG direction's sweep with the row field started before the
+// spread): a.F holds the rows of z, and the rows of p = z + beta p_prev are a.F + beta a.Fp (a.Fp: those
+// of p_prev, rewritten).
+template <typename T, int P, int MODE, int ACT, bool COMBINE = false>
+__global__ void __launch_bounds__(ATOMS_PER_BLOCK * QL) k_gather(Dev<T> a, const v4<T> *__restrict__ D, v4<T> *__restrict__ out) {
   pdl_enter();
-  __shared__ T sh[WARPS_PER_BLOCK][2][3][P];  // per atom of the block
-  __shared__ double red[WARPS_PER_BLOCK];
-  const int warp = threadIdx.x / LPA, lane = threadIdx.x % LPA;  // the atom's group of LPA lanes
-  const unsigned gm = group_mask<LPA>();
-  int s = a.wb_sys[blockIdx.x];
-  int i = a.wb_atom0[blockIdx.x] + warp;
+  __shared__ c2<T> sh[ATOMS_PER_BLOCK][3][P];  // per atom of the block: weight and derivative
+  __shared__ double red[ATOMS_PER_BLOCK];
+  const int sub = threadIdx.x / QL, lane = threadIdx.x % QL;  // the atom's group of lanes
+  const unsigned gm = group_mask<QL>();
+  const int s = a.qb_sys[blockIdx.x];
+  const int i = a.qb_atom0[blockIdx.x] + sub;
   const SysInfo &S = a.sys[s];
-  bool valid = i < S.atom0 + S.natom;
+  const bool valid = i < S.atom0 + S.natom;
   if (ACT == 1 && !a.cg[s].active) return;   // uniform over the block
   if (ACT == 2 && !a.cg[s].sweep2) return;
   if (ACT == 3 && !a.cg[s].fallback) return;
   double dotv = 0.0;
   if (valid) {
-    int n = ROWS ? min(a.rn[i], a.mce) : 0;
-    size_t base = (size_t)i * a.mc;
-    T f0 = 0, f1 = 0, f2 = 0;
-    auto pair = [&](int k, T x, T y, T z, T g1, T g2) {
-      v4<T> dk = D[k];
-      T dkx = dk.x * x + dk.y * y + dk.z * z;
-      T c = -g2 * dkx;
-      if (WITH_Q) c -= a.q[k] * g1;
-      f0 += c * x + g1 * dk.x;
-      f1 += c * y + g1 * dk.y;
-      f2 += c * z + g1 * dk.z;
-    };
-    if constexpr (sizeof(T) == 4) {
-      // 16-byte loads: each lane takes 4 consecutive entries of the row (capacity is a multiple of 32)
-      const int4 *k4 = reinterpret_cast<const int4 *>(a.rk + base);
-      const float4 *x4 = reinterpret_cast<const float4 *>(a.rx + base), *y4 = reinterpret_cast<const float4 *>(a.ry + base),
-                   *z4 = reinterpret_cast<const float4 *>(a.rz + base), *p4 = reinterpret_cast<const float4 *>(a.rg1 + base),
-                   *q4 = reinterpret_cast<const float4 *>(a.rg2 + base);
-      for (int t4 = lane; 4 * t4 < n; t4 += LPA) {
-        int4 kk = k4[t4];
-        float4 xx = x4[t4], yy = y4[t4], zz = z4[t4], g1 = p4[t4], g2 = q4[t4];
-        int t = 4 * t4;
-        pair(kk.x, xx.x, yy.x, zz.x, g1.x, g2.x);
-        if (t + 1 < n) pair(kk.y, xx.y, yy.y, zz.y, g1.y, g2.y);
-        if (t + 2 < n) pair(kk.z, xx.z, yy.z, zz.z, g1.z, g2.z);
-        if (t + 3 < n) pair(kk.w, xx.w, yy.w, zz.w, g1.w, g2.w);
-      }
-    } else {
-      for (int t = lane; t < n; t += LPA) {
-        size_t o = base + t;
-        pair(a.rk[o], a.rx[o], a.ry[o], a.rz[o], a.rg1[o], a.rg2[o]);
-      }
-    }
     const BoxInfo &B = a.box[s];
-    int4 b = a.base[i];
-    v4<T> fr = a.frac[i];
+    const int4 b = a.base[i];
+    const v4<T> fr = a.frac[i];
+    const v4<T> rowf = a.F[i], di = D[i];  // the assembly's loads are in flight during the stencil
+    const T ia = MODE == 1 ? a.ialpha[i] : T(0);
     if (lane < 3) {
       T th[P], dth[P];
       bspline<T, P, false>(lane == 0 ? fr.x : (lane == 1 ? fr.y : fr.z), th, dth, nullptr);
 #pragma unroll
-      for (int k = 0; k < P; ++k) { sh[warp][0][lane][k] = th[k]; sh[warp][1][lane][k] = dth[k]; }
+      for (int k = 0; k < P; ++k) { sh[sub][lane][k].x = th[k]; sh[sub][lane][k].y = dth[k]; }
     }
     __syncwarp(gm);
     const T *phi = a.Phi + S.rgrid0;
     const int K1 = S.K[0], K2 = S.K[1], K3 = S.K[2];
     T g0 = 0, g1 = 0, g2 = 0;
-    bool vec = false;
-    if constexpr (sizeof(T) == 4) vec = (K3 & 3) == 0 && (S.rgrid0 & 3) == 0;
-    if (vec) {
-      // 16-byte loads: along k3 the P points of a stencil row fall into ng aligned groups of 4;
-      // one work item per (stencil row, group)
-      const int g0i = b.z >> 2, ng = ((b.z + P - 1) >> 2) - g0i + 1, K34 = K3 >> 2;
-      for (int sl = lane; sl < P * P * ng; sl += LPA) {
-        const int r = ng == 2 ? (sl >> 1) : (ng == 3 ? sl / 3 : sl / ng), gi = sl - r * ng;  // no runtime division for 2, 3
-        const int j1 = r / P, j2 = r - j1 * P;
-        int i1 = b.x + j1; if (i1 >= K1) i1 -= K1;
-        int i2 = b.y + j2; if (i2 >= K2) i2 -= K2;
-        const int g = g0i + gi, gp = g >= K34 ? g - K34 : g;
-        const float4 ph4 = reinterpret_cast<const float4 *>(phi + ((size_t)i1 * K2 + i2) * K3)[gp];
-        const T t1 = sh[warp][0][0][j1], t2 = sh[warp][0][1][j2];
-        const T u1 = sh[warp][1][0][j1], u2 = sh[warp][1][1][j2];
-        const T A0 = u1 * t2, A1 = t1 * u2, A2 = t1 * t2;
-        const float pv[4] = {ph4.x, ph4.y, ph4.z, ph4.w};
+    with_vec<T>(K3, [&](auto vw) {
+      constexpr int VW = decltype(vw)::value;
+      RowVectors<T, P, VW, 2> rv;
+      const T *wk[2] = {&sh[sub][2][0].x, &sh[sub][2][0].y};
+      rv.set(lane, b.z, K3, wk, 2);
+      for_rows<P, VW>(lane, b, K1, K2, K3, [&](int j1, int j2, size_t row) {
+        T st = 0, su = 0;  // the row's sums with the k3 weights and their derivatives
 #pragma unroll
-        for (int el = 0; el < 4; ++el) {
-          const int j3 = 4 * g + el - b.z;
-          if (j3 >= 0 && j3 < P) {
-            const T ph = T(pv[el]), t3 = sh[warp][0][2][j3], u3 = sh[warp][1][2][j3];
-            g0 += ph * A0 * t3;
-            g1 += ph * A1 * t3;
-            g2 += ph * A2 * u3;
-          }
+        for (int q = 0; q < rv.NQ; ++q) {
+          if (!rv.on[q]) continue;
+          T v[VW];
+          load_vec<T, VW>(phi + (row + rv.at[q]) * VW, v);
+#pragma unroll
+          for (int k = 0; k < VW; ++k) { st += v[k] * rv.w[0][q][k]; su += v[k] * rv.w[1][q][k]; }
         }
-      }
-    } else {
-      for (int p = lane; p < P * P * P; p += LPA) {
-        int j1 = p / (P * P), j2 = (p / P) % P, j3 = p % P;
-        int i1 = b.x + j1; if (i1 >= K1) i1 -= K1;
-        int i2 = b.y + j2; if (i2 >= K2) i2 -= K2;
-        int i3 = b.z + j3; if (i3 >= K3) i3 -= K3;
-        T ph = phi[((size_t)i1 * K2 + i2) * K3 + i3];
-        T t1 = sh[warp][0][0][j1], t2 = sh[warp][0][1][j2], t3 = sh[warp][0][2][j3];
-        T u1 = sh[warp][1][0][j1], u2 = sh[warp][1][1][j2], u3 = sh[warp][1][2][j3];
-        g0 += ph * u1 * t2 * t3;
-        g1 += ph * t1 * u2 * t3;
-        g2 += ph * t1 * t2 * u3;
-      }
-    }
-    if (ROWS) { f0 = group_sum<T, LPA>(f0, gm); f1 = group_sum<T, LPA>(f1, gm); f2 = group_sum<T, LPA>(f2, gm); }
-    g0 = group_sum<T, LPA>(g0, gm); g1 = group_sum<T, LPA>(g1, gm); g2 = group_sum<T, LPA>(g2, gm);
+        const c2<T> w1 = sh[sub][0][j1], w2 = sh[sub][1][j2];
+        g0 += w1.y * w2.x * st;
+        g1 += w1.x * w2.y * st;
+        g2 += w1.x * w2.x * su;
+      });
+    });
+    g0 = group_sum<T, QL>(g0, gm); g1 = group_sum<T, QL>(g1, gm); g2 = group_sum<T, QL>(g2, gm);
     if (lane == 0) {
-      if (!ROWS) { v4<T> fr = a.F[i]; f0 = fr.x; f1 = fr.y; f2 = fr.z; }
+      T f0 = rowf.x, f1 = rowf.y, f2 = rowf.z;
       if (COMBINE) {
         const double beta = a.cg[s].beta;
         if (beta != 0.0) {
@@ -953,13 +967,11 @@ __global__ void __launch_bounds__(8 * LPA) k_rowmat(Dev<T> a, const v4<T> *__res
       T r0 = g0 * es[0] + g1 * es[1] + g2 * es[2];
       T r1 = g0 * es[3] + g1 * es[4] + g2 * es[5];
       T r2 = g0 * es[6] + g1 * es[7] + g2 * es[8];
-      v4<T> di = D[i];
       T cs = T(a.c_self);
       v4<T> o;
       if (MODE == 0) {
         o.x = -(f0 + r0 - cs * di.x); o.y = -(f1 + r1 - cs * di.y); o.z = -(f2 + r2 - cs * di.z);
       } else {
-        T ia = a.ialpha[i];
         o.x = di.x * ia + f0 + r0 - cs * di.x;
         o.y = di.y * ia + f1 + r1 - cs * di.y;
         o.z = di.z * ia + f2 + r2 - cs * di.z;
@@ -970,12 +982,11 @@ __global__ void __launch_bounds__(8 * LPA) k_rowmat(Dev<T> a, const v4<T> *__res
     }
   }
   if (MODE == 1) {
-    if (lane == 0) red[warp] = dotv;
+    if (lane == 0) red[sub] = dotv;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      double v = 0;
-      for (int w = 0; w < WARPS_PER_BLOCK; ++w) v += red[w];
-      atomicAdd(&a.cg[s].acc_pap, v);
+    if (threadIdx.x < 32) {
+      const double v = warp_sum<double>(red[threadIdx.x]);
+      if (threadIdx.x == 0) atomicAdd(&a.cg[s].acc_pap, v);
     }
   }
 }
