@@ -406,19 +406,23 @@ __device__ __forceinline__ T group_sum(T v, unsigned m) {
   }
 }
 
-// FP32 sequential minimum image (the mixed-precision row build's candidate loop).
+// FP32 sequential minimum image (the mixed-precision row build's candidate loop).  Rounding to the
+// nearest integer by adding and subtracting 1.5 2^23 (wrapped positions: |argument| < 2): two
+// additions, where rintf is a conversion at a quarter of their rate.
+__device__ __forceinline__ float nearest_f(float x) { return __fadd_rn(__fadd_rn(x, 12582912.f), -12582912.f); }
 __device__ __forceinline__ void min_image_fast_f(float &x, float &y, float &z, const float *H, const float *id) {
-  float n = rintf(z * id[2]);
+  float n = nearest_f(z * id[2]);
   x -= n * H[6]; y -= n * H[7]; z -= n * H[8];
-  n = rintf(y * id[1]);
+  n = nearest_f(y * id[1]);
   x -= n * H[3]; y -= n * H[4];
-  n = rintf(x * id[0]);
+  n = nearest_f(x * id[0]);
   x -= n * H[0];
 }
 
 // The row scan of atom i by its warp: the molecule partners (special = true), then the
-// candidates, one entry per lane and round, the next round's candidate loaded before the current one
-// is tested.  visit(keep, j, x, y, z, special) runs on all lanes every round (it may use the warp's
+// candidates, one entry per lane and round; the index two rounds ahead and the position one round ahead
+// are in flight while the current one is tested (a round that waited for its indices and then for
+// their positions took 1900 cycles on 32 resident warps).  visit(keep, j, x, y, z, special) runs on all lanes every round (it may use the warp's
 // collectives); keep is r < rc for an entry of another atom, false on lanes without one; the displacement
 // comes as T, as the rows store it.  Mixed precision: the candidates' FP32 displacements from the wrapped
 // FP32 positions (16-byte gathers), the molecule partners' rounded from FP64.
@@ -443,25 +447,17 @@ __device__ __forceinline__ void row_scan(const Dev<T> &a, const SysInfo &S, cons
     }
     visit(keep, j, T(x), T(y), T(z), true);
   }
-  const int mi = (int)pi.w;
-  const int *row;
-  int nc;
-  if (a.idx) {  // the caller's candidate rows (local indices, padding natom)
-    row = a.idx + (size_t)i * a.idx_width;
-    nc = a.idx_width;
-  } else {      // the engine's Verlet candidates (within cutoff + skin at the last rebuild)
-    row = a.cand + (size_t)i * a.cc;
-    nc = min(a.ncand[i], a.cc);
-  }
-  auto partner = [&](int c) {
-    int j = -1;
-    if (c < nc) {
-      int jl = row[c];
-      if (a.idx) j = (jl >= 0 && jl < S.natom) ? S.atom0 + jl : -1;
-      else j = jl;
-    }
-    return j;
-  };
+  // the caller's candidate rows (local indices, padding natom), or the engine's Verlet candidates (within
+  // cutoff + skin at the last rebuild)
+  const bool own = a.idx == nullptr;
+  const int *row = own ? a.cand + (size_t)i * a.cc : a.idx + (size_t)i * a.idx_width;
+  const int nc = own ? min(a.ncand[i], a.cc) : a.idx_width;
+  const int first = own ? 0 : S.atom0, limit = own ? a.nt : S.natom;
+  auto index = [&](int c) { return c < nc ? row[c] : -1; };  // as stored: nothing waits for the load here
+  auto partner = [&](int jl) { return jl >= 0 && jl < limit ? jl + first : -1; };
+  // indices two rounds ahead and positions one round ahead are in flight
+  int l2 = index(32 + lane);
+  int jn = partner(index(lane));
   if constexpr (sizeof(T) == 4) {
     float Hf[9], idf[3];
 #pragma unroll
@@ -469,16 +465,16 @@ __device__ __forceinline__ void row_scan(const Dev<T> &a, const SysInfo &S, cons
     idf[0] = float(id[0]); idf[1] = float(id[1]); idf[2] = float(id[2]);
     const float4 pf = a.pos4f[i];
     const float rc2f = float(rc2);
-    int jn = partner(lane);
-    float4 pn = jn >= 0 ? a.pos4f[jn] : make_float4(0.f, 0.f, 0.f, -1.f);
+    float4 pn = jn >= 0 ? a.pos4f[jn] : pf;
     for (int c0 = 0; c0 < nc; c0 += 32) {
       const int j = jn;
       const float4 pj = pn;
-      jn = partner(c0 + 32 + lane);  // prefetch the next round
+      jn = partner(l2);
+      l2 = index(c0 + 64 + lane);
       if (jn >= 0) pn = a.pos4f[jn];
       bool keep = false;
       float x = 0.f, y = 0.f, z = 0.f;
-      if (j >= 0 && (int)pj.w != mi) {
+      if (j >= 0 && pj.w != pf.w) {
         x = pf.x - pj.x; y = pf.y - pj.y; z = pf.z - pj.z;
         min_image_fast_f(x, y, z, Hf, idf);
         keep = x * x + y * y + z * z < rc2f;
@@ -486,16 +482,16 @@ __device__ __forceinline__ void row_scan(const Dev<T> &a, const SysInfo &S, cons
       visit(keep, j, x, y, z, false);
     }
   } else {
-    int jn = partner(lane);
-    double4 pn = jn >= 0 ? a.pos4[jn] : make_double4(0, 0, 0, -1);
+    double4 pn = jn >= 0 ? a.pos4[jn] : pi;
     for (int c0 = 0; c0 < nc; c0 += 32) {
       const int j = jn;
       const double4 pj = pn;
-      jn = partner(c0 + 32 + lane);  // prefetch the next round
+      jn = partner(l2);
+      l2 = index(c0 + 64 + lane);
       if (jn >= 0) pn = a.pos4[jn];
       bool keep = false;
       double x = 0, y = 0, z = 0;
-      if (j >= 0 && (int)pj.w != mi) {
+      if (j >= 0 && pj.w != pi.w) {
         x = pi.x - pj.x; y = pi.y - pj.y; z = pi.z - pj.z;
         min_image_fast(x, y, z, H, id);
         keep = x * x + y * y + z * z < rc2;
