@@ -176,7 +176,7 @@ struct Engine : EngineBase {
   DBuf<int> wb_sys, wb_atom0, qb_sys, qb_atom0, tb_sys, tb_atom0;
   DBuf<int> sysid, molid, molfirst, molend, mol_start, cov_start, cov_j, cov_i_flat, cov_j_flat;
   DBuf<T> q, radius, alpha, ialpha, rminh, seps;
-  DBuf<pgm::v4<T>> qls;
+  DBuf<pgm::c2<T>> ljp;
   DBuf<double> mass, cov_c, cov_c_flat, bmod;
   DBuf<int4> base;
   DBuf<pgm::v4<T>> frac, X, R, Z, Pv, AP, Bv, D, Fv, Fpv;
@@ -224,9 +224,9 @@ struct Engine : EngineBase {
   DBuf<T> c_x, c_y, c_z, c_g1, c_g2;
   DBuf<pgm::v4<T>> LRR, LZZ, LP0, LP1, DRv;
   static constexpr int NN_EMAX = 128;
-  static constexpr int QT = pgm::ATOMS_PER_BLOCK * pgm::QL;  // threads of the spread and the PME gather
-  // lanes per atom of the force pass and the learned guess's channel pass (32: a warp per atom; 16, 8: two, four atoms per warp)
-  static constexpr int FORCES_LPA = 8, CHAN_LPA = 32;
+  static constexpr int QT = pgm::ATOMS_PER_BLOCK * pgm::QL;  // threads of the spread, the PME gather and the force pass
+  // lanes per atom of the learned guess's channel pass (32: a warp per atom; 16, 8: two, four atoms per warp)
+  static constexpr int CHAN_LPA = 32;
   float nn_sigma = 2e-4f, nn_rg = 0.5f;  // until pgm_set_nn_model
   int *h_any = nullptr;
   const double *last_pos = nullptr;
@@ -270,7 +270,7 @@ struct Engine : EngineBase {
     a.wb_sys = wb_sys.p; a.wb_atom0 = wb_atom0.p; a.qb_sys = qb_sys.p; a.qb_atom0 = qb_atom0.p; a.tb_sys = tb_sys.p; a.tb_atom0 = tb_atom0.p;
     a.sysid = sysid.p; a.molid = molid.p; a.molfirst = molfirst.p; a.molend = molend.p; a.mol_start = mol_start.p;
     a.q = q.p; a.radius = radius.p; a.alpha = alpha.p; a.ialpha = ialpha.p; a.rminh = rminh.p; a.seps = seps.p;
-    a.qls = qls.p;
+    a.ljp = ljp.p;
     a.mass = mass.p;
     a.cov_start = cov_start.p; a.cov_j = cov_j.p; a.cov_i_flat = cov_i_flat.p; a.cov_j_flat = cov_j_flat.p;
     a.cov_c = cov_c.p; a.cov_c_flat = cov_c_flat.p;
@@ -523,11 +523,9 @@ struct Engine : EngineBase {
     cov_i_flat.upload(h_covi_flat); cov_j_flat.upload(h_covj_flat);
     q.upload(h_q); radius.upload(h_rad); alpha.upload(h_al); ialpha.upload(h_ial); rminh.upload(h_rh); seps.upload(h_se);
     {
-      std::vector<pgm::v4<T>> h_qls(nt);
-      for (int k = 0; k < nt; ++k) {
-        h_qls[k].x = h_q[k]; h_qls[k].y = h_rh[k]; h_qls[k].z = h_se[k]; h_qls[k].w = T(0);
-      }
-      qls.upload(h_qls);
+      std::vector<pgm::c2<T>> h_ljp(nt);
+      for (int k = 0; k < nt; ++k) { h_ljp[k].x = h_rh[k]; h_ljp[k].y = h_se[k]; }
+      ljp.upload(h_ljp);
     }
     mass.upload(h_mass); cov_c.upload(h_covc); cov_c_flat.upload(h_covc_flat); bmod.upload(h_bmod);
     tw.upload(h_tw);
@@ -669,11 +667,11 @@ struct Engine : EngineBase {
     auto go = [&](auto B) {
       constexpr int MINB = decltype(B)::value;
       if (shadow) {  // iEL/0-SCF: the shadow potential's energy and forces
-        launch_pdl(pgm::k_forces<T, P, MINB, true, FORCES_LPA>, nwblk, 8 * FORCES_LPA, 0, st, a, mu);
+        launch_pdl(pgm::k_forces<T, P, MINB, true>, nqblk, QT, 0, st, a, mu);
       } else if (pdl) {
-        launch_pdl(pgm::k_forces<T, P, MINB, false, FORCES_LPA>, nwblk, 8 * FORCES_LPA, 0, st, a, mu);
+        launch_pdl(pgm::k_forces<T, P, MINB, false>, nqblk, QT, 0, st, a, mu);
       } else {
-        pgm::k_forces<T, P, MINB, false, FORCES_LPA><<<nwblk, 8 * FORCES_LPA, 0, st>>>(a, mu);
+        pgm::k_forces<T, P, MINB, false><<<nqblk, QT, 0, st>>>(a, mu);
         check_launch();
       }
     };

@@ -45,7 +45,7 @@ struct Dev {
   // atoms
   const int *sysid, *molid, *molfirst, *molend, *mol_start;
   const T *q, *radius, *alpha, *ialpha, *rminh, *seps;
-  const v4<T> *qls;  // per atom (q, R*/2, sqrt(eps), 0): one load per partner in the force pass
+  const c2<T> *ljp;  // per atom (R*/2, sqrt(eps)): one load per LJ partner in the force pass
   const double *mass;
   const int *cov_start, *cov_j, *cov_i_flat, *cov_j_flat;
   const double *cov_c, *cov_c_flat;
@@ -696,12 +696,12 @@ struct RowVectors {
 };
 
 // f(j1, j2, row) for the rows of a lane's slot; row = index of the row's first vector.
-template <int P, int VW, typename F>
+template <int P, int VW, int UNROLL, typename F>
 __device__ __forceinline__ void for_rows(int lane, int4 b, int K1, int K2, int K3, F &&f) {
   using S = Stencil<P, VW>;
   int j1 = 0, j2 = lane / S::GPL;
   const int KV = K3 / VW;
-#pragma unroll(S::ROUNDS <= 9 ? S::ROUNDS : 4)
+#pragma unroll(UNROLL)
   for (int r = 0; r < S::ROUNDS; ++r) {
     int i1 = b.x + j1; if (i1 >= K1) i1 -= K1;
     int i2 = b.y + j2; if (i2 >= K2) i2 -= K2;
@@ -785,7 +785,7 @@ __global__ void __launch_bounds__(ATOMS_PER_BLOCK * QL) k_spread(Dev<T> a, const
     RowVectors<T, P, VW, 2> rv;
     const T *wk[2] = {&sh[sub][2][0].x, &sh[sub][2][0].y};
     rv.set(lane, b.z, K3, wk, 2);
-    for_rows<P, VW>(lane, b, K1, K2, K3, [&](int j1, int j2, size_t row) {
+    for_rows<P, VW, Stencil<P, VW>::ROUNDS <= 9 ? Stencil<P, VW>::ROUNDS : 4>(lane, b, K1, K2, K3, [&](int j1, int j2, size_t row) {
       const c2<T> w1 = sh[sub][0][j1], w2 = sh[sub][1][j2];
       const T A = (qi * w1.x + e0 * w1.y) * w2.x + e1 * w1.x * w2.y, Bw = e2 * w1.x * w2.x;
 #pragma unroll
@@ -832,7 +832,7 @@ __global__ void __launch_bounds__(8 * LPR) k_rowfield(Dev<T> a, const v4<T> *__r
     v4<T> dk = D[k];
     T dkx = dk.x * x + dk.y * y + dk.z * z;
     T c = -g2 * dkx;
-    if (WITH_Q) c -= a.q[k] * g1;
+    if (WITH_Q) c -= dk.w * g1;  // the charge rides with the dipole (k_start1, k_load_vec)
     f0 += c * x + g1 * dk.x;
     f1 += c * y + g1 * dk.y;
     f2 += c * z + g1 * dk.z;
@@ -927,7 +927,7 @@ __global__ void __launch_bounds__(ATOMS_PER_BLOCK * QL) k_gather(Dev<T> a, const
       RowVectors<T, P, VW, 2> rv;
       const T *wk[2] = {&sh[sub][2][0].x, &sh[sub][2][0].y};
       rv.set(lane, b.z, K3, wk, 2);
-      for_rows<P, VW>(lane, b, K1, K2, K3, [&](int j1, int j2, size_t row) {
+      for_rows<P, VW, Stencil<P, VW>::ROUNDS <= 9 ? Stencil<P, VW>::ROUNDS : 4>(lane, b, K1, K2, K3, [&](int j1, int j2, size_t row) {
         T st = 0, su = 0;  // the row's sums with the k3 weights and their derivatives
 #pragma unroll
         for (int q = 0; q < rv.NQ; ++q) {
@@ -1217,7 +1217,7 @@ __global__ void k_start1(Dev<T> a, const double *hist, int K, double c0, double 
   v4<T> d, x;
   if (G.fused) { d.x = T(p.x + x0[0]); d.y = T(p.y + x0[1]); d.z = T(p.z + x0[2]); }
   else { d.x = T(p.x); d.y = T(p.y); d.z = T(p.z); }
-  d.w = T(0);
+  d.w = a.q[i];  // read with the dipole by the field sweep
   x.x = T(x0[0]); x.y = T(x0[1]); x.z = T(x0[2]); x.w = T(0);
   a.D[i] = d;
   a.X[i] = x;
@@ -1763,7 +1763,7 @@ __global__ void k_energy_start(Dev<T> a, const double *mu) {
   if (i >= a.nt) return;
   double4 p = a.pperm[i];
   v4<T> d, x;
-  d.x = T(p.x); d.y = T(p.y); d.z = T(p.z); d.w = T(0);
+  d.x = T(p.x); d.y = T(p.y); d.z = T(p.z); d.w = a.q[i];
   x.x = T(mu[3 * i]); x.y = T(mu[3 * i + 1]); x.z = T(mu[3 * i + 2]); x.w = T(0);
   a.D[i] = d;
   a.X[i] = x;
@@ -1826,7 +1826,7 @@ __global__ void k_iel_start1(Dev<T> a, const double *xl, const double *mu) {
   v4<T> d, x;
   if (G.fused) { d.x = T(p.x + x0[0]); d.y = T(p.y + x0[1]); d.z = T(p.z + x0[2]); }
   else { d.x = T(p.x); d.y = T(p.y); d.z = T(p.z); }
-  d.w = T(0);
+  d.w = a.q[i];  // read with the dipole by the field sweep
   x.x = T(x0[0]); x.y = T(x0[1]); x.z = T(x0[2]); x.w = T(0);
   a.D[i] = d;
   a.X[i] = x;
@@ -1986,7 +1986,7 @@ __global__ void k_iel_finish(Dev<T> a, double *mu, double *hist, double *xl, Iel
 }
 
 // ------------------------------------------------------------------ energy, forces, virial
-// One group of LPA lanes per atom over its row: pair energies and their row gradients with the analytic
+// One group of QL lanes per atom over its row: pair energies and their row gradients with the analytic
 // kernels G0..G3 (forcefield.py:2294-2360), LJ rows, the row field at (q, d) (dE/dd), the pair
 // virial sum g (x) x - gx (x) off; then the PME gradients of the atom: dU/dd and dU/dr through the
 // spline derivatives (the autodiff of pme.py:390-411 written out).
@@ -1995,16 +1995,16 @@ __global__ void k_iel_finish(Dev<T> a, double *mu, double *hist, double *xl, Iel
 // atoms with the block preconditioner, the i-side delta scaled by a.iel_keep = 1 - 1/omega); their
 // position gradients at fixed delta go to the forces, not to the virial (the fixed-mu strain
 // derivative); the sums of |delta|^2 and |delta|^2 / (2 alpha) go to the energy accumulators.
-template <typename T, int P, int MINB = 3, bool SHADOW = false, int LPA = 32>
-__global__ void __launch_bounds__(8 * LPA, MINB * 32 / LPA) k_forces(Dev<T> a, const double *mu) {
-  static_assert(LPA == 32 || LPA == 16 || LPA == 8, "lanes per atom");
+template <typename T, int P, int MINB = 3, bool SHADOW = false>
+__global__ void __launch_bounds__(ATOMS_PER_BLOCK * QL, MINB) k_forces(Dev<T> a, const double *mu) {
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
-  __shared__ T sh[WARPS_PER_BLOCK][3][3][P];  // per atom of the block
-  __shared__ double red[WARPS_PER_BLOCK][16];
-  const int warp = threadIdx.x / LPA, lane = threadIdx.x % LPA;  // the atom's group of LPA lanes
-  const unsigned gm = group_mask<LPA>();
-  int s = a.wb_sys[blockIdx.x];
-  int i = a.wb_atom0[blockIdx.x] + warp;
+  __shared__ T sh[ATOMS_PER_BLOCK][3][3][P];  // per atom of the block: weights, first and second derivatives
+  __shared__ T rec[ATOMS_PER_BLOCK][6];        // dU/dd and dU/dr along the mesh axes
+  __shared__ double red[ATOMS_PER_BLOCK][16];
+  const int sub = threadIdx.x / QL, lane = threadIdx.x % QL;  // the atom's group of lanes
+  const unsigned gm = group_mask<QL>();
+  int s = a.qb_sys[blockIdx.x];
+  int i = a.qb_atom0[blockIdx.x] + sub;
   const SysInfo &S = a.sys[s];
   bool valid = i < S.atom0 + S.natom;
   double vals[16];
@@ -2026,6 +2026,84 @@ __global__ void __launch_bounds__(8 * LPA, MINB * 32 / LPA) k_forces(Dev<T> a, c
       const int msz = a.molend[i] - a.molfirst[i];
       blk_i = a.iel_keep_on && msz >= 2 && msz <= 8;
     }
+    // reciprocal gradients of the atom first; their sums wait in shared memory, not in registers, for
+    // the pair loop
+    int4 b = a.base[i];
+    v4<T> fr = a.frac[i];
+    if (lane < 3) {
+      T th[P], dth[P], d2[P];
+      bspline<T, P, true>(lane == 0 ? fr.x : (lane == 1 ? fr.y : fr.z), th, dth, d2);
+#pragma unroll
+      for (int k = 0; k < P; ++k) { sh[sub][0][lane][k] = th[k]; sh[sub][1][lane][k] = dth[k]; sh[sub][2][lane][k] = d2[k]; }
+    }
+    __syncwarp(gm);
+    auto scaled = [&](int bb, int aa) { return T(B.Hinv[bb * 3 + aa] * S.K[aa]); };  // dU/dr_b = sum_a g_a scaled(b, a)
+    {
+    T es[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) es[k] = scaled(k / 3, k % 3);
+    const int K1 = S.K[0], K2 = S.K[1], K3 = S.K[2];
+    // The stencil rows of a potential: f(j1, A, B, C, D, E, F) with the row's sums along k3 (weights, first, second
+    // derivatives: st, su, sv) times the k2 weights t2, u2, v2: A = t2 st, B = u2 st, C = t2 su, D = v2 st,
+    // E = u2 su, F = t2 sv.
+    auto stencil = [&](const T *phi, auto &&f) {
+      with_vec<T>(K3, [&](auto vw) {
+        constexpr int VW = decltype(vw)::value;
+        RowVectors<T, P, VW, 3> rv;
+        const T *wk[3] = {sh[sub][0][2], sh[sub][1][2], sh[sub][2][2]};
+        rv.set(lane, b.z, K3, wk, 1);
+        for_rows<P, VW, 3>(lane, b, K1, K2, K3, [&](int j1, int j2, size_t row) {
+          T st = 0, su = 0, sv = 0;
+#pragma unroll
+          for (int q = 0; q < rv.NQ; ++q) {
+            if (!rv.on[q]) continue;
+            T v[VW];
+            load_vec<T, VW>(phi + (row + rv.at[q]) * VW, v);
+#pragma unroll
+            for (int k = 0; k < VW; ++k) { st += v[k] * rv.w[0][q][k]; su += v[k] * rv.w[1][q][k]; sv += v[k] * rv.w[2][q][k]; }
+          }
+          const T t2 = sh[sub][0][1][j2], u2 = sh[sub][1][1][j2], v2 = sh[sub][2][1][j2];
+          f(j1, t2 * st, u2 * st, t2 * su, v2 * st, u2 * su, t2 * sv);
+        });
+      });
+    };
+    T ge0 = 0, ge1 = 0, ge2 = 0, gw0 = 0, gw1 = 0, gw2 = 0;
+    if constexpr (SHADOW) {  // d/dr of the reciprocal energy of delta alone (its potential in Phi2)
+      const T f0 = Dli.x * es[0] + Dli.y * es[3] + Dli.z * es[6];
+      const T f1 = Dli.x * es[1] + Dli.y * es[4] + Dli.z * es[7];
+      const T f2 = Dli.x * es[2] + Dli.y * es[5] + Dli.z * es[8];
+      T h0 = 0, h1 = 0, h2 = 0;
+      stencil(a.Phi2 + S.rgrid0, [&](int j1, T A, T Bv, T C, T Dv, T E, T F) {
+        const T t1 = sh[sub][0][0][j1], u1 = sh[sub][1][0][j1], v1 = sh[sub][2][0][j1];
+        h0 += f0 * v1 * A + f1 * u1 * Bv + f2 * u1 * C;
+        h1 += f0 * u1 * Bv + f1 * t1 * Dv + f2 * t1 * E;
+        h2 += f0 * u1 * C + f1 * t1 * E + f2 * t1 * F;
+      });
+      // the pair part is KE (gx + gs); the reciprocal part of -U_rec(0, delta) enters with a minus sign
+      gs0 = -h0 * es[0] - h1 * es[1] - h2 * es[2];
+      gs1 = -h0 * es[3] - h1 * es[4] - h2 * es[5];
+      gs2 = -h0 * es[6] - h1 * es[7] - h2 * es[8];
+    }
+    const T e0 = di.x * es[0] + di.y * es[3] + di.z * es[6];
+    const T e1 = di.x * es[1] + di.y * es[4] + di.z * es[7];
+    const T e2 = di.x * es[2] + di.y * es[5] + di.z * es[8];
+    stencil(a.Phi + S.rgrid0, [&](int j1, T A, T Bv, T C, T Dv, T E, T F) {
+      const T t1 = sh[sub][0][0][j1], u1 = sh[sub][1][0][j1], v1 = sh[sub][2][0][j1];
+      const T qt = qi * t1 + e0 * u1, qu = qi * u1 + e0 * v1;
+      ge0 += u1 * A;
+      ge1 += t1 * Bv;
+      ge2 += t1 * C;
+      gw0 += qu * A + e1 * u1 * Bv + e2 * u1 * C;
+      gw1 += qt * Bv + e1 * t1 * Dv + e2 * t1 * E;
+      gw2 += qt * C + e1 * t1 * E + e2 * t1 * F;
+    });
+    ge0 = group_sum<T, QL>(ge0, gm); ge1 = group_sum<T, QL>(ge1, gm); ge2 = group_sum<T, QL>(ge2, gm);
+    gw0 = group_sum<T, QL>(gw0, gm); gw1 = group_sum<T, QL>(gw1, gm); gw2 = group_sum<T, QL>(gw2, gm);
+    if (lane == 0) {
+      T *o = rec[sub];
+      o[0] = ge0; o[1] = ge1; o[2] = ge2; o[3] = gw0; o[4] = gw1; o[5] = gw2;
+    }
+    }
     auto pair = [&](int k, T x, T y, T z, T G0, T G1, T G2, T G3, int t) {
       v4<T> dk = a.D[k];
       if constexpr (SHADOW) {
@@ -2039,8 +2117,7 @@ __global__ void __launch_bounds__(8 * LPA, MINB * 32 / LPA) k_forces(Dev<T> a, c
         gs1 += rad2 * y + G2 * (wb * Dli.y * Dkx + Dk.y * Dix);
         gs2 += rad2 * z + G2 * (wb * Dli.z * Dkx + Dk.z * Dix);
       }
-      v4<T> pk = a.qls[k];  // q, R*/2, sqrt(eps) of the partner in one load
-      T qk = pk.x;
+      const T qk = dk.w;
       T dix = di.x * x + di.y * y + di.z * z;
       T dkx = dk.x * x + dk.y * y + dk.z * z;
       T didk = di.x * dk.x + di.y * dk.y + di.z * dk.z;
@@ -2055,9 +2132,12 @@ __global__ void __launch_bounds__(8 * LPA, MINB * 32 / LPA) k_forces(Dev<T> a, c
       T gzv = radial * z + u1 * dk.z - u2 * di.z;
       fd0 += G1 * dk.x - u2 * x; fd1 += G1 * dk.y - u2 * y; fd2 += G1 * dk.z - u2 * z;
       T kx = T(KE) * gxv, ky = T(KE) * gyv, kz = T(KE) * gzv;
-      T ep = sei * pk.z;
-      if (a.lj && t >= nsp && ep != T(0)) {  // LJ: not for molecule partners, nor pairs without an LJ term
-        T rm = rhi + pk.y;
+      c2<T> lj;
+      lj.x = T(0); lj.y = T(0);
+      if (a.lj && sei != T(0)) lj = a.ljp[k];  // only the rows of atoms with an LJ term ask for it
+      T ep = sei * lj.y;
+      if (t >= nsp && ep != T(0)) {  // LJ: not for molecule partners, nor pairs without an LJ term
+        T rm = rhi + lj.x;
         T r2 = x * x + y * y + z * z;
         const T ir2 = T(1) / r2;
         T s2 = rm * rm * ir2, s6 = s2 * s2 * s2;
@@ -2078,7 +2158,7 @@ __global__ void __launch_bounds__(8 * LPA, MINB * 32 / LPA) k_forces(Dev<T> a, c
                    *z4 = reinterpret_cast<const float4 *>(a.rz + base), *h0 = reinterpret_cast<const float4 *>(a.rg0 + base),
                    *h1 = reinterpret_cast<const float4 *>(a.rg1 + base), *h2 = reinterpret_cast<const float4 *>(a.rg2 + base),
                    *h3 = reinterpret_cast<const float4 *>(a.rg3 + base);
-      for (int t4 = lane; 4 * t4 < n; t4 += LPA) {
+      for (int t4 = lane; 4 * t4 < n; t4 += QL) {
         int4 kk = __ldcs(k4 + t4);
         float4 xx = __ldcs(x4 + t4), yy = __ldcs(y4 + t4), zz = __ldcs(z4 + t4);
         float4 a0 = __ldcs(h0 + t4), a1 = __ldcs(h1 + t4), a2 = __ldcs(h2 + t4), a3 = __ldcs(h3 + t4);
@@ -2089,14 +2169,14 @@ __global__ void __launch_bounds__(8 * LPA, MINB * 32 / LPA) k_forces(Dev<T> a, c
         if (t + 3 < n) pair(kk.w, xx.w, yy.w, zz.w, a0.w, a1.w, a2.w, a3.w, t + 3);
       }
     } else {
-      for (int t = lane; t < n; t += LPA) {
+      for (int t = lane; t < n; t += QL) {
         size_t o = base + t;
         pair(a.rk[o], a.rx[o], a.ry[o], a.rz[o], a.rg0[o], a.rg1[o], a.rg2[o], a.rg3[o], t);
       }
     }
     if (a.rnv) {  // split rows: the LJ pairs between elec_cutoff and cutoff
       const int nv = min(a.rnv[i], a.mc - a.mce);
-      for (int t = lane; t < nv; t += LPA) {
+      for (int t = lane; t < nv; t += QL) {
         size_t o = base + a.mce + t;
         int k = a.rk[o];
         T x = a.rx[o], y = a.ry[o], z = a.rz[o];
@@ -2113,78 +2193,16 @@ __global__ void __launch_bounds__(8 * LPA, MINB * 32 / LPA) k_forces(Dev<T> a, c
         w[6] += kz * x; w[7] += kz * y; w[8] += kz * z;
       }
     }
-    // reciprocal gradients of the atom
-    int4 b = a.base[i];
-    v4<T> fr = a.frac[i];
-    if (lane < 3) {
-      T th[P], dth[P], d2[P];
-      bspline<T, P, true>(lane == 0 ? fr.x : (lane == 1 ? fr.y : fr.z), th, dth, d2);
+    T red_in[20] = {gx0, gx1, gx2, gl0, gl1, gl2, fd0, fd1, fd2, ee, el, w[0], w[1], w[2], w[3], w[4], w[5], w[6], w[7], w[8]};
 #pragma unroll
-      for (int k = 0; k < P; ++k) { sh[warp][0][lane][k] = th[k]; sh[warp][1][lane][k] = dth[k]; sh[warp][2][lane][k] = d2[k]; }
-    }
-    __syncwarp(gm);
-    T es[9];
-#pragma unroll
-    for (int bb = 0; bb < 3; ++bb)
-#pragma unroll
-      for (int aa = 0; aa < 3; ++aa) es[bb * 3 + aa] = T(B.Hinv[bb * 3 + aa] * S.K[aa]);
-    T e0 = di.x * es[0] + di.y * es[3] + di.z * es[6];
-    T e1 = di.x * es[1] + di.y * es[4] + di.z * es[7];
-    T e2 = di.x * es[2] + di.y * es[5] + di.z * es[8];
-    const T *phi = a.Phi + S.rgrid0;
-    const int K1 = S.K[0], K2 = S.K[1], K3 = S.K[2];
-    T ge0 = 0, ge1 = 0, ge2 = 0, gw0 = 0, gw1 = 0, gw2 = 0;
-    if constexpr (SHADOW) {  // d/dr of the reciprocal energy of delta alone (its potential in Phi2)
-      const T f0 = Dli.x * es[0] + Dli.y * es[3] + Dli.z * es[6];
-      const T f1 = Dli.x * es[1] + Dli.y * es[4] + Dli.z * es[7];
-      const T f2 = Dli.x * es[2] + Dli.y * es[5] + Dli.z * es[8];
-      const T *phi2 = a.Phi2 + S.rgrid0;
-      T h0 = 0, h1 = 0, h2 = 0;
-      for (int p = lane; p < P * P * P; p += LPA) {
-        int j1 = p / (P * P), j2 = (p / P) % P, j3 = p % P;
-        int i1 = b.x + j1; if (i1 >= K1) i1 -= K1;
-        int i2 = b.y + j2; if (i2 >= K2) i2 -= K2;
-        int i3 = b.z + j3; if (i3 >= K3) i3 -= K3;
-        T ph = phi2[((size_t)i1 * K2 + i2) * K3 + i3];
-        T t1 = sh[warp][0][0][j1], t2 = sh[warp][0][1][j2], t3 = sh[warp][0][2][j3];
-        T u1 = sh[warp][1][0][j1], u2 = sh[warp][1][1][j2], u3 = sh[warp][1][2][j3];
-        T v1 = sh[warp][2][0][j1], v2 = sh[warp][2][1][j2], v3 = sh[warp][2][2][j3];
-        h0 += ph * (f0 * v1 * t2 * t3 + f1 * u1 * u2 * t3 + f2 * u1 * t2 * u3);
-        h1 += ph * (f0 * u1 * u2 * t3 + f1 * t1 * v2 * t3 + f2 * t1 * u2 * u3);
-        h2 += ph * (f0 * u1 * t2 * u3 + f1 * t1 * u2 * u3 + f2 * t1 * t2 * v3);
-      }
-      // the pair part is KE (gx + gs); the reciprocal part of -U_rec(0, delta) enters with a minus sign
-      gs0 = gs0 - h0 * es[0] - h1 * es[1] - h2 * es[2];
-      gs1 = gs1 - h0 * es[3] - h1 * es[4] - h2 * es[5];
-      gs2 = gs2 - h0 * es[6] - h1 * es[7] - h2 * es[8];
-    }
-    for (int p = lane; p < P * P * P; p += LPA) {
-      int j1 = p / (P * P), j2 = (p / P) % P, j3 = p % P;
-      int i1 = b.x + j1; if (i1 >= K1) i1 -= K1;
-      int i2 = b.y + j2; if (i2 >= K2) i2 -= K2;
-      int i3 = b.z + j3; if (i3 >= K3) i3 -= K3;
-      T ph = phi[((size_t)i1 * K2 + i2) * K3 + i3];
-      T t1 = sh[warp][0][0][j1], t2 = sh[warp][0][1][j2], t3 = sh[warp][0][2][j3];
-      T u1 = sh[warp][1][0][j1], u2 = sh[warp][1][1][j2], u3 = sh[warp][1][2][j3];
-      T v1 = sh[warp][2][0][j1], v2 = sh[warp][2][1][j2], v3 = sh[warp][2][2][j3];
-      ge0 += ph * u1 * t2 * t3;
-      ge1 += ph * t1 * u2 * t3;
-      ge2 += ph * t1 * t2 * u3;
-      gw0 += ph * (qi * u1 * t2 * t3 + e0 * v1 * t2 * t3 + e1 * u1 * u2 * t3 + e2 * u1 * t2 * u3);
-      gw1 += ph * (qi * t1 * u2 * t3 + e0 * u1 * u2 * t3 + e1 * t1 * v2 * t3 + e2 * t1 * u2 * u3);
-      gw2 += ph * (qi * t1 * t2 * u3 + e0 * u1 * t2 * u3 + e1 * t1 * u2 * u3 + e2 * t1 * t2 * v3);
-    }
-    T red_in[24] = {gx0, gx1, gx2, gl0, gl1, gl2, fd0, fd1, fd2, ee, el, ge0, ge1, ge2, gw0, gw1, gw2,
-                    w[0], w[1], w[2], w[3], w[4], w[5], w[6]};
-#pragma unroll
-    for (int k = 0; k < 24; ++k) red_in[k] = group_sum<T, LPA>(red_in[k], gm);
-    T w7 = group_sum<T, LPA>(w[7], gm), w8 = group_sum<T, LPA>(w[8], gm);
-    if constexpr (SHADOW) { gs0 = group_sum<T, LPA>(gs0, gm); gs1 = group_sum<T, LPA>(gs1, gm); gs2 = group_sum<T, LPA>(gs2, gm); }
+    for (int k = 0; k < 20; ++k) red_in[k] = group_sum<T, QL>(red_in[k], gm);
+    if constexpr (SHADOW) { gs0 = group_sum<T, QL>(gs0, gm); gs1 = group_sum<T, QL>(gs1, gm); gs2 = group_sum<T, QL>(gs2, gm); }
     if (lane == 0) {
       double gd[3], gr[3];
       for (int bb = 0; bb < 3; ++bb) {
-        gd[bb] = double(red_in[11]) * double(es[bb * 3 + 0]) + double(red_in[12]) * double(es[bb * 3 + 1]) + double(red_in[13]) * double(es[bb * 3 + 2]);
-        gr[bb] = double(red_in[14]) * double(es[bb * 3 + 0]) + double(red_in[15]) * double(es[bb * 3 + 1]) + double(red_in[16]) * double(es[bb * 3 + 2]);
+        const double s0 = double(scaled(bb, 0)), s1 = double(scaled(bb, 1)), s2 = double(scaled(bb, 2));
+        gd[bb] = double(rec[sub][0]) * s0 + double(rec[sub][1]) * s1 + double(rec[sub][2]) * s2;
+        gr[bb] = double(rec[sub][3]) * s0 + double(rec[sub][4]) * s1 + double(rec[sub][5]) * s2;
       }
       double d3[3] = {double(di.x), double(di.y), double(di.z)};
       double gx[3] = {double(red_in[0]), double(red_in[1]), double(red_in[2])};
@@ -2213,20 +2231,18 @@ __global__ void __launch_bounds__(8 * LPA, MINB * 32 / LPA) k_forces(Dev<T> a, c
         vals[3] = (m0 * m0 + m1 * m1 + m2 * m2) / (2.0 * double(a.alpha[i]));
       }
       // virial: 1/2 sum_rows g (x) x - (KE gx + gl) (x) off - KE (dU/dr (x) off + dU/dd (x) d)
-      double wsum[9] = {double(red_in[17]), double(red_in[18]), double(red_in[19]), double(red_in[20]), double(red_in[21]),
-                        double(red_in[22]), double(red_in[23]), double(w7), double(w8)};
       for (int aa = 0; aa < 3; ++aa)
         for (int bb = 0; bb < 3; ++bb)
-          vals[4 + aa * 3 + bb] = 0.5 * wsum[aa * 3 + bb] - (KE * gx[aa] + gl[aa]) * ofs[bb] - KE * (gr[aa] * ofs[bb] + gd[aa] * d3[bb]);
+          vals[4 + aa * 3 + bb] = 0.5 * double(red_in[11 + aa * 3 + bb]) - (KE * gx[aa] + gl[aa]) * ofs[bb] - KE * (gr[aa] * ofs[bb] + gd[aa] * d3[bb]);
     }
   }
   constexpr int NV = SHADOW ? 15 : 13;
   if (lane == 0)
-    for (int k = 0; k < NV; ++k) red[warp][k] = vals[k];
+    for (int k = 0; k < NV; ++k) red[sub][k] = vals[k];
   __syncthreads();
   if (threadIdx.x < NV) {
     double v = 0;
-    for (int w2 = 0; w2 < WARPS_PER_BLOCK; ++w2) v += red[w2][threadIdx.x];
+    for (int w2 = 0; w2 < ATOMS_PER_BLOCK; ++w2) v += red[w2][threadIdx.x];
     EnergyAcc &E = a.eacc[s];
     double *dst = threadIdx.x == 0 ? &E.e_pair : threadIdx.x == 1 ? &E.e_lj : threadIdx.x == 2 ? &E.d2
                   : threadIdx.x == 3 ? &E.upol : threadIdx.x == 13 ? &E.dd2 : threadIdx.x == 14 ? &E.dda
@@ -2308,7 +2324,7 @@ __global__ void k_total_dipoles(Dev<T> a, const double *mu) {
   double4 p = a.pperm[i];
   double m0 = mu ? mu[3 * i] : 0.0, m1 = mu ? mu[3 * i + 1] : 0.0, m2 = mu ? mu[3 * i + 2] : 0.0;
   v4<T> d;
-  d.x = T(p.x + m0); d.y = T(p.y + m1); d.z = T(p.z + m2); d.w = T(0);
+  d.x = T(p.x + m0); d.y = T(p.y + m1); d.z = T(p.z + m2); d.w = a.q[i];
   a.D[i] = d;
 }
 
@@ -2319,7 +2335,7 @@ __global__ void k_load_vec(Dev<T> a, const double *v, v4<T> *out) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.nt) return;
   v4<T> d;
-  d.x = T(v[3 * i]); d.y = T(v[3 * i + 1]); d.z = T(v[3 * i + 2]); d.w = T(0);
+  d.x = T(v[3 * i]); d.y = T(v[3 * i + 1]); d.z = T(v[3 * i + 2]); d.w = a.q[i];
   out[i] = d;
 }
 
