@@ -186,9 +186,9 @@ struct Engine : EngineBase {
   DBuf<float4> pos4f;  // mixed precision: wrapped FP32 positions for the row build
   DBuf<int> cand, ncand, nb_flag;
   DBuf<long long> nb_builds;
-  DBuf<int> rn, rnsp, rk, dmax, dany;
+  DBuf<int> rn, rnsp, dmax, dany;
   DBuf<unsigned> cg_done;  // blocks of the fused CG update that have finished (the last one checks)
-  DBuf<T> rx, ry, rz, rg0, rg1, rg2, rg3;
+  DBuf<unsigned char> rows;
   DBuf<T> Q, Phi, Ginf;
   DBuf<pgm::c2<T>> C, tw;
   DBuf<double> mu_tmp, forces_tmp, energy_tmp;
@@ -282,8 +282,7 @@ struct Engine : EngineBase {
     a.skin = skin; a.cc = cc; a.nb_flag = nb_flag.p; a.nb_builds = nb_builds.p; a.cand = cand.p; a.ncand = ncand.p;
     a.pos_ref = pos_ref.p; a.pos4 = pos4.p; a.pos4f = pos4f.p;
     a.idx = idx; a.idx_width = idx_width;
-    a.rn = rn.p; a.rnsp = rnsp.p; a.rk = rk.p;
-    a.rx = rx.p; a.ry = ry.p; a.rz = rz.p; a.rg0 = rg0.p; a.rg1 = rg1.p; a.rg2 = rg2.p; a.rg3 = rg3.p;
+    a.rn = rn.p; a.rnsp = rnsp.p; a.rows = rows.p;
     a.max_count = dmax.p;
     a.mce = mce; a.rnv = split ? rnv.p : nullptr; a.rce2 = rc_e * rc_e;
     a.nn_e4 = nn_e4.p; a.nn_g = nn_g.p; a.nn_ne = nn_ne.p; a.nn_emax = NN_EMAX; a.nn_rg2 = nn_rg * nn_rg;
@@ -610,8 +609,7 @@ struct Engine : EngineBase {
 
   void alloc_rows() {
     ++generation;
-    size_t m = (size_t)nt * mc;
-    rk.alloc(m); rx.alloc(m); ry.alloc(m); rz.alloc(m); rg0.alloc(m); rg1.alloc(m); rg2.alloc(m); rg3.alloc(m);
+    rows.alloc((size_t)nt * (mc / 32) * pgm::RowChunk<T>::SIZE);
   }
 
   // One pass of the FFTs over its groups of systems.

@@ -2,7 +2,7 @@
 //
 // Layout in HBM (all systems of a batch concatenated; a block never straddles two systems):
 //   atoms      SoA per-atom parameters (T) and state; 3-vectors as 16/32-byte v4<T> for single loads
-//   rows       [atom][capacity] structure of arrays: partner k (int32), x, y, z, G0..G3 (T);
+//   rows       [atom][chunk of 32 entries]: partner k (int32), x, y, z, G1, G2, G0, G3 (T), 32 of each (RowChunk);
 //              molecule partners first (the rigid special table), then the in-cutoff neighbours
 //   PME        per system a real grid K1 x K2 x K3 (k3 fastest) and a half-complex grid
 //              K1 x K2 x (K3/2 + 1), both as flat offsets into batch-wide buffers
@@ -59,8 +59,8 @@ struct Dev {
   const int *idx;
   int idx_width;
   // rows
-  int *rn, *rnsp, *rk;
-  T *rx, *ry, *rz, *rg0, *rg1, *rg2, *rg3;
+  int *rn, *rnsp;
+  unsigned char *rows;
   int *max_count;  // [0] largest electrostatic (or only) part, [1] largest van der Waals part
   // split rows: the electrostatic part of a row is [0, mce), the van der Waals part [mce, mc) with
   // its counts in rnv (null: one cutoff, mce == mc); rce2 = elec_cutoff^2
@@ -106,6 +106,29 @@ struct Dev {
   double *forces;
   double4 *dEdd;
 };
+
+// A chunk of 32 row entries: 32 each of k, x, y, z, G1, G2, G0, G3, so that a warp writes or reads
+// every array of a chunk at constant offsets from one address (separate arrays took a 64-bit address each:
+// a third of the row build's instructions) and the sweeps' six arrays are contiguous.
+template <typename T>
+struct RowChunk {
+  static constexpr int SIZE = 32 * (4 + 7 * (int)sizeof(T));
+  static constexpr int X = 128, Y = X + 32 * (int)sizeof(T), Z = Y + 32 * (int)sizeof(T), G1 = Z + 32 * (int)sizeof(T),
+                       G2 = G1 + 32 * (int)sizeof(T), G0 = G2 + 32 * (int)sizeof(T), G3 = G0 + 32 * (int)sizeof(T);
+};
+template <typename T>
+__device__ __forceinline__ unsigned char *row_of(const Dev<T> &a, int i) {
+  return a.rows + (size_t)i * (a.mc >> 5) * RowChunk<T>::SIZE;
+}
+// Entry t of a row: its k (AT = 0) and the T values at RowChunk offset AT.
+template <typename T>
+__device__ __forceinline__ unsigned char *row_entry(unsigned char *row, int t) {
+  return row + (size_t)(t >> 5) * RowChunk<T>::SIZE;
+}
+template <typename T>
+__device__ __forceinline__ int &entry_k(unsigned char *chunk, int t) { return reinterpret_cast<int *>(chunk)[t & 31]; }
+template <typename T, int AT>
+__device__ __forceinline__ T &entry_v(unsigned char *chunk, int t) { return reinterpret_cast<T *>(chunk + AT)[t & 31]; }
 
 // ------------------------------------------------------------------ box and per-atom set-up
 template <typename T>
@@ -410,7 +433,10 @@ __device__ __forceinline__ T group_sum(T v, unsigned m) {
 // nearest integer by adding and subtracting 1.5 2^23 (wrapped positions: |argument| < 2): two
 // additions, where rintf is a conversion at a quarter of their rate.
 __device__ __forceinline__ float nearest_f(float x) { return __fadd_rn(__fadd_rn(x, 12582912.f), -12582912.f); }
-__device__ __forceinline__ void min_image_fast_f(float &x, float &y, float &z, const float *H, const float *id) {
+__device__ __forceinline__ void min_image_scan(double &x, double &y, double &z, const double *H, const double *id) {
+  min_image_fast(x, y, z, H, id);
+}
+__device__ __forceinline__ void min_image_scan(float &x, float &y, float &z, const float *H, const float *id) {
   float n = nearest_f(z * id[2]);
   x -= n * H[6]; y -= n * H[7]; z -= n * H[8];
   n = nearest_f(y * id[1]);
@@ -420,18 +446,32 @@ __device__ __forceinline__ void min_image_fast_f(float &x, float &y, float &z, c
 }
 
 // The row scan of atom i by its warp: the molecule partners (special = true), then the
-// candidates, one entry per lane and round; the index two rounds ahead and the position one round ahead
-// are in flight while the current one is tested (a round that waited for its indices and then for
-// their positions took 1900 cycles on 32 resident warps).  visit(keep, j, x, y, z, special) runs on all lanes every round (it may use the warp's
-// collectives); keep is r < rc for an entry of another atom, false on lanes without one; the displacement
+// candidates, two entries per lane and round; the indices two rounds ahead and the positions one round ahead
+// are in flight while the current ones are tested (a round that waited for its indices and then for
+// their positions took 1900 cycles on 32 resident warps).  visit(keep, j, x, y, z, special) runs on all
+// lanes for every 32 entries (it may use the warp's collectives), then round() after every round; keep is
+// r < rc for an entry of another atom, false on lanes without one; the displacement
 // comes as T, as the rows store it.  Mixed precision: the candidates' FP32 displacements from the wrapped
 // FP32 positions (16-byte gathers), the molecule partners' rounded from FP64.
-template <typename T, typename Visit>
-__device__ __forceinline__ void row_scan(const Dev<T> &a, const SysInfo &S, const BoxInfo &B, int i, int lane, Visit &&visit) {
+template <typename T, typename Visit, typename Round>
+__device__ __forceinline__ void row_scan(const Dev<T> &a, const SysInfo &S, const BoxInfo &B, int i, int lane, Visit &&visit,
+                                         Round &&round) {
   double H[9], id[3];
 #pragma unroll
   for (int k = 0; k < 9; ++k) H[k] = B.H[k];
   id[0] = B.idiag[0]; id[1] = B.idiag[1]; id[2] = B.idiag[2];
+  // the caller's candidate rows (local indices, padding natom), or the engine's Verlet candidates (within
+  // cutoff + skin at the last rebuild)
+  const bool own = a.idx == nullptr;
+  const int *row = own ? a.cand + (size_t)i * a.cc : a.idx + (size_t)i * a.idx_width;
+  const int nc = own ? min(a.ncand[i], a.cc) : a.idx_width;
+  const int first = own ? 0 : S.atom0, limit = own ? a.nt : S.natom;
+  auto index = [&](int c) { return c < nc ? row[c] : -1; };  // as stored: nothing waits for the load here
+  auto partner = [&](int jl) { return jl >= 0 && jl < limit ? jl + first : -1; };
+  constexpr int U = 2;
+  int jn[U], l2[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) { jn[u] = index(32 * u + lane); l2[u] = index(32 * (U + u) + lane); }
   const double4 pi = a.pos4[i];
   const double rc2 = a.cutoff * a.cutoff;
   const int mf = a.molfirst[i], me = a.molend[i];
@@ -446,66 +486,48 @@ __device__ __forceinline__ void row_scan(const Dev<T> &a, const SysInfo &S, cons
       keep = x * x + y * y + z * z < rc2;
     }
     visit(keep, j, T(x), T(y), T(z), true);
+    round();
   }
-  // the caller's candidate rows (local indices, padding natom), or the engine's Verlet candidates (within
-  // cutoff + skin at the last rebuild)
-  const bool own = a.idx == nullptr;
-  const int *row = own ? a.cand + (size_t)i * a.cc : a.idx + (size_t)i * a.idx_width;
-  const int nc = own ? min(a.ncand[i], a.cc) : a.idx_width;
-  const int first = own ? 0 : S.atom0, limit = own ? a.nt : S.natom;
-  auto index = [&](int c) { return c < nc ? row[c] : -1; };  // as stored: nothing waits for the load here
-  auto partner = [&](int jl) { return jl >= 0 && jl < limit ? jl + first : -1; };
-  // indices two rounds ahead and positions one round ahead are in flight
-  int l2 = index(32 + lane);
-  int jn = partner(index(lane));
-  if constexpr (sizeof(T) == 4) {
-    float Hf[9], idf[3];
+  // positions in the scan's precision, .w the molecule
+  const v4<T> *pos;
+  T Ht[9], idt[3];
+  if constexpr (sizeof(T) == 4) pos = a.pos4f;
+  else pos = a.pos4;
 #pragma unroll
-    for (int k = 0; k < 9; ++k) Hf[k] = float(H[k]);
-    idf[0] = float(id[0]); idf[1] = float(id[1]); idf[2] = float(id[2]);
-    const float4 pf = a.pos4f[i];
-    const float rc2f = float(rc2);
-    float4 pn = jn >= 0 ? a.pos4f[jn] : pf;
-    for (int c0 = 0; c0 < nc; c0 += 32) {
-      const int j = jn;
-      const float4 pj = pn;
-      jn = partner(l2);
-      l2 = index(c0 + 64 + lane);
-      if (jn >= 0) pn = a.pos4f[jn];
-      bool keep = false;
-      float x = 0.f, y = 0.f, z = 0.f;
-      if (j >= 0 && pj.w != pf.w) {
-        x = pf.x - pj.x; y = pf.y - pj.y; z = pf.z - pj.z;
-        min_image_fast_f(x, y, z, Hf, idf);
-        keep = x * x + y * y + z * z < rc2f;
-      }
-      visit(keep, j, x, y, z, false);
+  for (int k = 0; k < 9; ++k) Ht[k] = T(H[k]);
+  idt[0] = T(id[0]); idt[1] = T(id[1]); idt[2] = T(id[2]);
+  const v4<T> p0 = pos[i];
+  const T rc2t = T(rc2);
+  v4<T> pn[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) { jn[u] = partner(jn[u]); pn[u] = pos[jn[u] >= 0 ? jn[u] : i]; }
+  for (int c0 = 0; c0 < nc; c0 += 32 * U) {
+    int j[U];
+    v4<T> pj[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      j[u] = jn[u];
+      pj[u] = pn[u];
+      jn[u] = partner(l2[u]);
+      l2[u] = index(c0 + 32 * (2 * U + u) + lane);
+      pn[u] = pos[jn[u] >= 0 ? jn[u] : i];
     }
-  } else {
-    double4 pn = jn >= 0 ? a.pos4[jn] : pi;
-    for (int c0 = 0; c0 < nc; c0 += 32) {
-      const int j = jn;
-      const double4 pj = pn;
-      jn = partner(l2);
-      l2 = index(c0 + 64 + lane);
-      if (jn >= 0) pn = a.pos4[jn];
-      bool keep = false;
-      double x = 0, y = 0, z = 0;
-      if (j >= 0 && pj.w != pi.w) {
-        x = pi.x - pj.x; y = pi.y - pj.y; z = pi.z - pj.z;
-        min_image_fast(x, y, z, H, id);
-        keep = x * x + y * y + z * z < rc2;
-      }
-      visit(keep, j, x, y, z, false);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      T x = p0.x - pj[u].x, y = p0.y - pj[u].y, z = p0.z - pj[u].z;
+      min_image_scan(x, y, z, Ht, idt);
+      // a lane without a candidate holds atom i itself: its own molecule
+      visit(j[u] >= 0 && pj[u].w != p0.w && x * x + y * y + z * z < rc2t, j[u], x, y, z, false);
     }
+    round();
   }
 }
 
-// Kept entries waiting for their evaluation (ring; at most 63 at a time).
+// Kept entries waiting for their evaluation (ring; at most 95 at a time: 31 and a round's 64).
 template <typename T>
 struct RowQueue {
-  int j[64];
-  T x[64], y[64], z[64];
+  int j[128];
+  T x[128], y[128], z[128];
 };
 
 template <typename T>
@@ -520,10 +542,10 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_rows(Dev<T> a) 
   RowQueue<T> &q = queues[warp];
   const unsigned lt = (1u << lane) - 1u;
   const T Ri2 = T(2) * a.radius[i] * a.radius[i], beta = T(a.beta);
-  const size_t base = (size_t)i * a.mc;
+  unsigned char *row = row_of(a, i);
   int head = 0, tail = 0, ecount = 0, vcount = 0, scount = 0, nsp = 0;  // head: evaluated, tail: found
   auto evaluate = [&](int n) {  // the next n <= 32 entries of the queue, to row slots head .. head + n - 1
-    const int w = (head + lane) & 63, slot = head + lane;
+    const int w = (head + lane) & 127, slot = head + lane;
     const bool in = lane < n && slot < a.mce;
     const int j = in ? q.j[w] : i;
     const T x = q.x[w], y = q.y[w], z = q.z[w];
@@ -546,12 +568,14 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_rows(Dev<T> a) 
       ed = ed && at_e < a.nn_emax;
     }
     if (in) {
-      const size_t o = base + slot;
-      a.rk[o] = j;
-      a.rx[o] = x; a.ry[o] = y; a.rz[o] = z;
+      using C = RowChunk<T>;
+      unsigned char *chunk = row_entry<T>(row, head);  // head is a multiple of 32
+      entry_k<T>(chunk, lane) = j;
+      entry_v<T, C::X>(chunk, lane) = x; entry_v<T, C::Y>(chunk, lane) = y; entry_v<T, C::Z>(chunk, lane) = z;
       T g[4];
       pair_kernels<T>(Ri2 + T(2) * Rk * Rk, beta, r2, g);
-      a.rg0[o] = g[0]; a.rg1[o] = g[1]; a.rg2[o] = g[2]; a.rg3[o] = g[3];
+      entry_v<T, C::G1>(chunk, lane) = g[1]; entry_v<T, C::G2>(chunk, lane) = g[2];
+      entry_v<T, C::G0>(chunk, lane) = g[0]; entry_v<T, C::G3>(chunk, lane) = g[3];
       if (sh) {
         const size_t c = (size_t)at_s * a.nt + i;
         a.c_k[c] = j;
@@ -576,25 +600,27 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_rows(Dev<T> a) 
       const unsigned bv = __ballot_sync(0xffffffffu, kv);
       const int sv = vcount + __popc(bv & lt);
       if (kv && sv < a.mc - a.mce) {
-        const size_t o = base + a.mce + sv;
-        a.rk[o] = j;
-        a.rx[o] = x; a.ry[o] = y; a.rz[o] = z;
+        using C = RowChunk<T>;
+        const int t = a.mce + sv;
+        unsigned char *chunk = row_entry<T>(row, t);
+        entry_k<T>(chunk, t) = j;
+        entry_v<T, C::X>(chunk, t) = x; entry_v<T, C::Y>(chunk, t) = y; entry_v<T, C::Z>(chunk, t) = z;
       }
       vcount += __popc(bv);
     }
     const unsigned bal = __ballot_sync(0xffffffffu, keep);
     if (keep) {
-      const int w = (tail + __popc(bal & lt)) & 63;
+      const int w = (tail + __popc(bal & lt)) & 127;
       q.j[w] = j;
       q.x[w] = x; q.y[w] = y; q.z[w] = z;
     }
     tail += __popc(bal);
     if (special) nsp = tail;
-    if (tail - head >= 32) {
-      __syncwarp();  // the queue's entries, stored by other lanes
-      evaluate(32);
-      __syncwarp();  // read before their slots are filled again
-    }
+  }, [&] {
+    if (tail - head < 32) return;
+    __syncwarp();  // the queue's entries, stored by other lanes
+    do evaluate(32); while (tail - head >= 32);
+    __syncwarp();  // read before their slots are filled again
   });
   __syncwarp();
   if (tail > head) evaluate(tail - head);
@@ -826,7 +852,8 @@ __global__ void __launch_bounds__(8 * LPR) k_rowfield(Dev<T> a, const v4<T> *__r
   const bool valid = i < S.atom0 + S.natom;
   if (LPR == 32 && !valid) continue;  // uniform over the warp
   int n = valid ? min(a.rn[i], a.mce) : 0;
-  size_t base = (size_t)(valid ? i : 0) * a.mc;
+  unsigned char *row = row_of(a, valid ? i : 0);
+  using C = RowChunk<T>;
   T f0 = 0, f1 = 0, f2 = 0;
   auto pair = [&](int k, T x, T y, T z, T g1, T g2) {
     v4<T> dk = D[k];
@@ -838,26 +865,27 @@ __global__ void __launch_bounds__(8 * LPR) k_rowfield(Dev<T> a, const v4<T> *__r
     f2 += c * z + g1 * dk.z;
   };
   if constexpr (sizeof(T) == 4) {
-    const int4 *k4 = reinterpret_cast<const int4 *>(a.rk + base);
-    const float4 *x4 = reinterpret_cast<const float4 *>(a.rx + base), *y4 = reinterpret_cast<const float4 *>(a.ry + base),
-                 *z4 = reinterpret_cast<const float4 *>(a.rz + base), *p4 = reinterpret_cast<const float4 *>(a.rg1 + base),
-                 *q4 = reinterpret_cast<const float4 *>(a.rg2 + base);
     // streaming loads (evict first): the 90+ MB of rows pass through L2 once per sweep and must
     // not push out the PME grids that the FFT passes read next.  The next group of four entries
     // is loaded before the current one is used (two groups of row data in flight per lane).
+    // Eight lanes cover a chunk, so a lane steps by whole chunks from one address.
+    const unsigned char *at = row + (lane >> 3) * C::SIZE + (lane & 7) * 16;
+    constexpr int STEP = LPR / 8 * C::SIZE;
+    auto v4at = [](const unsigned char *p) { return __ldcs(reinterpret_cast<const float4 *>(p)); };
     int4 kk = make_int4(0, 0, 0, 0);
     float4 xx = make_float4(0, 0, 0, 0), yy = xx, zz = xx, g1 = xx, g2 = xx;
     if (4 * lane < n) {
-      kk = __ldcs(k4 + lane);
-      xx = __ldcs(x4 + lane); yy = __ldcs(y4 + lane); zz = __ldcs(z4 + lane); g1 = __ldcs(p4 + lane); g2 = __ldcs(q4 + lane);
+      kk = __ldcs(reinterpret_cast<const int4 *>(at));
+      xx = v4at(at + C::X); yy = v4at(at + C::Y); zz = v4at(at + C::Z); g1 = v4at(at + C::G1); g2 = v4at(at + C::G2);
     }
     for (int t4 = lane; 4 * t4 < n; t4 += LPR) {
       const int t4n = t4 + LPR;
+      at += STEP;
       int4 kn = make_int4(0, 0, 0, 0);
       float4 xn = make_float4(0, 0, 0, 0), yn = xn, zn = xn, g1n = xn, g2n = xn;
       if (4 * t4n < n) {
-        kn = __ldcs(k4 + t4n);
-        xn = __ldcs(x4 + t4n); yn = __ldcs(y4 + t4n); zn = __ldcs(z4 + t4n); g1n = __ldcs(p4 + t4n); g2n = __ldcs(q4 + t4n);
+        kn = __ldcs(reinterpret_cast<const int4 *>(at));
+        xn = v4at(at + C::X); yn = v4at(at + C::Y); zn = v4at(at + C::Z); g1n = v4at(at + C::G1); g2n = v4at(at + C::G2);
       }
       int t = 4 * t4;
       pair(kk.x, xx.x, yy.x, zz.x, g1.x, g2.x);
@@ -868,8 +896,9 @@ __global__ void __launch_bounds__(8 * LPR) k_rowfield(Dev<T> a, const v4<T> *__r
     }
   } else {
     for (int t = lane; t < n; t += LPR) {
-      size_t o = base + t;
-      pair(a.rk[o], a.rx[o], a.ry[o], a.rz[o], a.rg1[o], a.rg2[o]);
+      unsigned char *c = row_entry<T>(row, t);
+      pair(entry_k<T>(c, t), entry_v<T, C::X>(c, t), entry_v<T, C::Y>(c, t), entry_v<T, C::Z>(c, t), entry_v<T, C::G1>(c, t),
+           entry_v<T, C::G2>(c, t));
     }
   }
   // every lane of the warp takes part in the butterfly (a row past the system's end adds zeros)
@@ -1846,13 +1875,15 @@ __device__ void iel_block_solve(const Dev<T> &a, int i0, int nb, double (*M)[25]
     const double rr[3] = {double(r.x), double(r.y), double(r.z)};
     for (int c = 0; c < 3; ++c) { M[3 * li + c][3 * li + c] += ia; M[3 * li + c][N] = rr[c]; }
     const int nsp = a.rnsp[i];  // molecule partners first in every row
-    const size_t base = (size_t)i * a.mc;
+    using C = RowChunk<T>;
+    unsigned char *row = row_of(a, i);
     for (int t = 0; t < nsp; ++t) {
-      const int k = a.rk[base + t];
+      unsigned char *c = row_entry<T>(row, t);
+      const int k = entry_k<T>(c, t);
       const int lk = k - i0;
       if (lk < 0 || lk >= nb) continue;
-      const double x[3] = {double(a.rx[base + t]), double(a.ry[base + t]), double(a.rz[base + t])};
-      const double g1 = double(a.rg1[base + t]), g2 = double(a.rg2[base + t]);
+      const double x[3] = {double(entry_v<T, C::X>(c, t)), double(entry_v<T, C::Y>(c, t)), double(entry_v<T, C::Z>(c, t))};
+      const double g1 = double(entry_v<T, C::G1>(c, t)), g2 = double(entry_v<T, C::G2>(c, t));
       for (int u = 0; u < 3; ++u)
         for (int v = 0; v < 3; ++v) M[3 * li + u][3 * lk + v] += (u == v ? g1 : 0.0) - g2 * x[u] * x[v];
     }
@@ -2014,7 +2045,8 @@ __global__ void __launch_bounds__(ATOMS_PER_BLOCK * QL, MINB) k_forces(Dev<T> a,
     v4<T> di = a.D[i];
     T qi = a.q[i], rhi = a.rminh[i], sei = a.seps[i];
     int n = min(a.rn[i], a.mce), nsp = a.rnsp[i];
-    size_t base = (size_t)i * a.mc;
+    unsigned char *row = row_of(a, i);
+    using C = RowChunk<T>;
     T gx0 = 0, gx1 = 0, gx2 = 0, gl0 = 0, gl1 = 0, gl2 = 0, fd0 = 0, fd1 = 0, fd2 = 0;
     T ee = 0, el = 0;
     T w[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
@@ -2152,17 +2184,14 @@ __global__ void __launch_bounds__(ATOMS_PER_BLOCK * QL, MINB) k_forces(Dev<T> a,
       w[6] += kz * x; w[7] += kz * y; w[8] += kz * z;
     };
     if constexpr (sizeof(T) == 4) {
-      // 16-byte loads of four consecutive entries of every row array
-      const int4 *k4 = reinterpret_cast<const int4 *>(a.rk + base);
-      const float4 *x4 = reinterpret_cast<const float4 *>(a.rx + base), *y4 = reinterpret_cast<const float4 *>(a.ry + base),
-                   *z4 = reinterpret_cast<const float4 *>(a.rz + base), *h0 = reinterpret_cast<const float4 *>(a.rg0 + base),
-                   *h1 = reinterpret_cast<const float4 *>(a.rg1 + base), *h2 = reinterpret_cast<const float4 *>(a.rg2 + base),
-                   *h3 = reinterpret_cast<const float4 *>(a.rg3 + base);
-      for (int t4 = lane; 4 * t4 < n; t4 += QL) {
-        int4 kk = __ldcs(k4 + t4);
-        float4 xx = __ldcs(x4 + t4), yy = __ldcs(y4 + t4), zz = __ldcs(z4 + t4);
-        float4 a0 = __ldcs(h0 + t4), a1 = __ldcs(h1 + t4), a2 = __ldcs(h2 + t4), a3 = __ldcs(h3 + t4);
-        int t = 4 * t4;
+      // 16-byte loads of four consecutive entries of every row array: a chunk per round
+      static_assert(QL == 8, "eight lanes cover a chunk");
+      const unsigned char *at = row + lane * 16;
+      auto v4at = [](const unsigned char *p) { return __ldcs(reinterpret_cast<const float4 *>(p)); };
+      for (int t = 4 * lane; t < n; t += 32, at += C::SIZE) {
+        const int4 kk = __ldcs(reinterpret_cast<const int4 *>(at));
+        const float4 xx = v4at(at + C::X), yy = v4at(at + C::Y), zz = v4at(at + C::Z);
+        const float4 a1 = v4at(at + C::G1), a2 = v4at(at + C::G2), a0 = v4at(at + C::G0), a3 = v4at(at + C::G3);
         pair(kk.x, xx.x, yy.x, zz.x, a0.x, a1.x, a2.x, a3.x, t);
         if (t + 1 < n) pair(kk.y, xx.y, yy.y, zz.y, a0.y, a1.y, a2.y, a3.y, t + 1);
         if (t + 2 < n) pair(kk.z, xx.z, yy.z, zz.z, a0.z, a1.z, a2.z, a3.z, t + 2);
@@ -2170,16 +2199,18 @@ __global__ void __launch_bounds__(ATOMS_PER_BLOCK * QL, MINB) k_forces(Dev<T> a,
       }
     } else {
       for (int t = lane; t < n; t += QL) {
-        size_t o = base + t;
-        pair(a.rk[o], a.rx[o], a.ry[o], a.rz[o], a.rg0[o], a.rg1[o], a.rg2[o], a.rg3[o], t);
+        unsigned char *c = row_entry<T>(row, t);
+        pair(entry_k<T>(c, t), entry_v<T, C::X>(c, t), entry_v<T, C::Y>(c, t), entry_v<T, C::Z>(c, t), entry_v<T, C::G0>(c, t),
+             entry_v<T, C::G1>(c, t), entry_v<T, C::G2>(c, t), entry_v<T, C::G3>(c, t), t);
       }
     }
     if (a.rnv) {  // split rows: the LJ pairs between elec_cutoff and cutoff
       const int nv = min(a.rnv[i], a.mc - a.mce);
       for (int t = lane; t < nv; t += QL) {
-        size_t o = base + a.mce + t;
-        int k = a.rk[o];
-        T x = a.rx[o], y = a.ry[o], z = a.rz[o];
+        const int e = a.mce + t;
+        unsigned char *c = row_entry<T>(row, e);
+        const int k = entry_k<T>(c, e);
+        const T x = entry_v<T, C::X>(c, e), y = entry_v<T, C::Y>(c, e), z = entry_v<T, C::Z>(c, e);
         T rm = rhi + a.rminh[k], ep = sei * a.seps[k];
         T r2 = x * x + y * y + z * z;
         const T ir2 = T(1) / r2;
