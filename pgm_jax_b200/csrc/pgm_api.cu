@@ -1003,21 +1003,16 @@ struct Engine : EngineBase {
   }
 
   void prepare(cudaStream_t st, pgm::Dev<T> &a, const double *boxes, const double *nn_hist = nullptr) {
-    launch_pdl(pgm::k_box<T>, grid1(nsys, 64), 64, 0, st, a, boxes);
-    launch_pdl(pgm::k_prep<T>, grid1(nt), 256, 0, st, a);
-    launch_pdl(pgm::k_mol<T>, grid1(nmol_total), 256, 0, st, a);
+    launch_pdl(pgm::k_prep<T>, ntblk, 256, 0, st, a, boxes);
     if (!a.idx) {  // the Verlet candidate list, rebuilt on the device when the flag is up
       launch_pdl(pgm::k_cell_assign<T>, grid1(nt), 256, 0, st, a);
-      launch_pdl(pgm::k_scan_cells, 1, 1024, 0, st, (const int *)cell_count.p, cell_start.p, ncell, (const int *)nb_flag.p);
+      launch_pdl(pgm::k_scan_cells, 1, 1024, 0, st, cell_count.p, cell_start.p, ncell, (const int *)nb_flag.p);
       launch_pdl(pgm::k_scatter<T>, grid1(nt), 256, 0, st, a);
       launch_pdl(pgm::k_cand<T>, nwblk, 256, 0, st, a);
-      launch_pdl(pgm::k_nb_finish, std::max(1, std::min(1024, grid1(ncell))), 256, 0, st, cell_count.p, ncell, nb_flag.p,
-                 nb_builds.p);
-      launch_pdl(pgm::k_nb_lower, 1, 1, 0, st, nb_flag.p, nb_builds.p);
     }
     launch_pdl(pgm::k_rows<T>, nwblk, 256, 0, st, a);
     if (nn_hist) nn_fork(st, a, nn_hist);
-    launch_pdl(pgm::k_influence<T>, (int)std::min<long long>(4096, (cgrid + 255) / 256), 256, 0, st, a, (long long)cgrid);
+    launch_pdl(pgm::k_influence<T>, (int)std::min<long long>(8 * nsm, (cgrid + 255) / 256), 256, 0, st, a, (long long)cgrid);
   }
 
   void set_list_capacity(int c) override {
@@ -1088,23 +1083,24 @@ struct Engine : EngineBase {
     launch_pdl(pgm::k_gather<T, P, MODE, ACT>, nqblk, QT, 0, st, a, vin, out);
   }
 
+  // What the solve's kernels need to evaluate a start (cg_begin) or an iteration's check.
+  pgm::BeginArgs begin_args(double fb_factor = 0.0, cudaGraphConditionalHandle fbcond = 0, int use_fbcond = 0, int *fb_any = nullptr) {
+    return pgm::BeginArgs{d_cg.p, nsys, set.dipole_tol, set.max_iter, dany.p, fb_factor, fbcond, use_fbcond, fb_any, cg_done.p};
+  }
+
   // The local preconditioner's chain z = M^-1 r (k_lp_start, then per inner iteration k_lp_ap and
   // k_lp_step), for the systems ACT selects (0 all, 1 iterating, 3 falling back); MODE 0 ends with
-  // p = z and r.z (a start), MODE 1 with the outer CG's check (an iteration).
+  // p = z, r.z and the start's scalars, MODE 1 with the outer CG's check (an iteration).
   template <int ACT, int MODE>
-  void local_precond(cudaStream_t st, pgm::Dev<T> &a, cudaGraphConditionalHandle cond, int use_cond) {
+  void local_precond(cudaStream_t st, pgm::Dev<T> &a, const pgm::BeginArgs &b, cudaGraphConditionalHandle cond, int use_cond) {
     const int L = set.local_niter;
     launch_pdl(pgm::k_lp_start<T, ACT>, ntblk, 256, 0, st, a);
     for (int j = 1; j <= L; ++j) {
       pgm::v4<T> *cur = (j & 1) ? LP0.p : LP1.p, *prev = (j & 1) ? LP1.p : LP0.p;
       if (j == 1) launch_pdl(pgm::k_lp_ap<T, ACT, true>, ntblk, 256, 0, st, a, (const pgm::v4<T> *)prev, cur);
       else launch_pdl(pgm::k_lp_ap<T, ACT, false>, ntblk, 256, 0, st, a, (const pgm::v4<T> *)prev, cur);
-      if (j < L)
-        launch_pdl(pgm::k_lp_step<T, ACT, false, MODE>, ntblk, 256, 0, st, a, (const pgm::v4<T> *)cur, nsys, set.dipole_tol,
-                   set.max_iter, dany.p, cond, use_cond, cg_done.p);
-      else
-        launch_pdl(pgm::k_lp_step<T, ACT, true, MODE>, ntblk, 256, 0, st, a, (const pgm::v4<T> *)cur, nsys, set.dipole_tol,
-                   set.max_iter, dany.p, cond, use_cond, cg_done.p);
+      if (j < L) launch_pdl(pgm::k_lp_step<T, ACT, false, MODE>, ntblk, 256, 0, st, a, (const pgm::v4<T> *)cur, b, cond, use_cond);
+      else launch_pdl(pgm::k_lp_step<T, ACT, true, MODE>, ntblk, 256, 0, st, a, (const pgm::v4<T> *)cur, b, cond, use_cond);
     }
   }
 
@@ -1114,7 +1110,7 @@ struct Engine : EngineBase {
     sweep<false, true, 1, 1>(st, a, Pv.p, AP.p);
     if (set.local_niter > 0) {
       launch_pdl(pgm::k_cg_update_r<T>, ntblk, 256, 0, st, a);
-      local_precond<1, 1>(st, a, cond, use_cond);
+      local_precond<1, 1>(st, a, begin_args(), cond, use_cond);
       return;
     }
     launch_pdl(pgm::k_cg_update_check<T>, ntblk, 256, 0, st, a, nsys, set.dipole_tol, set.max_iter, dany.p, cond, use_cond,
@@ -1177,9 +1173,9 @@ struct Engine : EngineBase {
     CK(cudaStreamIsCapturing(st, &cs));
     const bool captured = cs == cudaStreamCaptureStatusActive;
     // captured: the plain start's second sweep sits in a conditional IF node whose condition
-    // k_cg_setup raises when some system takes the plain start (else the node's kernels are skipped)
+    // k_start1 raises when some system takes the plain start (else the node's kernels are skipped)
     // the learned guess's check: its start residual against the record of the extrapolation's
-    // (k_cg_begin); a fallback restarts those systems from x4 with one operator sweep, captured in
+    // (cg_begin); a fallback restarts those systems from x4 with one operator sweep, captured in
     // a conditional IF node that runs only when some system falls back
     const bool check_nn = use_nn && nn_fb_factor > 0.0;
     cudaGraphConditionalHandle cond2 = 0, condfb = 0;
@@ -1192,13 +1188,11 @@ struct Engine : EngineBase {
       CK(cudaGraphConditionalHandleCreate(&cond2, g, 0, cudaGraphCondAssignDefault));
       if (check_nn) CK(cudaGraphConditionalHandleCreate(&condfb, g, 0, cudaGraphCondAssignDefault));
     }
-    launch_pdl(pgm::k_cg_setup, grid1(nsys, 64), 64, 0, st, d_cg.p, nsys, mode == 0 ? (const int32_t *)ind->count : nullptr,
-               (const double *)ind->norm, mode == 0 ? K : 0, set.fused, std::max(1, set.norm_refresh), mode, cond2, captured ? 1 : 0,
-               use_nn ? 1 : 0);
+    const pgm::StartRule rule{mode == 0 ? K : 0, set.fused, std::max(1, set.norm_refresh), mode, use_nn ? 1 : 0,
+                              mode == 0 ? (const int32_t *)ind->count : nullptr, (const double *)ind->norm};
     if (mode == 1) {
       // x0 = ind->mu with the plain start: X = mu, have = 1
-      pgm::k_energy_start<T><<<grid1(nt), 256, 0, st>>>(a, ind->mu);
-      check_launch();
+      launch_pdl(pgm::k_energy_start<T>, grid1(nt), 256, 0, st, a, rule, (const double *)ind->mu, cond2, captured ? 1 : 0);
     } else {
       last_hist = ind->hist;
       if (use_nn && !nn_forked) nn_fork(st, a, ind->hist);
@@ -1206,37 +1200,37 @@ struct Engine : EngineBase {
         CK(cudaStreamWaitEvent(st, ev_nn_join, 0));  // the prediction, computed beside the row build
         nn_forked = false;
       }
-      launch_pdl(pgm::k_start1<T>, grid1(nt), 256, 0, st, a, (const double *)ind->hist, K, cc[0], cc[1], cc[2], cc[3],
-                 use_nn ? (const float *)nn_mu.p : nullptr);
+      launch_pdl(pgm::k_start1<T>, grid1(nt), 256, 0, st, a, rule, (const double *)ind->hist, cc[0], cc[1], cc[2], cc[3],
+                 use_nn ? (const float *)nn_mu.p : nullptr, cond2, captured ? 1 : 0);
     }
     sweep<true, false, 0, 0>(st, a, D.p, Bv.p);
-    launch_pdl(pgm::k_start2<T>, ntblk, 256, 0, st, a);
+    // the fused systems' start ends with k_start2, the plain ones' in their conditional node; with the local
+    // preconditioner both end with its chain
+    const bool local = set.local_niter > 0;
+    const double fb_factor = mode == 0 && set.predictor == 5 ? nn_fb_factor : 0.0;
+    const pgm::BeginArgs begin = begin_args(fb_factor, condfb, captured && check_nn ? 1 : 0, dfb.p);
+    if (local) launch_pdl(pgm::k_start2<T, true>, ntblk, 256, 0, st, a, begin);
+    else launch_pdl(pgm::k_start2<T, false>, ntblk, 256, 0, st, a, begin);
     auto plain_start = [&](cudaStream_t s2) {
       sweep<false, false, 2, 1>(s2, a, X.p, AP.p);
       launch_pdl(pgm::k_start3<T>, grid1(nt), 256, 0, s2, a);
+      if (local) launch_pdl(pgm::k_cg_init<T, false, true>, ntblk, 256, 0, s2, a, (const float *)nullptr, begin);
+      else launch_pdl(pgm::k_cg_init<T, false, false>, ntblk, 256, 0, s2, a, (const float *)nullptr, begin);
     };
     if (captured) conditional_node(st, cond2, cudaGraphCondTypeIf, plain_start);
     else plain_start(st);
-    if (set.local_niter > 0) {
-      pgm::k_cg_init<T, false, true><<<ntblk, 256, 0, st>>>(a); check_launch();
-      local_precond<0, 0>(st, a, 0, 0);
-    } else {
-      pgm::k_cg_init<T><<<ntblk, 256, 0, st>>>(a); check_launch();
-    }
-    launch_pdl(pgm::k_cg_begin, 1, 256, 0, st, d_cg.p, nsys, set.dipole_tol, set.max_iter, dany.p,
-               mode == 0 && set.predictor == 5 ? nn_fb_factor : 0.0, 0, condfb, captured && check_nn ? 1 : 0, dfb.p);
+    if (local) local_precond<0, 0>(st, a, begin, 0, 0);
     if (check_nn) {
       auto fallback = [&](cudaStream_t s2) {
         launch_pdl(pgm::k_fb_prep<T>, grid1(nt), 256, 0, s2, a, (const float *)nn_mu.p);
         sweep<false, false, 3, 1>(s2, a, D.p, AP.p);  // A delta
-        if (set.local_niter > 0) {
-          launch_pdl(pgm::k_cg_init<T, true, true>, ntblk, 256, 0, s2, a, (const float *)nn_mu.p);
-          local_precond<3, 0>(s2, a, 0, 0);
+        const pgm::BeginArgs again = begin_args(nn_fb_factor);
+        if (local) {
+          launch_pdl(pgm::k_cg_init<T, true, true>, ntblk, 256, 0, s2, a, (const float *)nn_mu.p, again);
+          local_precond<3, 0>(s2, a, again, 0, 0);
         } else {
-          launch_pdl(pgm::k_cg_init<T, true>, ntblk, 256, 0, s2, a, (const float *)nn_mu.p);
+          launch_pdl(pgm::k_cg_init<T, true, false>, ntblk, 256, 0, s2, a, (const float *)nn_mu.p, again);
         }
-        launch_pdl(pgm::k_cg_begin, 1, 256, 0, s2, d_cg.p, nsys, set.dipole_tol, set.max_iter, dany.p, nn_fb_factor, 1,
-                   condfb, 0, (int *)nullptr);
       };
       if (captured) {
         conditional_node(st, condfb, cudaGraphCondTypeIf, fallback);
@@ -1278,14 +1272,15 @@ struct Engine : EngineBase {
       }
       last_iters = it;
     }
-    launch_pdl(pgm::k_cg_finish<T>, grid1(nt), 256, 0, st, a, mu_out, mode == 0 ? ind->hist : nullptr, mode == 0 ? 1 : 0);
-    launch_pdl(pgm::k_cg_state_out, grid1(nsys, 64), 64, 0, st, (const pgm::CGSys *)d_cg.p, nsys, ind->count, ind->norm, iters,
-               resid, a.status, mode == 0 ? 1 : 0, set.dipole_tol);
+    const int push = mode == 0 ? 1 : 0;
+    launch_pdl(pgm::k_cg_finish<T>, grid1(nt), 256, 0, st, a, mu_out, push ? ind->hist : nullptr, push,
+               pgm::StateOut{ind->count, ind->norm, iters, resid, a.status, push, set.dipole_tol});
   }
 
-  // Energies, forces and virial at fixed mu (forcefield.py:2362-2430).
-  void energy_pass(cudaStream_t st, pgm::Dev<T> &a, const double *mu, double *energy, double *virial, bool shadow = false) {
-    launch_pdl(pgm::k_total_dipoles<T>, grid1(nt), 256, 0, st, a, mu);
+  // Energies, forces and virial at fixed mu (forcefield.py:2362-2430); solved: k_cg_finish has left the total
+  // dipoles and the zero accumulators.
+  void energy_pass(cudaStream_t st, pgm::Dev<T> &a, const double *mu, double *energy, double *virial, bool solved, bool shadow = false) {
+    if (!solved) launch_pdl(pgm::k_total_dipoles<T>, grid1(nt), 256, 0, st, a, mu);
     if (shadow) {
       // the reciprocal energy and potential of delta alone (zero outside extended steps), into
       // Phi2 and the second accumulators
@@ -1297,11 +1292,8 @@ struct Engine : EngineBase {
     }
     pme<true, false, 0, true>(st, a, D.p);
     forces_pass(st, a, mu, true, 0, shadow);
-    if (ncov) launch_pdl(pgm::k_cov_forces<T>, grid1(ncov), 256, 0, st, a);
-    launch_pdl(pgm::k_energy_finish, grid1(nsys, 64), 64, 0, st, (const pgm::SysInfo *)d_sys.p, (const pgm::BoxInfo *)d_box.p,
-               (const pgm::EnergyAcc *)d_eacc.p, nsys, set.ewald_beta, a.c_self, set.cutoff, set.vdw == 1, set.lj_lrc, a.induce, energy,
-               virial, a.status, shadow ? (const pgm::EnergyAcc *)d_eacc2.p : (const pgm::EnergyAcc *)nullptr,
-               set.iel_omega > 0 ? set.iel_omega : 1.0);
+    launch_pdl(pgm::k_finish<T>, std::max(1, grid1(ncov)), 256, 0, st, a, energy, virial,
+               shadow ? (const pgm::EnergyAcc *)d_eacc2.p : (const pgm::EnergyAcc *)nullptr, set.iel_omega > 0 ? set.iel_omega : 1.0);
   }
 
   // The extended-Lagrangian step (forcefield.py:1558-1650) on the solver's kernels: per system a
@@ -1327,16 +1319,15 @@ struct Engine : EngineBase {
                (const double *)ind->norm, (const double *)ind->mu, iel_warmup, set.iel, set.iel_iter, cond2, captured ? 1 : 0);
     launch_pdl(pgm::k_iel_start1<T>, grid1(nt), 256, 0, st, a, (const double *)ind->xl, (const double *)ind->mu);
     sweep<true, false, 0, 0>(st, a, D.p, Bv.p);
-    launch_pdl(pgm::k_start2<T>, ntblk, 256, 0, st, a);
+    const pgm::BeginArgs begin = begin_args();
+    launch_pdl(pgm::k_start2<T, false>, ntblk, 256, 0, st, a, begin);
     auto plain_start = [&](cudaStream_t s2) {
       sweep<false, false, 2, 1>(s2, a, X.p, AP.p);
       launch_pdl(pgm::k_start3<T>, grid1(nt), 256, 0, s2, a);
+      launch_pdl(pgm::k_cg_init<T, false, false>, ntblk, 256, 0, s2, a, (const float *)nullptr, begin);
     };
     if (captured) conditional_node(st, cond2, cudaGraphCondTypeIf, plain_start);
     else plain_start(st);
-    pgm::k_cg_init<T><<<ntblk, 256, 0, st>>>(a); check_launch();
-    launch_pdl(pgm::k_cg_begin, 1, 256, 0, st, d_cg.p, nsys, set.dipole_tol, set.max_iter, dany.p, 0.0, 0,
-               (cudaGraphConditionalHandle)0, 0, (int *)nullptr);
     if (set.iel == 1) {
       const double om = set.iel_omega > 0 ? set.iel_omega : 1.0;
       launch_pdl(pgm::k_iel_delta<T>, grid1(nmol_total, 128), 128, 0, st, a, (const double *)ind->xl, om,
@@ -1364,8 +1355,8 @@ struct Engine : EngineBase {
       last_iters = it;
     }
     launch_pdl(pgm::k_iel_finish<T>, grid1(nt), 256, 0, st, a, mu_out, ind->hist, ind->xl, iel_co);
-    launch_pdl(pgm::k_cg_state_out, grid1(nsys, 64), 64, 0, st, (const pgm::CGSys *)d_cg.p, nsys, ind->count, ind->norm, iters,
-               resid, a.status, 1, set.dipole_tol);
+    launch_pdl(pgm::k_cg_state_out, grid1(nsys, 64), 64, 0, st, (const pgm::CGSys *)d_cg.p, nsys,
+               pgm::StateOut{ind->count, ind->norm, iters, resid, a.status, 1, set.dipole_tol});
   }
 
   void compute(cudaStream_t st, const double *pos, const double *box, const int32_t *idx, int idx_width, PgmInduction *ind,
@@ -1373,7 +1364,7 @@ struct Engine : EngineBase {
     launches = 0;
     unsigned *status = out->status ? out->status : d_status.p;
     double *forces = out->forces ? out->forces : forces_tmp.p;
-    pgm::Dev<T> a = dev(pos, idx, idx_width, forces, status);  // k_box zeroes the status words
+    pgm::Dev<T> a = dev(pos, idx, idx_width, forces, status);  // k_prep starts the status words
     last_pos = pos;
     nn_forked = false;
     prepare(st, a, box, a.induce && set.predictor == 5 && nn_on ? ind->hist : nullptr);
@@ -1388,7 +1379,7 @@ struct Engine : EngineBase {
       if (out->iterations) CK(cudaMemsetAsync(out->iterations, 0, sizeof(int32_t) * nsys, st));
       if (out->residual) CK(cudaMemsetAsync(out->residual, 0, sizeof(double) * nsys, st));
     }
-    energy_pass(st, a, mu, out->energy ? out->energy : energy_tmp.p, out->virial, a.induce && iel_shadow);
+    energy_pass(st, a, mu, out->energy ? out->energy : energy_tmp.p, out->virial, a.induce && !set.iel, a.induce && iel_shadow);
     if (!tune.tuned && !tune_fixed) {  // the first direct step: time the kernel variants on its rows
       cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
       CK(cudaStreamIsCapturing(st, &cs));
@@ -1409,7 +1400,7 @@ struct Engine : EngineBase {
       CK(cudaMemsetAsync(ind->mu, 0, sizeof(double) * 3 * nt, st));
       if (iters) CK(cudaMemsetAsync(iters, 0, sizeof(int32_t) * nsys, st));
     }
-    energy_pass(st, a, ind->mu, energy_out, nullptr);
+    energy_pass(st, a, ind->mu, energy_out, nullptr, a.induce);
   }
 
   void fixed_mu(cudaStream_t st, const double *pos, const double *box, const int32_t *idx, int idx_width, const double *mu,
@@ -1419,7 +1410,7 @@ struct Engine : EngineBase {
     CK(cudaMemsetAsync(status, 0, sizeof(unsigned) * nsys, st));
     pgm::Dev<T> a = dev(pos, idx, idx_width, forces_out ? forces_out : forces_tmp.p, status);
     prepare(st, a, box);
-    energy_pass(st, a, mu, energy_out ? energy_out : energy_tmp.p, virial);
+    energy_pass(st, a, mu, energy_out ? energy_out : energy_tmp.p, virial, false);
   }
 
   void field(cudaStream_t st, const double *pos, const double *box, int with_q, const double *d, double *out) override {

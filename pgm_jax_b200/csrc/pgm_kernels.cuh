@@ -131,25 +131,20 @@ template <typename T, int AT>
 __device__ __forceinline__ T &entry_v(unsigned char *chunk, int t) { return reinterpret_cast<T *>(chunk + AT)[t & 31]; }
 
 // ------------------------------------------------------------------ box and per-atom set-up
+// Box-dependent values of system s (every block of the system computes its own copy; the system's first
+// block, `first`, publishes them and starts the step's status word).
 template <typename T>
-__global__ void k_box(Dev<T> a, const double *boxes) {
-  pdl_enter();  // launched as a programmatic dependent of the previous kernel
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s == 0) { a.max_count[0] = 0; a.max_count[1] = 0; }  // the step's largest row counts start here
-  if (s >= a.nsys) return;
-  const double *H = boxes + 9 * s;
-  BoxInfo &B = a.box[s];
-  int changed = 0;
-  for (int k = 0; k < 9; ++k) changed |= (B.H[k] != H[k]);
-  double d = H[0] * (H[4] * H[8] - H[5] * H[7]) - H[1] * (H[3] * H[8] - H[5] * H[6]) + H[2] * (H[3] * H[7] - H[4] * H[6]);
-  double Hi[9];  // cofactor inverse (box.py:195-234)
+__device__ __forceinline__ void box_setup(Dev<T> &a, int s, const double *H, BoxInfo &B, bool first) {
+  const SysInfo &S = a.sys[s];
+  const double d = H[0] * (H[4] * H[8] - H[5] * H[7]) - H[1] * (H[3] * H[8] - H[5] * H[6]) + H[2] * (H[3] * H[7] - H[4] * H[6]);
+  double *Hi = B.Hinv;  // cofactor inverse (box.py:195-234)
   Hi[0] = (H[4] * H[8] - H[5] * H[7]) / d; Hi[1] = (H[2] * H[7] - H[1] * H[8]) / d; Hi[2] = (H[1] * H[5] - H[2] * H[4]) / d;
   Hi[3] = (H[5] * H[6] - H[3] * H[8]) / d; Hi[4] = (H[0] * H[8] - H[2] * H[6]) / d; Hi[5] = (H[2] * H[3] - H[0] * H[5]) / d;
   Hi[6] = (H[3] * H[7] - H[4] * H[6]) / d; Hi[7] = (H[1] * H[6] - H[0] * H[7]) / d; Hi[8] = (H[0] * H[4] - H[1] * H[3]) / d;
-  for (int k = 0; k < 9; ++k) { B.H[k] = H[k]; B.Hinv[k] = Hi[k]; }
+  for (int k = 0; k < 9; ++k) B.H[k] = H[k];
+  if (!first) return;
   B.vol = fabs(d);
   for (int c = 0; c < 3; ++c) B.idiag[c] = 1.0 / H[4 * c];
-  const SysInfo &S = a.sys[s];
   for (int ax = 0; ax < 3; ++ax) {
     // plane height h_a = 1 / |column a of H^-1|
     double c0 = Hi[0 * 3 + ax], c1 = Hi[1 * 3 + ax], c2v = Hi[2 * 3 + ax];
@@ -158,6 +153,8 @@ __global__ void k_box(Dev<T> a, const double *boxes) {
     int R = (int)ceil((a.cutoff + a.skin) * nc / B.h[ax] - 1e-12);
     B.R[ax] = (2 * R + 1 >= nc) ? -1 : R;
   }
+  int changed = 0;
+  for (int k = 0; k < 9; ++k) changed |= (a.box[s].H[k] != H[k]);
   B.changed = changed;
   if (changed) atomicOr(a.nb_flag, 1);
   int bad = (fabs(H[1]) > 1e-12 * fabs(H[0])) || (fabs(H[2]) > 1e-12 * fabs(H[0])) || (fabs(H[5]) > 1e-12 * fabs(H[0])) ||
@@ -165,19 +162,26 @@ __global__ void k_box(Dev<T> a, const double *boxes) {
   double mc = 0.5 * fmin(H[0], fmin(H[4], H[8]));
   if (a.cutoff > mc) bad = 1;
   B.bad = bad;
-  a.status[s] = bad ? 0x8u : 0u;  // the step's status word starts here
+  a.box[s] = B;
+  a.status[s] = bad ? 0x8u : 0u;
+  if (s == 0) { a.max_count[0] = 0; a.max_count[1] = 0; }  // the step's largest row counts start here
 }
 
-// Fractional coordinates, spline base and offset (pme.py:269-304), permanent dipoles
-// (forcefield.py:1032-1042) and the cell of every atom.
+// The step's set-up in one launch (thread per atom): the box, fractional coordinates, spline base and offset
+// (pme.py:269-304), permanent dipoles (forcefield.py:1032-1042), the list's displacement test, and, on the
+// thread of a molecule's first atom, the offsets of its atoms from its centre of mass (the molecule made
+// whole from its first atom), for the molecular virial.  A non-finite position is marked in base.w (the
+// status word is being started by another block) and reported by the force pass.
 template <typename T>
-__global__ void k_prep(Dev<T> a) {
+__global__ void k_prep(Dev<T> a, const double *boxes) {
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.nt) return;
-  int s = a.sysid[i];
+  __shared__ BoxInfo B;
+  const int s = a.tb_sys[blockIdx.x];
   const SysInfo &S = a.sys[s];
-  const BoxInfo &B = a.box[s];
+  const int a0 = a.tb_atom0[blockIdx.x], i = a0 + threadIdx.x;
+  if (threadIdx.x == 0) box_setup(a, s, boxes + 9 * (size_t)s, B, a0 == S.atom0);
+  __syncthreads();
+  if (i >= S.atom0 + S.natom) return;
   double px = a.pos[3 * i], py = a.pos[3 * i + 1], pz = a.pos[3 * i + 2];
   double uc[3];
   int4 b;
@@ -198,8 +202,7 @@ __global__ void k_prep(Dev<T> a) {
     bb[ax] = bv;
     ff[ax] = T(w - fl);
   }
-  if (!finite) atomicOr(&a.status[s], 0x4u);
-  b.x = bb[0]; b.y = bb[1]; b.z = bb[2]; b.w = 0;
+  b.x = bb[0]; b.y = bb[1]; b.z = bb[2]; b.w = finite ? 0 : 1;
   f.x = ff[0]; f.y = ff[1]; f.z = ff[2]; f.w = T(0);
   a.base[i] = b;
   a.frac[i] = f;
@@ -227,7 +230,20 @@ __global__ void k_prep(Dev<T> a) {
   min_image(dx, dy, dz, B.H);
   double h2 = 0.25 * a.skin * a.skin;
   if (!(dx * dx + dy * dy + dz * dz <= h2)) atomicOr(a.nb_flag, 1);
-  (void)uc;
+  const int i0 = a.molfirst[i], i1 = a.molend[i];
+  if (i != i0) return;
+  double cx = 0, cy = 0, cz = 0, mt = 0;
+  for (int j = i0; j < i1; ++j) {
+    double vx = a.pos[3 * j] - px, vy = a.pos[3 * j + 1] - py, vz = a.pos[3 * j + 2] - pz;
+    min_image(vx, vy, vz, B.H);
+    a.off[j] = make_double4(vx, vy, vz, 0);
+    cx += a.mass[j] * vx; cy += a.mass[j] * vy; cz += a.mass[j] * vz; mt += a.mass[j];
+  }
+  cx /= mt; cy /= mt; cz /= mt;
+  for (int j = i0; j < i1; ++j) {
+    double4 o = a.off[j];
+    a.off[j] = make_double4(o.x - cx, o.y - cy, o.z - cz, 0);
+  }
 }
 
 // Cell of every atom (only when the candidate list is rebuilt).
@@ -256,31 +272,8 @@ __global__ void k_cell_assign(Dev<T> a) {
   a.slot_of[i] = atomicAdd(&a.cell_count[cell], 1);
 }
 
-// Offsets of every atom from its molecule's centre of mass (molecule made whole from its first
-// atom), for the molecular virial.
-template <typename T>
-__global__ void k_mol(Dev<T> a) {
-  pdl_enter();  // launched as a programmatic dependent of the previous kernel
-  int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= a.nmol) return;
-  int i0 = a.mol_start[m], i1 = a.mol_start[m + 1];
-  const BoxInfo &B = a.box[a.sysid[i0]];
-  double cx = 0, cy = 0, cz = 0, mt = 0;
-  for (int i = i0; i < i1; ++i) {
-    double vx = a.pos[3 * i] - a.pos[3 * i0], vy = a.pos[3 * i + 1] - a.pos[3 * i0 + 1], vz = a.pos[3 * i + 2] - a.pos[3 * i0 + 2];
-    min_image(vx, vy, vz, B.H);
-    a.off[i] = make_double4(vx, vy, vz, 0);
-    cx += a.mass[i] * vx; cy += a.mass[i] * vy; cz += a.mass[i] * vz; mt += a.mass[i];
-  }
-  cx /= mt; cy /= mt; cz /= mt;
-  for (int i = i0; i < i1; ++i) {
-    double4 o = a.off[i];
-    a.off[i] = make_double4(o.x - cx, o.y - cy, o.z - cz, 0);
-  }
-}
-
-// Exclusive scan of the cell counts of all systems (one block).
-__global__ void k_scan_cells(const int *count, int *start, int n, const int *flag) {
+// Exclusive scan of the cell counts of all systems (one block), which are cleared for the next rebuild.
+__global__ void k_scan_cells(int *count, int *start, int n, const int *flag) {
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
   if (!*flag) return;
   __shared__ int part[1024];
@@ -290,6 +283,7 @@ __global__ void k_scan_cells(const int *count, int *start, int n, const int *fla
   for (int base = 0; base < n; base += 1024) {
     int i = base + threadIdx.x;
     int v = i < n ? count[i] : 0;
+    if (v) count[i] = 0;
     part[threadIdx.x] = v;
     __syncthreads();
     for (int o = 1; o < 1024; o <<= 1) {
@@ -390,17 +384,6 @@ __global__ void __launch_bounds__(256) k_cand(Dev<T> a) {
     a.pos_ref[i] = pi;
     if (count > a.cc) atomicOr(&a.status[s], 0x10u);
   }
-}
-
-// End of a rebuild: clear the cell counts for the next one, count it, lower the flag.
-__global__ void k_nb_finish(int *cell_count, int ncell, int *flag, long long *builds) {
-  pdl_enter();  // launched as a programmatic dependent of the previous kernel
-  if (!*flag) return;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncell; c += gridDim.x * blockDim.x) cell_count[c] = 0;
-}
-__global__ void k_nb_lower(int *flag, long long *builds) {
-  pdl_enter();  // launched as a programmatic dependent of the previous kernel
-  if (*flag) { *flag = 0; *builds += 1; }
 }
 
 // ------------------------------------------------------------------ pair rows
@@ -645,9 +628,14 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_rows(Dev<T> a) 
 // ------------------------------------------------------------------ PME influence function
 // G(m) = exp(-pi^2 |m*|^2 / beta^2) / (2 pi V |m*|^2) / (b1 b2 b3), 0 at m = 0 (pme.py:243-267),
 // on the half spectrum, computed in FP64, stored in T; recomputed only when the box changed.
+// Ends a rebuild of the candidate list too (it runs after it): counts it and lowers the flag.
 template <typename T>
 __global__ void k_influence(Dev<T> a, long long total) {
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
+  if (blockIdx.x == 0 && threadIdx.x == 0 && !a.idx && *a.nb_flag) { *a.nb_flag = 0; *a.nb_builds += 1; }
+  int any = 0;
+  for (int s = threadIdx.x; s < a.nsys; s += blockDim.x) any |= a.box[s].changed;
+  if (!__syncthreads_or(any)) return;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total; g += (long long)gridDim.x * blockDim.x) {
     int s = 0;
     while (s + 1 < a.nsys && a.sys[s + 1].cgrid0 <= g) ++s;
@@ -1225,26 +1213,52 @@ __global__ void k_vec_from_f64(int n, const double *src, v4<T> *dst) {
 }
 
 // ------------------------------------------------------------------ CG
+// Which start a solve takes (forcefield.py:1951-1966): `have` the history predictor applies, `fused`
+// its one-sweep start.  mode 1: the guess is the state's mu, plain start (energy, forcefield.py:2606-2612).
+struct StartRule {
+  int K, fused, refresh, mode, use_nn;
+  const int32_t *count;
+  const double *norm;
+  __device__ __forceinline__ bool have(int s) const { return mode == 1 || (K > 0 && count[s] >= K); }
+  __device__ __forceinline__ bool is_fused(int s) const { return mode == 0 && fused && have(s) && count[s] % refresh != 0; }
+};
+// The system's solver state before the start, and the condition of the plain start's node.
+__device__ __forceinline__ void cg_setup(CGSys &G, int s, const StartRule &r, cudaGraphConditionalHandle plain, int use_cond) {
+  G.have = r.have(s);
+  G.nn = r.use_nn && G.have;  // k_start1 adds the model's correction to the extrapolation
+  G.fallback = 0;
+  G.iel_ext = 0; G.iel_first = 0; G.maxit_s = -1; G.tol_s = -1.0;
+  G.fused = r.is_fused(s);
+  G.sweep2 = !G.fused;
+  if (use_cond && G.sweep2) cudaGraphSetConditional(plain, 1u);  // the plain start's sweep runs (default 0)
+  G.active = 0;
+  G.norm = G.fused ? r.norm[s] : 1.0;
+  G.acc_abs = 0; G.acc_rz = 0; G.acc_max = 0; G.acc_pap = 0; G.acc_num = 0;
+}
+
 // Start, step 1 (thread per atom): the predictor guess x0h = sum c_j hist_j (forcefield.py:605,
-// 1956-1958) and the dipoles of the first field sweep: p + x0h (fused start) or p (plain).
+// 1956-1958) and the dipoles of the first field sweep: p + x0h (fused start) or p (plain); the thread of a
+// system's first atom sets up its solver state.
 template <typename T>
-__global__ void k_start1(Dev<T> a, const double *hist, int K, double c0, double c1, double c2, double c3, const float *xnn) {
+__global__ void k_start1(Dev<T> a, StartRule rule, const double *hist, double c0, double c1, double c2, double c3, const float *xnn,
+                         cudaGraphConditionalHandle plain, int use_cond) {
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.nt) return;
   int s = a.sysid[i];
-  const CGSys &G = a.cg[s];
+  const bool have = rule.have(s), fused = rule.is_fused(s);
+  if (i == a.sys[s].atom0) cg_setup(a.cg[s], s, rule, plain, use_cond);
   double x0[3] = {0, 0, 0};
-  if (G.have) {
+  if (have) {
     const double cc[4] = {c0, c1, c2, c3};
-    for (int j = 0; j < K; ++j)
+    for (int j = 0; j < rule.K; ++j)
       for (int c = 0; c < 3; ++c) x0[c] += cc[j] * hist[((size_t)j * a.nt + i) * 3 + c];
     if (xnn)  // the learned correction to the extrapolation
       for (int c = 0; c < 3; ++c) x0[c] += double(xnn[3 * (size_t)i + c]);
   }
   double4 p = a.pperm[i];
   v4<T> d, x;
-  if (G.fused) { d.x = T(p.x + x0[0]); d.y = T(p.y + x0[1]); d.z = T(p.z + x0[2]); }
+  if (fused) { d.x = T(p.x + x0[0]); d.y = T(p.y + x0[1]); d.z = T(p.z + x0[2]); }
   else { d.x = T(p.x); d.y = T(p.y); d.z = T(p.z); }
   d.w = a.q[i];  // read with the dipole by the field sweep
   x.x = T(x0[0]); x.y = T(x0[1]); x.z = T(x0[2]); x.w = T(0);
@@ -1252,42 +1266,147 @@ __global__ void k_start1(Dev<T> a, const double *hist, int K, double c0, double 
   a.X[i] = x;
 }
 
-// Start, step 2: fused: r0 = field(q, p + x0) - x0 / alpha; plain: b = field(q, p), the norm
-// mean|alpha b| and, without history, x0 = alpha b (forcefield.py:1960-1997).
-template <typename T>
-__global__ void k_start2(Dev<T> a) {
+// What a solve's begin needs beside the systems' state (cg_begin).
+struct BeginArgs {
+  CGSys *cg;
+  int nsys;
+  double tol;
+  int max_iter;
+  int *any;
+  double fb_factor;
+  cudaGraphConditionalHandle fbcond;
+  int use_fbcond;
+  int *fb_any;
+  unsigned *done;
+};
+
+// Per-system scalars after the start (one block): norm, r.z, err, active; *any = some system iterates.
+// which 0: the systems with the fused start (*any and *fb_any start here); 1: those with the plain start;
+// 2: all; 3: the learned guess's fallbacks, re-evaluated after their sweep.
+// The learned guess's check (fb_factor > 0): a system that started from x4 + the model's
+// correction falls back to x4 when its start residual err exceeds fb_factor times the running
+// mean of the extrapolation's (raising the fallback node's condition, *fb_any); a system that
+// started from the extrapolation itself adds its err to that mean, and so does a fallback (which is counted).
+__device__ __forceinline__ void cg_begin(const BeginArgs &b, int which) {
+  __shared__ int act, fb;
+  if (threadIdx.x == 0) { act = 0; fb = 0; }
+  __syncthreads();
+  constexpr double W = 0.1;  // weight of a new sample in the running mean
+  for (int s = threadIdx.x; s < b.nsys; s += blockDim.x) {
+    CGSys &G = b.cg[s];
+    const bool mine = which == 2 || (which == 0 && G.fused) || (which == 1 && !G.fused) || (which == 3 && G.fallback);
+    if (mine) {
+      if (!G.fused) G.norm = G.acc_abs / G.n3 + 1e-300;
+      G.rz = G.acc_rz;
+      G.err = __longlong_as_double((long long)G.acc_max) / G.norm;
+      G.beta = 0.0;
+      G.it = 0;
+      G.active = (G.err > (G.tol_s >= 0.0 ? G.tol_s : b.tol)) && ((G.maxit_s >= 0 ? G.maxit_s : b.max_iter) > 0);
+      G.acc_abs = 0; G.acc_rz = 0; G.acc_max = 0; G.acc_pap = 0; G.acc_num = 0;
+      const bool record = which == 3 || (b.fb_factor > 0.0 && G.have && !G.nn);
+      if (which != 3 && b.fb_factor > 0.0 && G.nn && G.ref_n > 0 && G.err > b.fb_factor * G.ref_err) {
+        G.fallback = 1;
+        atomicOr(&fb, 1);
+      } else if (record) {
+        G.ref_err = G.ref_n == 0 ? G.err : (1.0 - W) * G.ref_err + W * G.err;
+        G.ref_n += 1;
+        if (which == 3) G.fallbacks += 1;
+      }
+    }
+    if (G.active) atomicOr(&act, 1);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    *b.any = act;
+    if (which != 3 && b.fb_any) *b.fb_any = which == 1 ? (*b.fb_any | fb) : fb;
+    if (which != 3 && b.use_fbcond && fb) cudaGraphSetConditional(b.fbcond, 1u);  // the fallback node runs (default 0)
+  }
+}
+// The block that finishes last (a counter after a memory fence) takes the caller's closing step.
+__device__ __forceinline__ bool last_block(unsigned *done) {
+  __shared__ bool last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();  // this block's partial sums are visible before it is counted
+    last = atomicAdd(done, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (last) {
+    __threadfence();
+    if (threadIdx.x == 0) *done = 0u;
+  }
+  return last;
+}
+
+// A block's sums of rz and max m of the start, added to its system's accumulators.
+__device__ __forceinline__ void start_sums(CGSys &G, double rz, double m) {
+  __shared__ double red[THREADS_PER_BLOCK / 32];
+  __shared__ unsigned long long mx[THREADS_PER_BLOCK / 32];
+  int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  rz = warp_sum<double>(rz);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if (lane == 0) { red[warp] = rz; mx[warp] = (unsigned long long)__double_as_longlong(m); }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double v = 0;
+    unsigned long long mm = 0;
+    for (int w = 0; w < THREADS_PER_BLOCK / 32; ++w) { v += red[w]; mm = max(mm, mx[w]); }
+    atomicAdd(&G.acc_rz, v);
+    atomicMax(&G.acc_max, mm);
+  }
+}
+
+// Start, step 2: fused: r0 = field(q, p + x0) - x0 / alpha, and the CG's initial z = alpha r, p = z, r.z and
+// max|alpha r| (forcefield.py:1796-1819); plain: b = field(q, p), the norm mean|alpha b| and, without history,
+// x0 = alpha b (forcefield.py:1960-1997).  The last block evaluates the fused systems' scalars (cg_begin).
+// LOCAL (the local preconditioner): only max|alpha r|; z, p, r.z and the scalars come with its kernels.
+template <typename T, bool LOCAL>
+__global__ void k_start2(Dev<T> a, BeginArgs begin) {
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
   __shared__ double red[THREADS_PER_BLOCK / 32];
   int s = a.tb_sys[blockIdx.x];
   int i = a.tb_atom0[blockIdx.x] + threadIdx.x;
   const SysInfo &S = a.sys[s];
   CGSys &G = a.cg[s];
-  double sab = 0.0;
+  const bool fused = G.fused;  // uniform over the block
+  double sab = 0.0, rz = 0.0, m = 0.0;
   if (i < S.atom0 + S.natom) {
     v4<T> b = a.B[i];
     v4<T> x = a.X[i];
     T al = a.alpha[i];
-    if (G.fused) {
+    if (fused) {
       T ia = a.ialpha[i];
-      v4<T> r;
+      v4<T> r, z;
       r.x = b.x - x.x * ia; r.y = b.y - x.y * ia; r.z = b.z - x.z * ia; r.w = T(0);
       a.R[i] = r;
+      z.x = al * r.x; z.y = al * r.y; z.z = al * r.z; z.w = T(0);
+      if (!LOCAL) {
+        a.Z[i] = z;
+        a.P[i] = z;
+        rz = double(r.x * z.x) + double(r.y * z.y) + double(r.z * z.z);
+      }
+      m = fmax(fabs(double(z.x)), fmax(fabs(double(z.y)), fabs(double(z.z))));
     } else {
-      double ax = double(a.alpha[i]) * double(b.x), ay = double(a.alpha[i]) * double(b.y), az = double(a.alpha[i]) * double(b.z);
+      double ax = double(al) * double(b.x), ay = double(al) * double(b.y), az = double(al) * double(b.z);
       sab = fabs(ax) + fabs(ay) + fabs(az);
       if (!G.have) { x.x = T(ax); x.y = T(ay); x.z = T(az); x.w = T(0); a.X[i] = x; }
-      (void)al;
     }
   }
-  int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  sab = warp_sum<double>(sab);
-  if (lane == 0) red[warp] = sab;
-  __syncthreads();
-  if (threadIdx.x == 0 && !G.fused) {
-    double v = 0;
-    for (int w = 0; w < THREADS_PER_BLOCK / 32; ++w) v += red[w];
-    atomicAdd(&G.acc_abs, v);
+  if (fused) {
+    start_sums(G, rz, m);
+  } else {
+    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    sab = warp_sum<double>(sab);
+    if (lane == 0) red[warp] = sab;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double v = 0;
+      for (int w = 0; w < THREADS_PER_BLOCK / 32; ++w) v += red[w];
+      atomicAdd(&G.acc_abs, v);
+    }
   }
+  if (!LOCAL && last_block(begin.done)) cg_begin(begin, 0);
 }
 
 // Start, step 3 (plain start only): r0 = b - A x0.
@@ -1303,96 +1422,41 @@ __global__ void k_start3(Dev<T> a) {
   a.R[i] = r;
 }
 
-// CG initialisation: z = alpha r, p = z, r.z and max|alpha r| (forcefield.py:1796-1819).
+// CG initialisation of the plain start's systems: z = alpha r, p = z, r.z and max|alpha r|, and, in the last
+// block, their scalars (cg_begin).
 // FB (the learned guess's fallback, systems with the flag only): first back to the extrapolation,
 // x = x4 = x - delta and r0 = b - A x4 = r0 + A delta (A delta in AP).
-// LOCAL (the local preconditioner): only max|alpha r|; z, p and r.z come from its kernels.
-template <typename T, bool FB = false, bool LOCAL = false>
-__global__ void k_cg_init(Dev<T> a, const float *delta = nullptr) {
-  __shared__ double red[THREADS_PER_BLOCK / 32];
-  __shared__ unsigned long long mx[THREADS_PER_BLOCK / 32];
-  if (FB) pdl_enter();  // launched as a programmatic dependent of the fallback sweep
-  int s = a.tb_sys[blockIdx.x];
-  if (FB && !a.cg[s].fallback) return;  // uniform over the block
-  int i = a.tb_atom0[blockIdx.x] + threadIdx.x;
-  const SysInfo &S = a.sys[s];
-  double rz = 0, m = 0;
-  if (i < S.atom0 + S.natom) {
-    if (FB) {
-      v4<T> r = a.R[i], ad = a.AP[i], x = a.X[i];
-      r.x += ad.x; r.y += ad.y; r.z += ad.z;
-      x.x -= T(delta[3 * (size_t)i]); x.y -= T(delta[3 * (size_t)i + 1]); x.z -= T(delta[3 * (size_t)i + 2]);
-      a.R[i] = r;
-      a.X[i] = x;
-    }
-    v4<T> r = a.R[i];
-    T al = a.alpha[i];
-    v4<T> z;
-    z.x = al * r.x; z.y = al * r.y; z.z = al * r.z; z.w = T(0);
-    if (!LOCAL) {
-      a.Z[i] = z;
-      a.P[i] = z;
-      rz = double(r.x * z.x) + double(r.y * z.y) + double(r.z * z.z);
-    }
-    m = fmax(fabs(double(z.x)), fmax(fabs(double(z.y)), fabs(double(z.z))));
-  }
-  int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  rz = warp_sum<double>(rz);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if (lane == 0) { red[warp] = rz; mx[warp] = (unsigned long long)__double_as_longlong(m); }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double v = 0;
-    unsigned long long mm = 0;
-    for (int w = 0; w < THREADS_PER_BLOCK / 32; ++w) { v += red[w]; mm = max(mm, mx[w]); }
-    atomicAdd(&a.cg[s].acc_rz, v);
-    atomicMax(&a.cg[s].acc_max, mm);
-  }
-}
-
-// Per-system scalars after the start: norm, r.z, err, active; *any = some system iterates.
-// The learned guess's check (fb_factor > 0, pass 0): a system that started from x4 + the model's
-// correction falls back to x4 when its start residual err exceeds fb_factor times the running
-// mean of the extrapolation's (raising the fallback node's condition, *fb_any); a system that
-// started from the extrapolation itself adds its err to that mean.  Pass 1 (after the fallback
-// sweep) re-evaluates the fallback systems, adds their (extrapolation) err to the mean and counts
-// the fallback; *any covers every system.
-__global__ void k_cg_begin(CGSys *cg, int nsys, double tol, int max_iter, int *any, double fb_factor = 0.0, int pass = 0,
-                           cudaGraphConditionalHandle fbcond = 0, int use_cond = 0, int *fb_any = nullptr) {
+// LOCAL (the local preconditioner): only max|alpha r|; z, p, r.z and the scalars come with its kernels.
+template <typename T, bool FB, bool LOCAL>
+__global__ void k_cg_init(Dev<T> a, const float *delta, BeginArgs begin) {
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
-  __shared__ int act, fb;
-  if (threadIdx.x == 0) { act = 0; fb = 0; }
-  __syncthreads();
-  constexpr double W = 0.1;  // weight of a new sample in the running mean
-  for (int s = threadIdx.x; s < nsys; s += blockDim.x) {
-    CGSys &G = cg[s];
-    if (pass == 0 || G.fallback) {
-      if (!G.fused) G.norm = G.acc_abs / G.n3 + 1e-300;
-      G.rz = G.acc_rz;
-      G.err = __longlong_as_double((long long)G.acc_max) / G.norm;
-      G.beta = 0.0;
-      G.it = 0;
-      G.active = (G.err > (G.tol_s >= 0.0 ? G.tol_s : tol)) && ((G.maxit_s >= 0 ? G.maxit_s : max_iter) > 0);
-      G.acc_abs = 0; G.acc_rz = 0; G.acc_max = 0; G.acc_pap = 0; G.acc_num = 0;
-      const bool record = (pass == 1) || (fb_factor > 0.0 && G.have && !G.nn);
-      if (pass == 0 && fb_factor > 0.0 && G.nn && G.ref_n > 0 && G.err > fb_factor * G.ref_err) {
-        G.fallback = 1;
-        atomicOr(&fb, 1);
-      } else if (record) {
-        G.ref_err = G.ref_n == 0 ? G.err : (1.0 - W) * G.ref_err + W * G.err;
-        G.ref_n += 1;
-        if (pass == 1) G.fallbacks += 1;
+  int s = a.tb_sys[blockIdx.x];
+  if (FB ? a.cg[s].fallback : !a.cg[s].fused) {  // uniform over the block
+    int i = a.tb_atom0[blockIdx.x] + threadIdx.x;
+    const SysInfo &S = a.sys[s];
+    double rz = 0, m = 0;
+    if (i < S.atom0 + S.natom) {
+      v4<T> r = a.R[i];
+      if (FB) {
+        v4<T> ad = a.AP[i], x = a.X[i];
+        r.x += ad.x; r.y += ad.y; r.z += ad.z;
+        x.x -= T(delta[3 * (size_t)i]); x.y -= T(delta[3 * (size_t)i + 1]); x.z -= T(delta[3 * (size_t)i + 2]);
+        a.R[i] = r;
+        a.X[i] = x;
       }
+      T al = a.alpha[i];
+      v4<T> z;
+      z.x = al * r.x; z.y = al * r.y; z.z = al * r.z; z.w = T(0);
+      if (!LOCAL) {
+        a.Z[i] = z;
+        a.P[i] = z;
+        rz = double(r.x * z.x) + double(r.y * z.y) + double(r.z * z.z);
+      }
+      m = fmax(fabs(double(z.x)), fmax(fabs(double(z.y)), fabs(double(z.z))));
     }
-    if (G.active) atomicOr(&act, 1);
+    start_sums(a.cg[s], rz, m);
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    *any = act;
-    if (pass == 0 && fb_any) *fb_any = fb;
-    if (pass == 0 && use_cond && fb) cudaGraphSetConditional(fbcond, 1u);  // the fallback node runs (default 0)
-  }
+  if (!LOCAL && last_block(begin.done)) cg_begin(begin, FB ? 3 : 1);
 }
 
 // Fallback, step 1: the model's correction delta of every fallback system's atoms as the dipoles
@@ -1486,17 +1550,7 @@ __global__ void k_cg_update_check(Dev<T> a, int nsys, double tol, int max_iter, 
                                   int use_cond, unsigned *done) {
   pdl_enter();
   cg_update_body(a);
-  __shared__ bool last;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();  // this block's partial sums are visible before it is counted
-    last = atomicAdd(done, 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  cg_check_body(a.cg, nsys, tol, max_iter, any, cond, use_cond);
-  if (threadIdx.x == 0) *done = 0u;
+  if (last_block(done)) cg_check_body(a.cg, nsys, tol, max_iter, any, cond, use_cond);
 }
 
 // ------------------------------------------------------------------ local preconditioner
@@ -1609,13 +1663,12 @@ __global__ void k_lp_ap(Dev<T> a, const v4<T> *__restrict__ Pin, v4<T> *__restri
 }
 
 // Inner update: z += al p (al = rr.zz / p.Ap); not LAST: rr -= al Ap, zz = alpha rr, partial rr.zz
-// for the next inner iteration.  LAST: the outer quantities -- MODE 0 (start, fallback): p = z
-// and r.z; MODE 1 (iteration): z.(r_new - r_old) and r_new.z.  The block that finishes last
+// for the next inner iteration.  LAST: the outer quantities -- MODE 0 (start, fallback): p = z,
+// r.z and the start's scalars (cg_begin); MODE 1 (iteration): z.(r_new - r_old) and r_new.z.  The block that finishes last
 // evaluates the inner scalars (lb, the next rr.zz) and, in MODE 1, the outer CG's per-system check
 // and loop condition (cg_check_body).
 template <typename T, int ACT, bool LAST, int MODE>
-__global__ void k_lp_step(Dev<T> a, const v4<T> *__restrict__ Pcur, int nsys, double tol, int max_iter, int *any,
-                          cudaGraphConditionalHandle cond, int use_cond, unsigned *done) {
+__global__ void k_lp_step(Dev<T> a, const v4<T> *__restrict__ Pcur, BeginArgs b, cudaGraphConditionalHandle cond, int use_cond) {
   pdl_enter();
   {
     const int s = a.tb_sys[blockIdx.x];
@@ -1660,16 +1713,8 @@ __global__ void k_lp_step(Dev<T> a, const v4<T> *__restrict__ Pcur, int nsys, do
       }
     }
   }
-  __shared__ bool last;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();  // this block's partial sums are visible before it is counted
-    last = atomicAdd(done, 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  for (int s = threadIdx.x; s < nsys; s += blockDim.x) {
+  if (!last_block(b.done)) return;
+  for (int s = threadIdx.x; s < b.nsys; s += blockDim.x) {
     CGSys &G = a.cg[s];
     if (!LAST) {
       G.lb = G.acc_lrz2 / fmax(G.acc_lrz, 1e-300);
@@ -1680,11 +1725,11 @@ __global__ void k_lp_step(Dev<T> a, const v4<T> *__restrict__ Pcur, int nsys, do
     G.acc_lrz2 = 0.0;
     G.acc_lpap = 0.0;
   }
-  if (LAST && MODE == 1) {
+  if (LAST) {
     __syncthreads();
-    cg_check_body(a.cg, nsys, tol, max_iter, any, cond, use_cond);
+    if (MODE == 1) cg_check_body(a.cg, b.nsys, b.tol, b.max_iter, b.any, cond, use_cond);
+    else cg_begin(b, ACT == 3 ? 3 : 2);  // the start's scalars
   }
-  if (threadIdx.x == 0) *done = 0u;
 }
 
 // The outer CG update with the local preconditioner (thread per atom): x += st p, r_new = r - st
@@ -1726,70 +1771,75 @@ __global__ void k_cg_update_r(Dev<T> a) {
 }
 
 // After the loop: the peek step mu = x + peek alpha r (forcefield.py:1819-1820), the dipoles
-// in FP64, the history push (forcefield.py:2005-2007) and mu + p for the energy pass.
+// in FP64, the history push (forcefield.py:2005-2007), mu + p and zero accumulators for the energy pass, and the
+// systems' solver state.
+struct StateOut {
+  int32_t *count;
+  double *norm;
+  int32_t *iters;
+  double *resid;
+  unsigned *status;
+  int push;
+  double tol;
+};
+__device__ __forceinline__ void cg_state_out(const CGSys *cg, int s, const StateOut &o) {
+  const CGSys &G = cg[s];
+  if (o.push) { o.count[s] += 1; o.norm[s] = G.norm; }
+  if (o.iters) o.iters[s] = G.it;
+  if (o.resid) o.resid[s] = G.err;
+  if (G.err > o.tol && !G.iel_ext) atomicOr(&o.status[s], 0x2u);  // an extended iEL step stops short of tol by design
+}
 template <typename T>
-__global__ void k_cg_finish(Dev<T> a, double *mu, double *hist, int push) {
+__device__ __forceinline__ void energy_start(Dev<T> &a, int i, const double *m) {  // all threads of the launch
+  constexpr int NACC = sizeof(EnergyAcc) / sizeof(double);
+  for (int t = i; t < NACC * a.nsys; t += gridDim.x * blockDim.x) reinterpret_cast<double *>(a.eacc)[t] = 0.0;
+  if (i >= a.nt) return;
+  const double4 p = a.pperm[i];
+  v4<T> d;
+  d.x = T(p.x + m[0]); d.y = T(p.y + m[1]); d.z = T(p.z + m[2]); d.w = a.q[i];
+  a.D[i] = d;
+}
+template <typename T>
+__global__ void k_cg_finish(Dev<T> a, double *mu, double *hist, int push, StateOut out) {
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.nt) return;
-  v4<T> x = a.X[i], r = a.R[i];
-  T al = a.alpha[i];
-  T pk = T(a.peek);
-  if (a.peek != 0.0) { x.x += pk * r.x * al; x.y += pk * r.y * al; x.z += pk * r.z * al; }
-  double m[3] = {double(x.x), double(x.y), double(x.z)};
-  for (int c = 0; c < 3; ++c) mu[3 * i + c] = m[c];
-  if (push) {
-    size_t st = (size_t)a.nt * 3;
-    for (int c = 0; c < 3; ++c) {
-      size_t o = (size_t)3 * i + c;
-      hist[3 * st + o] = hist[2 * st + o];
-      hist[2 * st + o] = hist[st + o];
-      hist[st + o] = hist[o];
-      hist[o] = m[c];
+  for (int s = i; s < a.nsys; s += gridDim.x * blockDim.x) cg_state_out(a.cg, s, out);
+  double m[3] = {0, 0, 0};
+  if (i < a.nt) {
+    v4<T> x = a.X[i], r = a.R[i];
+    T al = a.alpha[i];
+    T pk = T(a.peek);
+    if (a.peek != 0.0) { x.x += pk * r.x * al; x.y += pk * r.y * al; x.z += pk * r.z * al; }
+    m[0] = double(x.x); m[1] = double(x.y); m[2] = double(x.z);
+    for (int c = 0; c < 3; ++c) mu[3 * i + c] = m[c];
+    if (push) {
+      size_t st = (size_t)a.nt * 3;
+      for (int c = 0; c < 3; ++c) {
+        size_t o = (size_t)3 * i + c;
+        hist[3 * st + o] = hist[2 * st + o];
+        hist[2 * st + o] = hist[st + o];
+        hist[st + o] = hist[o];
+        hist[o] = m[c];
+      }
     }
   }
+  energy_start(a, i, m);
 }
 
-__global__ void k_cg_state_out(const CGSys *cg, int nsys, int32_t *count, double *norm, int32_t *iters, double *resid,
-                               unsigned *status, int push, double tol) {
+__global__ void k_cg_state_out(const CGSys *cg, int nsys, StateOut out) {
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
   int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nsys) return;
-  const CGSys &G = cg[s];
-  if (push) { count[s] += 1; norm[s] = G.norm; }
-  if (iters) iters[s] = G.it;
-  if (resid) resid[s] = G.err;
-  if (G.err > tol && !G.iel_ext) atomicOr(&status[s], 0x2u);  // an extended iEL step stops short of tol by design
-}
-
-// Per-system start of a solve: which predictor start applies (forcefield.py:1951-1966).
-// mode 0: history predictor (compute); mode 1: the guess is the state's mu, plain start (energy,
-// forcefield.py:2606-2612).
-__global__ void k_cg_setup(CGSys *cg, int nsys, const int32_t *count, const double *norm, int K, int fused, int refresh,
-                           int mode, cudaGraphConditionalHandle plain, int use_cond, int use_nn = 0) {
-  pdl_enter();  // launched as a programmatic dependent of the previous kernel
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nsys) return;
-  CGSys &G = cg[s];
-  int c = count ? count[s] : 0;
-  G.have = mode == 1 ? 1 : (K > 0 && c >= K);
-  G.nn = use_nn && G.have;  // k_start1 adds the model's correction to the extrapolation
-  G.fallback = 0;
-  G.iel_ext = 0; G.iel_first = 0; G.maxit_s = -1; G.tol_s = -1.0;
-  G.fused = mode == 0 && G.have && fused && (c % refresh) != 0;
-  G.sweep2 = !G.fused;
-  if (use_cond && G.sweep2) cudaGraphSetConditional(plain, 1u);  // the plain start's sweep runs (default 0)
-  G.active = 0;
-  G.norm = G.fused ? norm[s] : 1.0;
-  G.acc_abs = 0; G.acc_rz = 0; G.acc_max = 0; G.acc_pap = 0; G.acc_num = 0;
+  if (s < nsys) cg_state_out(cg, s, out);
 }
 
 // Energy-only start: x0 = the state's mu, first sweep at d = p.
 template <typename T>
-__global__ void k_energy_start(Dev<T> a, const double *mu) {
+__global__ void k_energy_start(Dev<T> a, StartRule rule, const double *mu, cudaGraphConditionalHandle plain, int use_cond) {
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.nt) return;
+  const int s = a.sysid[i];
+  if (i == a.sys[s].atom0) cg_setup(a.cg[s], s, rule, plain, use_cond);
   double4 p = a.pperm[i];
   v4<T> d, x;
   d.x = T(p.x); d.y = T(p.y); d.z = T(p.z); d.w = a.q[i];
@@ -2062,6 +2112,7 @@ __global__ void __launch_bounds__(ATOMS_PER_BLOCK * QL, MINB) k_forces(Dev<T> a,
     // the pair loop
     int4 b = a.base[i];
     v4<T> fr = a.frac[i];
+    if (b.w && lane == 0) atomicOr(&a.status[s], 0x4u);  // a non-finite position
     if (lane < 3) {
       T th[P], dth[P], d2[P];
       bspline<T, P, true>(lane == 0 ? fr.x : (lane == 1 ? fr.y : fr.z), th, dth, d2);
@@ -2282,38 +2333,16 @@ __global__ void __launch_bounds__(ATOMS_PER_BLOCK * QL, MINB) k_forces(Dev<T> a,
   }
 }
 
-// Covalent-dipole frames: p_i = sum c unit(r_j - r_i); the pull-back of dE/dd_i onto r_i and r_j
-// (the vector-Jacobian product of forcefield.py:2412).  One thread per covalent dipole.
-template <typename T>
-__global__ void k_cov_forces(Dev<T> a) {
-  pdl_enter();  // launched as a programmatic dependent of the previous kernel
-  int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= a.ncov || !a.perm) return;
-  int i = a.cov_i_flat[m], j = a.cov_j_flat[m];
-  const BoxInfo &B = a.box[a.sysid[i]];
-  double vx = a.pos[3 * j] - a.pos[3 * i], vy = a.pos[3 * j + 1] - a.pos[3 * i + 1], vz = a.pos[3 * j + 2] - a.pos[3 * i + 2];
-  min_image(vx, vy, vz, B.H);
-  double l = sqrt(vx * vx + vy * vy + vz * vz);
-  double ux = vx / l, uy = vy / l, uz = vz / l;
-  double4 g = a.dEdd[i];
-  double ug = ux * g.x + uy * g.y + uz * g.z;
-  double c = a.cov_c_flat[m] / l;
-  double gx = c * (g.x - ux * ug), gy = c * (g.y - uy * ug), gz = c * (g.z - uz * ug);
-  atomicAdd(&a.forces[3 * j], -gx); atomicAdd(&a.forces[3 * j + 1], -gy); atomicAdd(&a.forces[3 * j + 2], -gz);
-  atomicAdd(&a.forces[3 * i], gx); atomicAdd(&a.forces[3 * i + 1], gy); atomicAdd(&a.forces[3 * i + 2], gz);
-}
-
 // Energies and virial of every system (forcefield.py:2011-2045, 2420-2430, lj.py:87-114):
 // E_elec = KE [rows/2 + U_rec + U_self + U_bg + U_pol], E_vdw = rows/2 + tail.
-__global__ void k_energy_finish(const SysInfo *sys, const BoxInfo *box, const EnergyAcc *E, int nsys, double beta, double c_self,
-                                double cutoff, int lj, int lj_lrc, int induce, double *energy, double *virial, unsigned *status,
-                                const EnergyAcc *E2 = nullptr, double omega = 1.0) {
-  pdl_enter();  // launched as a programmatic dependent of the previous kernel
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nsys) return;
-  const EnergyAcc &e = E[s];
-  const SysInfo &S = sys[s];
-  double vol = box[s].vol;
+template <typename T>
+__device__ __forceinline__ void energy_finish(const Dev<T> &a, int s, double *energy, double *virial, const EnergyAcc *E2, double omega) {
+  const double beta = a.beta, c_self = a.c_self, cutoff = a.cutoff;
+  const int lj = a.lj, lj_lrc = a.lj_lrc, induce = a.induce;
+  unsigned *status = a.status;
+  const EnergyAcc &e = a.eacc[s];
+  const SysInfo &S = a.sys[s];
+  double vol = a.box[s].vol;
   double uself = -(beta / SQRT_PI) * S.sum_q2 - 0.5 * c_self * e.d2;
   double urec_delta = 0.0;
   if (E2) {  // iEL/0-SCF shadow energy (forcefield.py:2037-2042)
@@ -2343,20 +2372,38 @@ __global__ void k_energy_finish(const SysInfo *sys, const BoxInfo *box, const En
   }
 }
 
-// d = p + mu (energy pass), in T.
+// Covalent-dipole frames: p_i = sum c unit(r_j - r_i); the pull-back of dE/dd_i onto r_i and r_j
+// (the vector-Jacobian product of forcefield.py:2412).  One thread per covalent dipole; the first threads
+// finish the systems' energies.
+template <typename T>
+__global__ void k_finish(Dev<T> a, double *energy, double *virial, const EnergyAcc *E2, double omega) {
+  pdl_enter();  // launched as a programmatic dependent of the previous kernel
+  int m = blockIdx.x * blockDim.x + threadIdx.x;
+  for (int s = m; s < a.nsys; s += gridDim.x * blockDim.x) energy_finish(a, s, energy, virial, E2, omega);
+  if (m >= a.ncov || !a.perm) return;
+  int i = a.cov_i_flat[m], j = a.cov_j_flat[m];
+  const BoxInfo &B = a.box[a.sysid[i]];
+  double vx = a.pos[3 * j] - a.pos[3 * i], vy = a.pos[3 * j + 1] - a.pos[3 * i + 1], vz = a.pos[3 * j + 2] - a.pos[3 * i + 2];
+  min_image(vx, vy, vz, B.H);
+  double l = sqrt(vx * vx + vy * vy + vz * vz);
+  double ux = vx / l, uy = vy / l, uz = vz / l;
+  double4 g = a.dEdd[i];
+  double ug = ux * g.x + uy * g.y + uz * g.z;
+  double c = a.cov_c_flat[m] / l;
+  double gx = c * (g.x - ux * ug), gy = c * (g.y - uy * ug), gz = c * (g.z - uz * ug);
+  atomicAdd(&a.forces[3 * j], -gx); atomicAdd(&a.forces[3 * j + 1], -gy); atomicAdd(&a.forces[3 * j + 2], -gz);
+  atomicAdd(&a.forces[3 * i], gx); atomicAdd(&a.forces[3 * i + 1], gy); atomicAdd(&a.forces[3 * i + 2], gz);
+}
+
+// d = p + mu (energy pass), in T; the energy accumulators of the pass start at zero.
 template <typename T>
 __global__ void k_total_dipoles(Dev<T> a, const double *mu) {
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  // the energy accumulators of the pass start at zero
-  constexpr int NACC = sizeof(EnergyAcc) / sizeof(double);
-  for (int t = i; t < NACC * a.nsys; t += gridDim.x * blockDim.x) reinterpret_cast<double *>(a.eacc)[t] = 0.0;
-  if (i >= a.nt) return;
-  double4 p = a.pperm[i];
-  double m0 = mu ? mu[3 * i] : 0.0, m1 = mu ? mu[3 * i + 1] : 0.0, m2 = mu ? mu[3 * i + 2] : 0.0;
-  v4<T> d;
-  d.x = T(p.x + m0); d.y = T(p.y + m1); d.z = T(p.z + m2); d.w = a.q[i];
-  a.D[i] = d;
+  double m[3] = {0, 0, 0};
+  if (mu && i < a.nt)
+    for (int c = 0; c < 3; ++c) m[c] = mu[3 * (size_t)i + c];
+  energy_start(a, i, m);
 }
 
 // Copy of a (N, 3) FP64 array into v4<T> (pgm_field input).
