@@ -136,8 +136,9 @@ struct EngineBase {
 
 // The tiles of one FFT pass launch: the systems with the same mesh length along the pass's axis.
 struct FftGroup {
-  int K = 0;
-  DBuf<pgmfft::Tile> tiles;
+  int K = 0, ntiles = 0;
+  DBuf<pgmfft::Tile> table;
+  pgmfft::Tiles tiles{};
 };
 
 // Autotuner choices, shared by the handles of one process with the same precision, spline
@@ -173,7 +174,7 @@ struct Engine : EngineBase {
   DBuf<pgm::CGSys> d_cg;
   DBuf<pgm::EnergyAcc> d_eacc;
   DBuf<unsigned> d_status;
-  DBuf<int> wb_sys, wb_atom0, qb_sys, qb_atom0, tb_sys, tb_atom0;
+  DBuf<int4> wb, qb, tb;
   DBuf<int> sysid, molid, molfirst, molend, mol_start, cov_start, cov_j, cov_i_flat, cov_j_flat;
   DBuf<T> q, radius, alpha, ialpha, rminh, seps;
   DBuf<pgm::c2<T>> ljp;
@@ -267,7 +268,8 @@ struct Engine : EngineBase {
     a.c_self = 4.0 * std::pow(set.ewald_beta, 3) / (3.0 * pgm::SQRT_PI);
     a.tol = set.dipole_tol; a.peek = set.peek; a.max_iter = set.max_iter;
     a.sys = d_sys.p; a.box = d_box.p; a.cg = d_cg.p; a.eacc = d_eacc.p; a.status = status;
-    a.wb_sys = wb_sys.p; a.wb_atom0 = wb_atom0.p; a.qb_sys = qb_sys.p; a.qb_atom0 = qb_atom0.p; a.tb_sys = tb_sys.p; a.tb_atom0 = tb_atom0.p;
+    a.wb = wb.p; a.qb = qb.p; a.tb = tb.p;
+    for (int ax = 0; ax < 3; ++ax) a.K0[ax] = hsys[0].K[ax];
     a.sysid = sysid.p; a.molid = molid.p; a.molfirst = molfirst.p; a.molend = molend.p; a.mol_start = mol_start.p;
     a.q = q.p; a.radius = radius.p; a.alpha = alpha.p; a.ialpha = ialpha.p; a.rminh = rminh.p; a.seps = seps.p;
     a.ljp = ljp.p;
@@ -443,17 +445,18 @@ struct Engine : EngineBase {
     cc_auto = std::max(32, (int)std::ceil((shell * 1.25 + 32.0) / 32.0) * 32);
     cc = set.list_capacity > 0 ? ((set.list_capacity + 31) / 32) * 32 : cc_auto;
     // block maps
-    std::vector<int> wbs, wba, qbs, qba, tbs, tba;
-    for (int si = 0; si < n; ++si) {
-      const pgm::SysInfo &S = hsys[si];
-      for (int a = 0; a < S.natom; a += pgm::WARPS_PER_BLOCK) { wbs.push_back(si); wba.push_back(S.atom0 + a); }
-      for (int a = 0; a < S.natom; a += pgm::ATOMS_PER_BLOCK) { qbs.push_back(si); qba.push_back(S.atom0 + a); }
-      for (int a = 0; a < S.natom; a += pgm::THREADS_PER_BLOCK) { tbs.push_back(si); tba.push_back(S.atom0 + a); }
-    }
-    nwblk = (int)wbs.size();
-    nqblk = (int)qbs.size();
-    ntblk = (int)tbs.size();
-    wb_sys.upload(wbs); wb_atom0.upload(wba); qb_sys.upload(qbs); qb_atom0.upload(qba); tb_sys.upload(tbs); tb_atom0.upload(tba);
+    auto block_map = [&](int per, DBuf<int4> &map) {
+      std::vector<int4> v;
+      for (int si = 0; si < n; ++si) {
+        const pgm::SysInfo &S = hsys[si];
+        for (int a = 0; a < S.natom; a += per) v.push_back(make_int4(si, S.atom0 + a, S.atom0 + S.natom, 0));
+      }
+      map.upload(v);
+      return (int)v.size();
+    };
+    nwblk = block_map(pgm::WARPS_PER_BLOCK, wb);
+    nqblk = block_map(pgm::ATOMS_PER_BLOCK, qb);
+    ntblk = block_map(pgm::THREADS_PER_BLOCK, tb);
     // plane passes for the systems whose K2 = K3 plane fits in a CTA's shared memory; the others run
     // the k3 and k2 passes
     int cur_dev = 0, smem_optin = 0;
@@ -500,7 +503,27 @@ struct Engine : EngineBase {
       for (auto &kv : by) {
         std::unique_ptr<FftGroup> g(new FftGroup());
         g->K = kv.first;
-        g->tiles.upload(kv.second);
+        g->ntiles = (int)kv.second.size();
+        g->table.upload(kv.second);
+        pgmfft::Tiles &t = g->tiles;
+        t.table = g->table.p;
+        if (n == 1) {
+          const pgm::SysInfo &S = hsys[0];
+          t.one = 1;
+          t.base = kv.second[0];
+          if (planes) {
+            t.r_step = (long long)S.K[1] * S.K[2];
+            t.g_step = (long long)S.K[1] * S.K3h;
+          } else if (axis == 2) {
+            t.c_step = 2 * tc;
+            t.lines = S.K[0] * S.K[1];
+            t.base.n = tc;
+          } else {
+            t.c_step = tc;
+            t.share = t.base.q1;
+            t.total = (long long)S.K[0] * S.K[1] * S.K[2];
+          }
+        }
         out.push_back(std::move(g));
       }
     };
@@ -617,7 +640,7 @@ struct Engine : EngineBase {
                 int sign = 0) {
     const pgmfft::Args<T> f{a.Q, a.Phi, a.Ginf, a.C, a.tw, a.cg, a.box, a.eacc, a.beta};
     for (auto &g : groups) {
-      CK(pgmfft::launch<T>(p, g->K, f, g->tiles.p, (int)g->tiles.n, act, sign, st, true));
+      CK(pgmfft::launch<T>(p, g->K, f, g->tiles, g->ntiles, act, sign, st, true));
       ++launches;
     }
   }
@@ -1152,6 +1175,12 @@ struct Engine : EngineBase {
     CK(cudaStreamEndCapture(side, &bg));
   }
 
+  // CG iterations of a captured solve unrolled in front of its while node: the last host-driven solve's - 2, at
+  // most 3.  An unrolled iteration saves 1 to 2 us over one in the node, and one that finds every system
+  // converged costs 9 us (512 waters) to 30 us (24 boxes), so a count from a plain start (12 and more)
+  // must not set it for the predicted starts that follow (3 to 8).
+  int unroll_count() const { return std::max(0, std::min({last_iters - 2, 3, set.max_iter})); }
+
   bool any_active(cudaStream_t st) {
     CK(cudaMemcpyAsync(h_any, dany.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
@@ -1244,7 +1273,7 @@ struct Engine : EngineBase {
     }
     if (captured) {
       // captured: the first U iterations as plain kernel nodes (their kernels skip systems that
-      // have converged; U = the iterations of the last host-driven solve - 2), then a conditional
+      // have converged; unroll_count()), then a conditional
       // while node whose body is one CG iteration.  The last check before the node and the body's
       // last kernel set the condition to "some system still iterating" (max_iter on the device).
       cudaGraph_t g;
@@ -1252,7 +1281,7 @@ struct Engine : EngineBase {
       size_t nd = 0;
       unsigned long long id;
       CK(cudaStreamGetCaptureInfo(st, &cs, &id, &g, &deps, &nd));
-      const int U = std::max(0, std::min(last_iters - 2, set.max_iter));
+      const int U = unroll_count();
       cudaGraphConditionalHandle cond;
       CK(cudaGraphConditionalHandleCreate(&cond, g, U > 0 ? 0 : 1, cudaGraphCondAssignDefault));
       for (int k = 0; k < U; ++k) iteration(st, a, cond, k == U - 1 ? 1 : 0);
@@ -1312,7 +1341,7 @@ struct Engine : EngineBase {
       unsigned long long id;
       CK(cudaStreamGetCaptureInfo(st, &cs, &id, &g, &deps, &nd));
       CK(cudaGraphConditionalHandleCreate(&cond2, g, 0, cudaGraphCondAssignDefault));
-      U = std::max(0, std::min(last_iters - 2, set.max_iter));
+      U = unroll_count();
       CK(cudaGraphConditionalHandleCreate(&cond, g, 0, cudaGraphCondAssignDefault));
     }
     launch_pdl(pgm::k_iel_setup, nsys, 256, 0, st, d_cg.p, (const pgm::SysInfo *)d_sys.p, nsys, (const int32_t *)ind->count,

@@ -43,6 +43,16 @@ struct Tile {
   long long rg, cg, q0, q1;
 };
 
+// The tiles of a launch: a table, or, with one system, `base` and what follows from the block index --
+// c0 = b c_step, rg + b r_step, cg + b g_step, pairs left of `lines`, the share of b -- so that a pass does not
+// begin with a load that its other loads wait for.
+struct Tiles {
+  const Tile *table;
+  int one, c_step, lines, pad;
+  long long r_step, g_step, share, total;
+  Tile base;
+};
+
 // Passes of a convolution.
 enum Pass { X_FWD, X_INV, Y_PASS, Z_CONV, Z_ENERGY, PLANE_FWD, PLANE_INV };
 
@@ -60,6 +70,6 @@ template <typename T>
 cudaError_t prepare(Pass p, int N);
 // One launch of pass p over `ntiles` tiles; sign is the k2 pass's direction (-1 forward).
 template <typename T>
-cudaError_t launch(Pass p, int N, const Args<T> &a, const Tile *tiles, int ntiles, int act, int sign, cudaStream_t st, bool dependent);
+cudaError_t launch(Pass p, int N, const Args<T> &a, const Tiles &tiles, int ntiles, int act, int sign, cudaStream_t st, bool dependent);
 
 }  // namespace pgmfft

@@ -14,6 +14,6 @@ size_t plane_smem(int N, size_t real_size) {
 
 template bool supported<float>(int);
 template cudaError_t prepare<float>(Pass, int);
-template cudaError_t launch<float>(Pass, int, const Args<float> &, const Tile *, int, int, int, cudaStream_t, bool);
+template cudaError_t launch<float>(Pass, int, const Args<float> &, const Tiles &, int, int, int, cudaStream_t, bool);
 
 }  // namespace pgmfft

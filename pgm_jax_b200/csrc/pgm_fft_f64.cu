@@ -5,6 +5,6 @@ namespace pgmfft {
 
 template bool supported<double>(int);
 template cudaError_t prepare<double>(Pass, int);
-template cudaError_t launch<double>(Pass, int, const Args<double> &, const Tile *, int, int, int, cudaStream_t, bool);
+template cudaError_t launch<double>(Pass, int, const Args<double> &, const Tiles &, int, int, int, cudaStream_t, bool);
 
 }  // namespace pgmfft

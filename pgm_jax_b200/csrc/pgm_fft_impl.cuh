@@ -162,6 +162,19 @@ __device__ __forceinline__ bool pass_active(const CGSys *cg, int s, int act) {
   return act == 0 || (act == 1 && cg[s].active) || (act == 2 && cg[s].sweep2) || (act == 3 && cg[s].fallback);
 }
 
+__device__ __forceinline__ Tile tile_of(const Tiles &ts) {
+  if (!ts.one) return ts.table[blockIdx.x];
+  Tile t = ts.base;
+  const int b = blockIdx.x;
+  t.c0 = b * ts.c_step;
+  t.rg += b * ts.r_step;
+  t.cg += b * ts.g_step;
+  if (ts.lines) t.n = min(t.n, (ts.lines - t.c0) / 2);
+  t.q0 = min(ts.total, b * ts.share);
+  t.q1 = min(ts.total, (b + 1) * ts.share);
+  return t;
+}
+
 // ------------------------------------------------------------------ k3 passes
 // Two real lines packed as one complex line (z = a + i b).  Threads of a pair are consecutive, so
 // a pair's N2 loads of one n1 are contiguous; the shared line has an odd inner stride (N2 | 1) so that
@@ -173,21 +186,23 @@ struct XShape {
 };
 
 template <typename T, int N>
-__global__ void __launch_bounds__(XShape<T, N>::THREADS, min_blocks<T>(XShape<T, N>::THREADS, N1R<N>)) k_x_fwd(Args<T> a, const Tile *__restrict__ tiles, int act) {
+__global__ void __launch_bounds__(XShape<T, N>::THREADS, min_blocks<T>(XShape<T, N>::THREADS, N1R<N>)) k_x_fwd(Args<T> a, Tiles tiles, int act) {
   using X = XShape<T, N>;
   constexpr int N1 = X::N1, N2 = X::N2, Kh = N / 2 + 1;
   pgm::pdl_enter();
   __shared__ __align__(16) unsigned char raw[X::ELEMS * sizeof(c2<T>)];
   c2<T> *sh = reinterpret_cast<c2<T> *>(raw);
-  const Tile t = tiles[blockIdx.x];
-  if (!pass_active(a.cg, t.s, act)) return;
+  const Tile t = tile_of(tiles);
   const int p = threadIdx.x / N1, r = threadIdx.x - p * N1;
   const bool on = p < t.n;
+  c2<T> v[N1];  // loaded before the test of the system's flag
   if (on && r < N2) {
     const T *qa = a.Q + t.rg + (size_t)(t.c0 + 2 * p) * N + r, *qb = qa + N;
-    c2<T> v[N1];
 #pragma unroll
     for (int k = 0; k < N1; ++k) { v[k].x = qa[N2 * k]; v[k].y = qb[N2 * k]; }
+  }
+  if (!pass_active(a.cg, t.s, act)) return;
+  if (on && r < N2) {
     step1<T, N>(v, r, a.tw + t.tw);
 #pragma unroll
     for (int k = 0; k < N1; ++k) sh[p * X::PS + k * X::S2 + r] = v[k];
@@ -224,13 +239,13 @@ __device__ __forceinline__ c2<T> tangled(c2<T> A, c2<T> B, int mm, bool up) {
 }
 
 template <typename T, int N>
-__global__ void __launch_bounds__(XShape<T, N>::THREADS, min_blocks<T>(XShape<T, N>::THREADS, N1R<N>)) k_x_inv(Args<T> a, const Tile *__restrict__ tiles, int act) {
+__global__ void __launch_bounds__(XShape<T, N>::THREADS, min_blocks<T>(XShape<T, N>::THREADS, N1R<N>)) k_x_inv(Args<T> a, Tiles tiles, int act) {
   using X = XShape<T, N>;
   constexpr int N1 = X::N1, N2 = X::N2, Kh = N / 2 + 1;
   pgm::pdl_enter();
   __shared__ __align__(16) unsigned char raw[X::ELEMS * sizeof(c2<T>)];
   c2<T> *sh = reinterpret_cast<c2<T> *>(raw);
-  const Tile t = tiles[blockIdx.x];
+  const Tile t = tile_of(tiles);
   if (!pass_active(a.cg, t.s, act)) return;
   const int p = threadIdx.x / N1, r = threadIdx.x - p * N1;
   const bool on = p < t.n;
@@ -268,23 +283,24 @@ struct YShape {
 };
 
 template <typename T, int N>
-__global__ void __launch_bounds__(YShape<T, N>::THREADS, min_blocks<T>(YShape<T, N>::THREADS, N1R<N>)) k_y(Args<T> a, const Tile *__restrict__ tiles, int act, int sign) {
+__global__ void __launch_bounds__(YShape<T, N>::THREADS, min_blocks<T>(YShape<T, N>::THREADS, N1R<N>)) k_y(Args<T> a, Tiles tiles, int act, int sign) {
   using Y = YShape<T, N>;
   constexpr int N1 = Y::N1, N2 = Y::N2, TC = Y::TC;
   pgm::pdl_enter();
   __shared__ __align__(16) unsigned char raw[N * TC * sizeof(c2<T>)];
   c2<T> *sh = reinterpret_cast<c2<T> *>(raw);
-  const Tile t = tiles[blockIdx.x];
-  if (!pass_active(a.cg, t.s, act)) return;
+  const Tile t = tile_of(tiles);
   const int r = threadIdx.x / TC, c = threadIdx.x - r * TC, col = t.c0 + c;
   const bool on = col < t.n;
   const int k1 = col / t.K3h, m3 = col - k1 * t.K3h;
   const size_t rs = t.K3h;
   c2<T> *C = a.C + t.cg + (size_t)k1 * N * rs + m3;
-  if (on && r < N2) {
-    c2<T> v[N1];
+  c2<T> v[N1];  // loaded before the test of the system's flag
+  if (on && r < N2)
 #pragma unroll
     for (int k = 0; k < N1; ++k) v[k] = C[(r + N2 * k) * rs];
+  if (!pass_active(a.cg, t.s, act)) return;
+  if (on && r < N2) {
     if (sign > 0)
 #pragma unroll
       for (int k = 0; k < N1; ++k) v[k] = swapped<T>(v[k]);
@@ -314,14 +330,13 @@ __global__ void __launch_bounds__(YShape<T, N>::THREADS, min_blocks<T>(YShape<T,
 // pme.py:370-376), inverse.  With ENERGY the reciprocal energy sum w3 G |F|^2 (pme.py:390-411) and
 // the influence part of the virial are accumulated.
 template <typename T, int N, bool ENERGY>
-__global__ void __launch_bounds__(YShape<T, N>::THREADS, min_blocks<T>(YShape<T, N>::THREADS, N1R<N> + (ENERGY ? 32 : 16))) k_z(Args<T> a, const Tile *__restrict__ tiles, int act) {
+__global__ void __launch_bounds__(YShape<T, N>::THREADS, min_blocks<T>(YShape<T, N>::THREADS, N1R<N> + (ENERGY ? 32 : 16))) k_z(Args<T> a, Tiles tiles, int act) {
   using Y = YShape<T, N>;
   constexpr int N1 = Y::N1, N2 = Y::N2, TC = Y::TC;
   pgm::pdl_enter();
   __shared__ __align__(16) unsigned char raw[N * TC * sizeof(c2<T>)];
   c2<T> *sh = reinterpret_cast<c2<T> *>(raw);
-  const Tile t = tiles[blockIdx.x];
-  if (!pass_active(a.cg, t.s, act)) return;
+  const Tile t = tile_of(tiles);
   const int r = threadIdx.x / TC, c = threadIdx.x - r * TC, col = t.c0 + c;
   const bool on = col < t.n;
   const size_t rs = t.n;
@@ -333,6 +348,7 @@ __global__ void __launch_bounds__(YShape<T, N>::THREADS, min_blocks<T>(YShape<T,
   if (on && r < N2)
 #pragma unroll
     for (int k = 0; k < N1; ++k) v[k] = C[(r + N2 * k) * rs];
+  if (!pass_active(a.cg, t.s, act)) return;  // after the loads
 #pragma unroll
   for (int k = 0; k < N2; ++k) g[k] = on ? G[(r + N1 * k) * rs] : T(0);
   if (on && r < N2) {
@@ -429,13 +445,13 @@ struct PlaneShape {
 };
 
 template <typename T, int N>
-__global__ void __launch_bounds__(PlaneShape<N>::THREADS) k_plane_fwd(Args<T> a, const Tile *__restrict__ tiles, int act) {
+__global__ void __launch_bounds__(PlaneShape<N>::THREADS) k_plane_fwd(Args<T> a, Tiles tiles, int act) {
   using S = PlaneShape<N>;
   constexpr int N1 = S::N1, N2 = S::N2, Kh = S::Kh, NP = S::NP;
   pgm::pdl_enter();
   extern __shared__ __align__(16) unsigned char raw[];
   c2<T> *A = reinterpret_cast<c2<T> *>(raw), *B = A + S::REG_A;
-  const Tile t = tiles[blockIdx.x];
+  const Tile t = tile_of(tiles);
   if (!pass_active(a.cg, t.s, act)) return;
   const c2<T> *tw = a.tw + t.tw;
   T *Q = a.Q + t.rg;
@@ -491,13 +507,13 @@ __global__ void __launch_bounds__(PlaneShape<N>::THREADS) k_plane_fwd(Args<T> a,
 }
 
 template <typename T, int N>
-__global__ void __launch_bounds__(PlaneShape<N>::THREADS) k_plane_inv(Args<T> a, const Tile *__restrict__ tiles, int act) {
+__global__ void __launch_bounds__(PlaneShape<N>::THREADS) k_plane_inv(Args<T> a, Tiles tiles, int act) {
   using S = PlaneShape<N>;
   constexpr int N1 = S::N1, N2 = S::N2, Kh = S::Kh, NP = S::NP;
   pgm::pdl_enter();
   extern __shared__ __align__(16) unsigned char raw[];
   c2<T> *A = reinterpret_cast<c2<T> *>(raw), *B = A + S::REG_A;
-  const Tile t = tiles[blockIdx.x];
+  const Tile t = tile_of(tiles);
   if (!pass_active(a.cg, t.s, act)) return;
   const c2<T> *tw = a.tw + t.tw;
   const c2<T> *C = a.C + t.cg;
@@ -600,7 +616,7 @@ cudaError_t prepare(Pass p, int N) {
 }
 
 template <typename T>
-cudaError_t launch(Pass p, int N, const Args<T> &a, const Tile *tiles, int ntiles, int act, int sign, cudaStream_t st, bool dependent) {
+cudaError_t launch(Pass p, int N, const Args<T> &a, const Tiles &tiles, int ntiles, int act, int sign, cudaStream_t st, bool dependent) {
   cudaError_t e = cudaErrorInvalidValue;
   with_length(N, [&](auto Lc) {
     constexpr int L = decltype(Lc)::value;

@@ -40,8 +40,9 @@ struct Dev {
   CGSys *cg;
   EnergyAcc *eacc;
   unsigned *status;
-  // block maps (warp-per-atom and thread-per-atom kernels)
-  const int *wb_sys, *wb_atom0, *qb_sys, *qb_atom0, *tb_sys, *tb_atom0;  // 8, 32, 256 atoms per block
+  // block maps of 8, 32 and 256 atoms per block: (system, first atom, end of the system's atoms)
+  const int4 *wb, *qb, *tb;
+  int K0[3];  // the mesh of the first system (all there is, often: see where())
   // atoms
   const int *sysid, *molid, *molfirst, *molend, *mol_start;
   const T *q, *radius, *alpha, *ialpha, *rminh, *seps;
@@ -106,6 +107,36 @@ struct Dev {
   double *forces;
   double4 *dEdd;
 };
+
+// The system and atom of thread group `sub` of a block, and the end of the system's atoms.  With one system
+// they follow from the block index and the kernel's arguments; the map and the system table would be two
+// dependent loads at the head of every kernel of a latency-bound step (a load is 0.3 us from a cold L1).
+struct Where {
+  int s, i, end;
+};
+template <typename T>
+__device__ __forceinline__ Where where(const Dev<T> &a, const int4 *map, int block, int per, int sub) {
+  if (a.nsys == 1) return Where{0, block * per + sub, a.nt};
+  const int4 m = map[block];
+  return Where{m.x, m.y + sub, m.z};
+}
+template <typename T>
+__device__ __forceinline__ int system_of(const Dev<T> &a, int i) { return a.nsys == 1 ? 0 : a.sysid[i]; }
+// Whether a pass of the solve takes part in system s: act 0 always, 1 iterating, 2 plain start, 3 fallback.
+template <typename T>
+__device__ __forceinline__ bool solve_active(const Dev<T> &a, int s, int act) {
+  return act == 0 || (act == 1 && a.cg[s].active) || (act == 2 && a.cg[s].sweep2) || (act == 3 && a.cg[s].fallback);
+}
+struct Mesh {
+  int K1, K2, K3;
+  long long r0;
+};
+template <typename T>
+__device__ __forceinline__ Mesh mesh_of(const Dev<T> &a, int s) {
+  if (a.nsys == 1) return Mesh{a.K0[0], a.K0[1], a.K0[2], 0};
+  const SysInfo &S = a.sys[s];
+  return Mesh{S.K[0], S.K[1], S.K[2], S.rgrid0};
+}
 
 // A chunk of 32 row entries: 32 each of k, x, y, z, G1, G2, G0, G3, so that a warp writes or reads
 // every array of a chunk at constant offsets from one address (separate arrays took a 64-bit address each:
@@ -176,12 +207,12 @@ template <typename T>
 __global__ void k_prep(Dev<T> a, const double *boxes) {
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
   __shared__ BoxInfo B;
-  const int s = a.tb_sys[blockIdx.x];
+  const Where w = where(a, a.tb, blockIdx.x, THREADS_PER_BLOCK, threadIdx.x);
+  const int s = w.s, i = w.i;
   const SysInfo &S = a.sys[s];
-  const int a0 = a.tb_atom0[blockIdx.x], i = a0 + threadIdx.x;
-  if (threadIdx.x == 0) box_setup(a, s, boxes + 9 * (size_t)s, B, a0 == S.atom0);
+  if (threadIdx.x == 0) box_setup(a, s, boxes + 9 * (size_t)s, B, i == S.atom0);
   __syncthreads();
-  if (i >= S.atom0 + S.natom) return;
+  if (i >= w.end) return;
   double px = a.pos[3 * i], py = a.pos[3 * i + 1], pz = a.pos[3 * i + 2];
   double uc[3];
   int4 b;
@@ -253,7 +284,7 @@ __global__ void k_cell_assign(Dev<T> a) {
   if (!*a.nb_flag) return;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.nt) return;
-  int s = a.sysid[i];
+  int s = system_of(a, i);
   const SysInfo &S = a.sys[s];
   const BoxInfo &B = a.box[s];
   double4 p = a.pos4[i];
@@ -321,10 +352,10 @@ __global__ void __launch_bounds__(256) k_cand(Dev<T> a) {
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
   if (!*a.nb_flag) return;
   int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int s = a.wb_sys[blockIdx.x];
-  int i = a.wb_atom0[blockIdx.x] + warp;
+  const Where at = where(a, a.wb, blockIdx.x, WARPS_PER_BLOCK, warp);
+  const int s = at.s, i = at.i;
+  if (i >= at.end) return;
   const SysInfo &S = a.sys[s];
-  if (i >= S.atom0 + S.natom) return;
   const BoxInfo &B = a.box[s];
   double H[9], id[3];
 #pragma unroll
@@ -518,10 +549,10 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_rows(Dev<T> a) 
   __shared__ RowQueue<T> queues[WARPS_PER_BLOCK];
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int s = a.wb_sys[blockIdx.x];
-  const int i = a.wb_atom0[blockIdx.x] + warp;
+  const Where at = where(a, a.wb, blockIdx.x, WARPS_PER_BLOCK, warp);
+  const int s = at.s, i = at.i;
+  if (i >= at.end) return;
   const SysInfo &S = a.sys[s];
-  if (i >= S.atom0 + S.natom) return;
   RowQueue<T> &q = queues[warp];
   const unsigned lt = (1u << lane) - 1u;
   const T Ri2 = T(2) * a.radius[i] * a.radius[i], beta = T(a.beta);
@@ -760,40 +791,39 @@ __global__ void __launch_bounds__(ATOMS_PER_BLOCK * QL) k_spread(Dev<T> a, const
   __shared__ c2<T> sh[ATOMS_PER_BLOCK][3][P];  // per atom of the block: weight and derivative
   const int sub = threadIdx.x / QL, lane = threadIdx.x % QL;  // the atom's group of lanes
   const unsigned gm = group_mask<QL>();
-  const int s = a.qb_sys[blockIdx.x];
-  const int i = a.qb_atom0[blockIdx.x] + sub;
-  const SysInfo &S = a.sys[s];
-  if (i >= S.atom0 + S.natom) return;
-  if (ACT == 1 && !a.cg[s].active) return;
-  if (ACT == 2 && !a.cg[s].sweep2) return;
-  if (ACT == 3 && !a.cg[s].fallback) return;
+  const Where wh = where(a, a.qb, blockIdx.x, ATOMS_PER_BLOCK, sub);
+  const int s = wh.s, i = wh.i;
+  if (i >= wh.end) return;
+  // the loads go out before the test of the system's flag
   const int4 b = a.base[i];
   const v4<T> f = a.frac[i];
+  const v4<T> z = UPDATE_P ? a.Z[i] : vin[i], p = a.P[i];
+  const Mesh M = mesh_of(a, s);
+  if (!solve_active(a, s, ACT)) return;
   v4<T> d;
   if (UPDATE_P) {
-    v4<T> z = a.Z[i], p = a.P[i];
     T bt = T(a.cg[s].beta);
     d.x = z.x + bt * p.x; d.y = z.y + bt * p.y; d.z = z.z + bt * p.z; d.w = T(0);
     __syncwarp(gm);
     if (lane == 0) a.P[i] = d;
   } else {
-    d = vin[i];
+    d = z;
   }
   const BoxInfo &B = a.box[s];
-  const int K1 = S.K[0], K2 = S.K[1], K3 = S.K[2];
+  const int K1 = M.K1, K2 = M.K2, K3 = M.K3;
   T e = 0;
   if (lane < 3) {
     T th[P], dth[P];
     bspline<T, P, false>(lane == 0 ? f.x : (lane == 1 ? f.y : f.z), th, dth, nullptr);
 #pragma unroll
     for (int k = 0; k < P; ++k) { sh[sub][lane][k].x = th[k]; sh[sub][lane][k].y = dth[k]; }
-    e = T((double(d.x) * B.Hinv[lane] + double(d.y) * B.Hinv[3 + lane] + double(d.z) * B.Hinv[6 + lane]) * S.K[lane]);
+    e = T((double(d.x) * B.Hinv[lane] + double(d.y) * B.Hinv[3 + lane] + double(d.z) * B.Hinv[6 + lane]) * (lane == 0 ? K1 : lane == 1 ? K2 : K3));
   }
   const int l0 = (threadIdx.x & 31) & ~(QL - 1);
   const T e0 = __shfl_sync(gm, e, l0), e1 = __shfl_sync(gm, e, l0 + 1), e2 = __shfl_sync(gm, e, l0 + 2);
   __syncwarp(gm);
   const T qi = WITH_Q ? a.q[i] : T(0);
-  T *grid = a.Q + S.rgrid0;
+  T *grid = a.Q + M.r0;
   with_vec<T>(K3, [&](auto vw) {
     constexpr int VW = decltype(vw)::value;
     RowVectors<T, P, VW, 2> rv;
@@ -831,15 +861,12 @@ __global__ void __launch_bounds__(8 * LPR) k_rowfield(Dev<T> a, const v4<T> *__r
   // blocks of 8 rows (nvb of them); a grid smaller than nvb walks them at its stride (the row field
   // beside the FFT chain on a limited number of SMs)
   for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
-  int s = a.wb_sys[vb];
-  int i = a.wb_atom0[vb] + sub;
-  const SysInfo &S = a.sys[s];
-  if (ACT == 1 && !a.cg[s].active) continue;  // uniform over the block
-  if (ACT == 2 && !a.cg[s].sweep2) continue;
-  if (ACT == 3 && !a.cg[s].fallback) continue;
-  const bool valid = i < S.atom0 + S.natom;
-  if (LPR == 32 && !valid) continue;  // uniform over the warp
+  const Where wh = where(a, a.wb, vb, WARPS_PER_BLOCK, sub);
+  const int s = wh.s, i = wh.i;
+  const bool valid = i < wh.end;
   int n = valid ? min(a.rn[i], a.mce) : 0;
+  if (!solve_active(a, s, ACT)) continue;  // uniform over the block
+  if (LPR == 32 && !valid) continue;  // uniform over the warp
   unsigned char *row = row_of(a, valid ? i : 0);
   using C = RowChunk<T>;
   T f0 = 0, f1 = 0, f2 = 0;
@@ -915,20 +942,20 @@ __global__ void __launch_bounds__(ATOMS_PER_BLOCK * QL) k_gather(Dev<T> a, const
   __shared__ double red[ATOMS_PER_BLOCK];
   const int sub = threadIdx.x / QL, lane = threadIdx.x % QL;  // the atom's group of lanes
   const unsigned gm = group_mask<QL>();
-  const int s = a.qb_sys[blockIdx.x];
-  const int i = a.qb_atom0[blockIdx.x] + sub;
-  const SysInfo &S = a.sys[s];
-  const bool valid = i < S.atom0 + S.natom;
-  if (ACT == 1 && !a.cg[s].active) return;   // uniform over the block
-  if (ACT == 2 && !a.cg[s].sweep2) return;
-  if (ACT == 3 && !a.cg[s].fallback) return;
+  const Where wh = where(a, a.qb, blockIdx.x, ATOMS_PER_BLOCK, sub);
+  const int s = wh.s, i = wh.i;
+  const bool valid = i < wh.end;
+  // the loads go out before the test of the system's flag, and the assembly's are in flight during the stencil
+  const int il = valid ? i : wh.end - 1;
+  const int4 b = a.base[il];
+  const v4<T> fr = a.frac[il];
+  const v4<T> rowf = a.F[il], di = D[il];
+  const T ia = MODE == 1 ? a.ialpha[il] : T(0);
+  const Mesh M = mesh_of(a, s);
+  if (!solve_active(a, s, ACT)) return;   // uniform over the block
   double dotv = 0.0;
   if (valid) {
     const BoxInfo &B = a.box[s];
-    const int4 b = a.base[i];
-    const v4<T> fr = a.frac[i];
-    const v4<T> rowf = a.F[i], di = D[i];  // the assembly's loads are in flight during the stencil
-    const T ia = MODE == 1 ? a.ialpha[i] : T(0);
     if (lane < 3) {
       T th[P], dth[P];
       bspline<T, P, false>(lane == 0 ? fr.x : (lane == 1 ? fr.y : fr.z), th, dth, nullptr);
@@ -936,8 +963,8 @@ __global__ void __launch_bounds__(ATOMS_PER_BLOCK * QL) k_gather(Dev<T> a, const
       for (int k = 0; k < P; ++k) { sh[sub][lane][k].x = th[k]; sh[sub][lane][k].y = dth[k]; }
     }
     __syncwarp(gm);
-    const T *phi = a.Phi + S.rgrid0;
-    const int K1 = S.K[0], K2 = S.K[1], K3 = S.K[2];
+    const T *phi = a.Phi + M.r0;
+    const int K1 = M.K1, K2 = M.K2, K3 = M.K3;
     T g0 = 0, g1 = 0, g2 = 0;
     with_vec<T>(K3, [&](auto vw) {
       constexpr int VW = decltype(vw)::value;
@@ -976,7 +1003,7 @@ __global__ void __launch_bounds__(ATOMS_PER_BLOCK * QL) k_gather(Dev<T> a, const
 #pragma unroll
       for (int bb = 0; bb < 3; ++bb)
 #pragma unroll
-        for (int aa = 0; aa < 3; ++aa) es[bb * 3 + aa] = T(B.Hinv[bb * 3 + aa] * S.K[aa]);
+        for (int aa = 0; aa < 3; ++aa) es[bb * 3 + aa] = T(B.Hinv[bb * 3 + aa] * (aa == 0 ? K1 : aa == 1 ? K2 : K3));
       T r0 = g0 * es[0] + g1 * es[1] + g2 * es[2];
       T r1 = g0 * es[3] + g1 * es[4] + g2 * es[5];
       T r2 = g0 * es[6] + g1 * es[7] + g2 * es[8];
@@ -1042,10 +1069,10 @@ __global__ void __launch_bounds__(8 * LPA, 8 * 32 / LPA) k_nn_chan(Dev<T> a, con
   static_assert(LPA == 32 || LPA == 16 || LPA == 8, "lanes per atom");
   const int warp = threadIdx.x / LPA, lane = threadIdx.x % LPA;  // the atom's group of LPA lanes
   const unsigned gm = group_mask<LPA>();
-  int s = a.wb_sys[blockIdx.x];
-  int i = a.wb_atom0[blockIdx.x] + warp;
+  const Where at = where(a, a.wb, blockIdx.x, WARPS_PER_BLOCK, warp);
+  const int s = at.s, i = at.i;
+  if (i >= at.end) return;
   const SysInfo &S = a.sys[s];
-  if (i >= S.atom0 + S.natom) return;
   (void)rg;  // the graph radius is a.nn_rg2 here
   float f0 = 0.f, f1 = 0.f, f2 = 0.f;
   const float2 *G = a.nn_g + (size_t)i * a.nn_emax;
@@ -1154,10 +1181,10 @@ __global__ void __launch_bounds__(256, 4) k_nn_features(Dev<T> a, const float *c
                                                      int *valid) {
   int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (valid && blockIdx.x == 0 && threadIdx.x == 0) *valid = 1;  // read by the previous kernel only
-  int s = a.wb_sys[blockIdx.x];
-  int i = a.wb_atom0[blockIdx.x] + warp;
+  const Where at = where(a, a.wb, blockIdx.x, WARPS_PER_BLOCK, warp);
+  const int s = at.s, i = at.i;
+  if (i >= at.end) return;
   const SysInfo &S = a.sys[s];
-  if (i >= S.atom0 + S.natom) return;
   float *V = vec + (size_t)i * pgmnn::NN_CH * 3;
   float *F = inv + (size_t)i * pgmnn::NN_IN;
   const float is = 1.f / sigma, is2 = is * is;
@@ -1245,7 +1272,7 @@ __global__ void k_start1(Dev<T> a, StartRule rule, const double *hist, double c0
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.nt) return;
-  int s = a.sysid[i];
+  int s = system_of(a, i);
   const bool have = rule.have(s), fused = rule.is_fused(s);
   if (i == a.sys[s].atom0) cg_setup(a.cg[s], s, rule, plain, use_cond);
   double x0[3] = {0, 0, 0};
@@ -1365,13 +1392,13 @@ template <typename T, bool LOCAL>
 __global__ void k_start2(Dev<T> a, BeginArgs begin) {
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
   __shared__ double red[THREADS_PER_BLOCK / 32];
-  int s = a.tb_sys[blockIdx.x];
-  int i = a.tb_atom0[blockIdx.x] + threadIdx.x;
-  const SysInfo &S = a.sys[s];
+  const Where wh = where(a, a.tb, blockIdx.x, THREADS_PER_BLOCK, threadIdx.x);
+  const int s = wh.s;
+  const int i = wh.i;
   CGSys &G = a.cg[s];
   const bool fused = G.fused;  // uniform over the block
   double sab = 0.0, rz = 0.0, m = 0.0;
-  if (i < S.atom0 + S.natom) {
+  if (i < wh.end) {
     v4<T> b = a.B[i];
     v4<T> x = a.X[i];
     T al = a.alpha[i];
@@ -1415,7 +1442,7 @@ __global__ void k_start3(Dev<T> a) {
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.nt) return;
-  int s = a.sysid[i];
+  int s = system_of(a, i);
   if (a.cg[s].fused) return;
   v4<T> b = a.B[i], ap = a.AP[i], r;
   r.x = b.x - ap.x; r.y = b.y - ap.y; r.z = b.z - ap.z; r.w = T(0);
@@ -1430,12 +1457,12 @@ __global__ void k_start3(Dev<T> a) {
 template <typename T, bool FB, bool LOCAL>
 __global__ void k_cg_init(Dev<T> a, const float *delta, BeginArgs begin) {
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
-  int s = a.tb_sys[blockIdx.x];
+  const Where wh = where(a, a.tb, blockIdx.x, THREADS_PER_BLOCK, threadIdx.x);
+  const int s = wh.s;
   if (FB ? a.cg[s].fallback : !a.cg[s].fused) {  // uniform over the block
-    int i = a.tb_atom0[blockIdx.x] + threadIdx.x;
-    const SysInfo &S = a.sys[s];
+    const int i = wh.i;
     double rz = 0, m = 0;
-    if (i < S.atom0 + S.natom) {
+    if (i < wh.end) {
       v4<T> r = a.R[i];
       if (FB) {
         v4<T> ad = a.AP[i], x = a.X[i];
@@ -1465,7 +1492,7 @@ template <typename T>
 __global__ void k_fb_prep(Dev<T> a, const float *delta) {
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.nt || !a.cg[a.sysid[i]].fallback) return;
+  if (i >= a.nt || !a.cg[system_of(a, i)].fallback) return;
   v4<T> d;
   d.x = T(delta[3 * (size_t)i]); d.y = T(delta[3 * (size_t)i + 1]); d.z = T(delta[3 * (size_t)i + 2]); d.w = T(0);
   a.D[i] = d;
@@ -1479,16 +1506,16 @@ template <typename T>
 __device__ __forceinline__ void cg_update_body(Dev<T> &a) {
   __shared__ double red[2][THREADS_PER_BLOCK / 32];
   __shared__ unsigned long long mx[THREADS_PER_BLOCK / 32];
-  int s = a.tb_sys[blockIdx.x];
+  const Where wh = where(a, a.tb, blockIdx.x, THREADS_PER_BLOCK, threadIdx.x);
+  const int s = wh.s;
   CGSys &G = a.cg[s];
+  const int i = wh.i, il = min(i, wh.end - 1);
+  v4<T> x = a.X[il], r = a.R[il], p = a.P[il], ap = a.AP[il];  // out before the test of the system's flag
+  const T al = a.alpha[il];
   if (!G.active) return;  // the block's system has converged
-  int i = a.tb_atom0[blockIdx.x] + threadIdx.x;
-  const SysInfo &S = a.sys[s];
   double num = 0, rzn = 0, m = 0;
-  if (i < S.atom0 + S.natom) {
+  if (i < wh.end) {
     T st = T(G.rz / fmax(G.acc_pap, 1e-300));
-    v4<T> x = a.X[i], r = a.R[i], p = a.P[i], ap = a.AP[i];
-    T al = a.alpha[i];
     x.x += st * p.x; x.y += st * p.y; x.z += st * p.z;
     v4<T> rn, z;
     rn.x = r.x - st * ap.x; rn.y = r.y - st * ap.y; rn.z = r.z - st * ap.z; rn.w = T(0);
@@ -1598,13 +1625,13 @@ __device__ __forceinline__ bool lp_skip(int act, const CGSys &G) {
 template <typename T, int ACT>
 __global__ void k_lp_start(Dev<T> a) {
   pdl_enter();
-  const int s = a.tb_sys[blockIdx.x];
+  const Where wh = where(a, a.tb, blockIdx.x, THREADS_PER_BLOCK, threadIdx.x);
+  const int s = wh.s;
   CGSys &G = a.cg[s];
   if (lp_skip(ACT, G)) return;  // uniform over the block
-  const int i = a.tb_atom0[blockIdx.x] + threadIdx.x;
-  const SysInfo &S = a.sys[s];
+  const int i = wh.i;
   double rz = 0.0;
-  if (i < S.atom0 + S.natom) {
+  if (i < wh.end) {
     T f0 = 0, f1 = 0, f2 = 0;
     short_sum(a, i, [&](int k) {
       const v4<T> r = a.R[k];
@@ -1633,11 +1660,11 @@ __global__ void k_lp_start(Dev<T> a) {
 template <typename T, int ACT, bool FIRST>
 __global__ void k_lp_ap(Dev<T> a, const v4<T> *__restrict__ Pin, v4<T> *__restrict__ Pout) {
   pdl_enter();
-  const int s = a.tb_sys[blockIdx.x];
+  const Where wh = where(a, a.tb, blockIdx.x, THREADS_PER_BLOCK, threadIdx.x);
+  const int s = wh.s;
   CGSys &G = a.cg[s];
   if (lp_skip(ACT, G)) return;
-  const int i = a.tb_atom0[blockIdx.x] + threadIdx.x;
-  const SysInfo &S = a.sys[s];
+  const int i = wh.i;
   const T b = T(G.lb);
   auto pget = [&](int k) {
     v4<T> p = a.LZZ[k];
@@ -1648,7 +1675,7 @@ __global__ void k_lp_ap(Dev<T> a, const v4<T> *__restrict__ Pin, v4<T> *__restri
     return p;
   };
   double pap = 0.0;
-  if (i < S.atom0 + S.natom) {
+  if (i < wh.end) {
     T f0 = 0, f1 = 0, f2 = 0;
     short_sum(a, i, pget, f0, f1, f2);
     const v4<T> p = pget(i);
@@ -1671,14 +1698,14 @@ template <typename T, int ACT, bool LAST, int MODE>
 __global__ void k_lp_step(Dev<T> a, const v4<T> *__restrict__ Pcur, BeginArgs b, cudaGraphConditionalHandle cond, int use_cond) {
   pdl_enter();
   {
-    const int s = a.tb_sys[blockIdx.x];
+    const Where wh = where(a, a.tb, blockIdx.x, THREADS_PER_BLOCK, threadIdx.x);
+    const int s = wh.s;
     CGSys &G = a.cg[s];
     if (!lp_skip(ACT, G)) {
-      const int i = a.tb_atom0[blockIdx.x] + threadIdx.x;
-      const SysInfo &S = a.sys[s];
+      const int i = wh.i;
       const T al = T(G.acc_lrz / fmax(G.acc_lpap, 1e-300));
       double v0 = 0.0, v1 = 0.0;
-      if (i < S.atom0 + S.natom) {
+      if (i < wh.end) {
         const v4<T> p = Pcur[i];
         v4<T> z = a.Z[i];
         z.x += al * p.x; z.y += al * p.y; z.z += al * p.z;
@@ -1739,13 +1766,13 @@ template <typename T>
 __global__ void k_cg_update_r(Dev<T> a) {
   pdl_enter();
   __shared__ unsigned long long mx[THREADS_PER_BLOCK / 32];
-  const int s = a.tb_sys[blockIdx.x];
+  const Where wh = where(a, a.tb, blockIdx.x, THREADS_PER_BLOCK, threadIdx.x);
+  const int s = wh.s;
   CGSys &G = a.cg[s];
   if (!G.active) return;  // uniform over the block
-  const int i = a.tb_atom0[blockIdx.x] + threadIdx.x;
-  const SysInfo &S = a.sys[s];
+  const int i = wh.i;
   double m = 0.0;
-  if (i < S.atom0 + S.natom) {
+  if (i < wh.end) {
     const T st = T(G.rz / fmax(G.acc_pap, 1e-300));
     v4<T> x = a.X[i], r = a.R[i];
     const v4<T> p = a.P[i], ap = a.AP[i];
@@ -1838,7 +1865,7 @@ __global__ void k_energy_start(Dev<T> a, StartRule rule, const double *mu, cudaG
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.nt) return;
-  const int s = a.sysid[i];
+  const int s = system_of(a, i);
   if (i == a.sys[s].atom0) cg_setup(a.cg[s], s, rule, plain, use_cond);
   double4 p = a.pperm[i];
   v4<T> d, x;
@@ -1898,7 +1925,7 @@ __global__ void k_iel_start1(Dev<T> a, const double *xl, const double *mu) {
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.nt) return;
-  const CGSys &G = a.cg[a.sysid[i]];
+  const CGSys &G = a.cg[system_of(a, i)];
   double x0[3] = {0, 0, 0};
   for (int c = 0; c < 3; ++c) x0[c] = G.iel_first ? (G.have ? mu[3 * (size_t)i + c] : 0.0) : xl[3 * (size_t)i + c];
   double4 p = a.pperm[i];
@@ -1965,7 +1992,7 @@ __global__ void k_iel_delta(Dev<T> a, const double *xl, double omega, int block,
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= a.nmol) return;
   const int i0 = a.mol_start[m], nb = a.mol_start[m + 1] - i0;
-  CGSys &G = a.cg[a.sysid[i0]];
+  CGSys &G = a.cg[system_of(a, i0)];
   if (!G.iel_ext) {
     for (int i = i0; i < i0 + nb; ++i) Dl[i] = v4<T>{T(0), T(0), T(0), T(0)};
     return;
@@ -2038,7 +2065,7 @@ __global__ void k_iel_finish(Dev<T> a, double *mu, double *hist, double *xl, Iel
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.nt) return;
-  const CGSys &G = a.cg[a.sysid[i]];
+  const CGSys &G = a.cg[system_of(a, i)];
   const size_t st = (size_t)a.nt * 3;
   double m[3];
   if (G.iel_ext && co.zscf) {
@@ -2084,10 +2111,10 @@ __global__ void __launch_bounds__(ATOMS_PER_BLOCK * QL, MINB) k_forces(Dev<T> a,
   __shared__ double red[ATOMS_PER_BLOCK][16];
   const int sub = threadIdx.x / QL, lane = threadIdx.x % QL;  // the atom's group of lanes
   const unsigned gm = group_mask<QL>();
-  int s = a.qb_sys[blockIdx.x];
-  int i = a.qb_atom0[blockIdx.x] + sub;
-  const SysInfo &S = a.sys[s];
-  bool valid = i < S.atom0 + S.natom;
+  const Where wh = where(a, a.qb, blockIdx.x, ATOMS_PER_BLOCK, sub);
+  const int s = wh.s, i = wh.i;
+  const bool valid = i < wh.end;
+  const Mesh M = mesh_of(a, s);
   double vals[16];
   for (int k = 0; k < 16; ++k) vals[k] = 0.0;
   if (valid) {
@@ -2120,12 +2147,12 @@ __global__ void __launch_bounds__(ATOMS_PER_BLOCK * QL, MINB) k_forces(Dev<T> a,
       for (int k = 0; k < P; ++k) { sh[sub][0][lane][k] = th[k]; sh[sub][1][lane][k] = dth[k]; sh[sub][2][lane][k] = d2[k]; }
     }
     __syncwarp(gm);
-    auto scaled = [&](int bb, int aa) { return T(B.Hinv[bb * 3 + aa] * S.K[aa]); };  // dU/dr_b = sum_a g_a scaled(b, a)
+    auto scaled = [&](int bb, int aa) { return T(B.Hinv[bb * 3 + aa] * (aa == 0 ? M.K1 : aa == 1 ? M.K2 : M.K3)); };  // dU/dr_b = sum_a g_a scaled(b, a)
     {
     T es[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k) es[k] = scaled(k / 3, k % 3);
-    const int K1 = S.K[0], K2 = S.K[1], K3 = S.K[2];
+    const int K1 = M.K1, K2 = M.K2, K3 = M.K3;
     // The stencil rows of a potential: f(j1, A, B, C, D, E, F) with the row's sums along k3 (weights, first, second
     // derivatives: st, su, sv) times the k2 weights t2, u2, v2: A = t2 st, B = u2 st, C = t2 su, D = v2 st,
     // E = u2 su, F = t2 sv.
@@ -2156,7 +2183,7 @@ __global__ void __launch_bounds__(ATOMS_PER_BLOCK * QL, MINB) k_forces(Dev<T> a,
       const T f1 = Dli.x * es[1] + Dli.y * es[4] + Dli.z * es[7];
       const T f2 = Dli.x * es[2] + Dli.y * es[5] + Dli.z * es[8];
       T h0 = 0, h1 = 0, h2 = 0;
-      stencil(a.Phi2 + S.rgrid0, [&](int j1, T A, T Bv, T C, T Dv, T E, T F) {
+      stencil(a.Phi2 + M.r0, [&](int j1, T A, T Bv, T C, T Dv, T E, T F) {
         const T t1 = sh[sub][0][0][j1], u1 = sh[sub][1][0][j1], v1 = sh[sub][2][0][j1];
         h0 += f0 * v1 * A + f1 * u1 * Bv + f2 * u1 * C;
         h1 += f0 * u1 * Bv + f1 * t1 * Dv + f2 * t1 * E;
@@ -2170,7 +2197,7 @@ __global__ void __launch_bounds__(ATOMS_PER_BLOCK * QL, MINB) k_forces(Dev<T> a,
     const T e0 = di.x * es[0] + di.y * es[3] + di.z * es[6];
     const T e1 = di.x * es[1] + di.y * es[4] + di.z * es[7];
     const T e2 = di.x * es[2] + di.y * es[5] + di.z * es[8];
-    stencil(a.Phi + S.rgrid0, [&](int j1, T A, T Bv, T C, T Dv, T E, T F) {
+    stencil(a.Phi + M.r0, [&](int j1, T A, T Bv, T C, T Dv, T E, T F) {
       const T t1 = sh[sub][0][0][j1], u1 = sh[sub][1][0][j1], v1 = sh[sub][2][0][j1];
       const T qt = qi * t1 + e0 * u1, qu = qi * u1 + e0 * v1;
       ge0 += u1 * A;
@@ -2382,7 +2409,7 @@ __global__ void k_finish(Dev<T> a, double *energy, double *virial, const EnergyA
   for (int s = m; s < a.nsys; s += gridDim.x * blockDim.x) energy_finish(a, s, energy, virial, E2, omega);
   if (m >= a.ncov || !a.perm) return;
   int i = a.cov_i_flat[m], j = a.cov_j_flat[m];
-  const BoxInfo &B = a.box[a.sysid[i]];
+  const BoxInfo &B = a.box[system_of(a, i)];
   double vx = a.pos[3 * j] - a.pos[3 * i], vy = a.pos[3 * j + 1] - a.pos[3 * i + 1], vz = a.pos[3 * j + 2] - a.pos[3 * i + 2];
   min_image(vx, vy, vz, B.H);
   double l = sqrt(vx * vx + vy * vy + vz * vz);
