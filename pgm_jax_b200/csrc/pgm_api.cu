@@ -183,7 +183,8 @@ struct Engine : EngineBase {
   DBuf<pgm::v4<T>> frac, X, R, Z, Pv, AP, Bv, D, Fv, Fpv;
   DBuf<double4> pperm, off, dEdd;
   DBuf<int> cell_of, slot_of, cell_count, cell_start, cell_atoms;
-  DBuf<double4> spos, pos_ref, pos4;
+  DBuf<pgm::v4<T>> spos;
+  DBuf<double4> pos_ref, pos4;
   DBuf<float4> pos4f;  // mixed precision: wrapped FP32 positions for the row build
   DBuf<int> cand, ncand, nb_flag;
   DBuf<long long> nb_builds;

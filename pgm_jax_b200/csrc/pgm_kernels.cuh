@@ -56,7 +56,7 @@ struct Dev {
   v4<T> *frac;
   double4 *pperm, *off;
   int *cell_of, *slot_of, *cell_count, *cell_start, *cell_atoms;
-  double4 *spos;  // positions in cell order, .w = molecule
+  v4<T> *spos;  // positions in cell order (mixed: wrapped), .w = molecule
   const int *idx;
   int idx_width;
   // rows
@@ -339,14 +339,33 @@ __global__ void k_scatter(Dev<T> a) {
   if (i >= a.nt) return;
   int t = a.cell_start[a.cell_of[i]] + a.slot_of[i];
   a.cell_atoms[t] = i;
-  a.spos[t] = a.pos4[i];
+  if constexpr (sizeof(T) == 4) a.spos[t] = a.pos4f[i];
+  else a.spos[t] = a.pos4[i];
+}
+
+// FP32 sequential minimum image (the mixed-precision candidate list and row build).  Rounding to the
+// nearest integer by adding and subtracting 1.5 2^23 (wrapped positions: |argument| < 2): two
+// additions, where rintf is a conversion at a quarter of their rate.
+__device__ __forceinline__ float nearest_f(float x) { return __fadd_rn(__fadd_rn(x, 12582912.f), -12582912.f); }
+__device__ __forceinline__ void min_image_scan(double &x, double &y, double &z, const double *H, const double *id) {
+  min_image_fast(x, y, z, H, id);
+}
+__device__ __forceinline__ void min_image_scan(float &x, float &y, float &z, const float *H, const float *id) {
+  float n = nearest_f(z * id[2]);
+  x -= n * H[6]; y -= n * H[7]; z -= n * H[8];
+  n = nearest_f(y * id[1]);
+  x -= n * H[3]; y -= n * H[4];
+  n = nearest_f(x * id[0]);
+  x -= n * H[0];
 }
 
 // ------------------------------------------------------------------ Verlet candidate list
 // One warp per atom when the list is rebuilt: every atom of another molecule within
 // cutoff + skin, found through the cell list (cells within R along each axis), compacted by ballot;
 // the positions of the build are kept for the displacement test (the reference's neighbour list,
-// md/neighbors.py:169-304, rebuilt when an atom moved more than skin / 2).
+// md/neighbors.py:169-304, rebuilt when an atom moved more than skin / 2).  The lanes look up the
+// ranges of 32 cell columns at once (a column's range is a load that its atoms' loads wait for); mixed
+// precision tests FP32 displacements against a radius 1e-5 wider (they are good to 1e-6 nm).
 template <typename T>
 __global__ void __launch_bounds__(256) k_cand(Dev<T> a) {
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
@@ -357,13 +376,15 @@ __global__ void __launch_bounds__(256) k_cand(Dev<T> a) {
   if (i >= at.end) return;
   const SysInfo &S = a.sys[s];
   const BoxInfo &B = a.box[s];
-  double H[9], id[3];
+  T H[9], id[3];
 #pragma unroll
-  for (int k = 0; k < 9; ++k) H[k] = B.H[k];
-  id[0] = B.idiag[0]; id[1] = B.idiag[1]; id[2] = B.idiag[2];
-  double4 pi = a.pos4[i];
-  int mi = (int)pi.w;
-  double rl = a.cutoff + a.skin, rl2 = rl * rl;
+  for (int k = 0; k < 9; ++k) H[k] = T(B.H[k]);
+  id[0] = T(B.idiag[0]); id[1] = T(B.idiag[1]); id[2] = T(B.idiag[2]);
+  v4<T> pi;
+  if constexpr (sizeof(T) == 4) pi = a.pos4f[i];
+  else pi = a.pos4[i];
+  const double rl = (a.cutoff + a.skin) * (sizeof(T) == 4 ? 1.00001 : 1.0);
+  const T rl2 = T(rl * rl);
   int *out = a.cand + (size_t)i * a.cc;
   int count = 0;
   int cell = a.cell_of[i] - S.cell0;
@@ -372,47 +393,84 @@ __global__ void __launch_bounds__(256) k_cand(Dev<T> a) {
   int R0 = B.R[0], R1 = B.R[1], R2 = B.R[2];
   int lo0 = R0 < 0 ? 0 : -R0, hi0 = R0 < 0 ? n0 - 1 : R0;
   int lo1 = R1 < 0 ? 0 : -R1, hi1 = R1 < 0 ? n1 - 1 : R1;
-  for (int d0 = lo0; d0 <= hi0; ++d0) {
-    int c0 = R0 < 0 ? d0 : ((ci0 + d0) % n0 + n0) % n0;
-    for (int d1 = lo1; d1 <= hi1; ++d1) {
-      int c1 = R1 < 0 ? d1 : ((ci1 + d1) % n1 + n1) % n1;
-      int rowc = S.cell0 + (c0 * n1 + c1) * n2;
-      int segs[2][2];
-      int nseg = 0;
-      if (R2 < 0) {
-        segs[0][0] = 0; segs[0][1] = n2 - 1; nseg = 1;
-      } else {
-        int lo = ci2 - R2, hi = ci2 + R2;
-        if (lo < 0) { segs[0][0] = lo + n2; segs[0][1] = n2 - 1; segs[1][0] = 0; segs[1][1] = hi; nseg = 2; }
-        else if (hi >= n2) { segs[0][0] = lo; segs[0][1] = n2 - 1; segs[1][0] = 0; segs[1][1] = hi - n2; nseg = 2; }
-        else { segs[0][0] = lo; segs[0][1] = hi; nseg = 1; }
-      }
-      for (int g = 0; g < nseg; ++g) {
-        int a0 = a.cell_start[rowc + segs[g][0]], a1 = a.cell_start[rowc + segs[g][1] + 1];
-        for (int t0 = a0; t0 < a1; t0 += 32) {
-          int t = t0 + lane;
-          bool keep = false;
-          if (t < a1) {
-            double4 pj = a.spos[t];
-            if ((int)pj.w != mi) {
-              double x = pi.x - pj.x, y = pi.y - pj.y, z = pi.z - pj.z;
-              min_image_fast(x, y, z, H, id);
-              keep = x * x + y * y + z * z < rl2;
-            }
-          }
-          unsigned bal = __ballot_sync(0xffffffffu, keep);
-          if (keep) {
-            int slot = count + __popc(bal & ((1u << lane) - 1u));
-            if (slot < a.cc) out[slot] = a.cell_atoms[t];
-          }
-          count += __popc(bal);
+  const int nd1 = hi1 - lo1 + 1, ncol = (hi0 - lo0 + 1) * nd1;
+  // rectangular boxes: a column is as far as the nearest edge of its nearest image, and its range is what that
+  // leaves of the radius (a quarter of the cube of cells that the index ranges span); cw: cell widths, fc: the
+  // atom in its cell; reach: the radius with room for the rounding of these
+  const bool rect = B.H[3] == 0.0 && B.H[6] == 0.0 && B.H[7] == 0.0;
+  const T reach2 = T((rl + 1e-4) * (rl + 1e-4));
+  auto in_cell = [](T u, int n, int ci) {
+    const T f = (u - floor(u)) * T(n) - T(ci);
+    return f < T(-0.5) ? f + T(n) : f > T(1.5) ? f - T(n) : f;
+  };
+  const T cw0 = T(B.H[0] / n0), cw1 = T(B.H[4] / n1), cw2 = T(B.H[8] / n2);
+  const T fc0 = in_cell(pi.x * id[0], n0, ci0), fc1 = in_cell(pi.y * id[1], n1, ci1), fc2 = in_cell(pi.z * id[2], n2, ci2);
+  auto gap = [](int d, int n, T f) {  // cells between the atom and a column d cells away, of its images the nearest
+    d = d > n / 2 ? d - n : d < -(n / 2) ? d + n : d;
+    const T up = d > 0 ? T(d) - f : T(d + n) - f, down = d < 0 ? f - T(d + 1) : f - T(d - n + 1);
+    return d == 0 ? T(0) : min(up, down);
+  };
+  for (int cb = 0; cb < ncol; cb += 32) {
+    // this lane's column: its one or two ranges along the third axis, in cell order
+    int b0 = 0, l0 = 0, b1 = 0, l1 = 0;
+    const int c = cb + lane;
+    if (c < ncol) {
+      const int d0 = lo0 + c / nd1, d1 = lo1 + c % nd1;
+      const int c0 = R0 < 0 ? d0 : ((ci0 + d0) % n0 + n0) % n0, c1 = R1 < 0 ? d1 : ((ci1 + d1) % n1 + n1) % n1;
+      const int *st = a.cell_start + S.cell0 + (c0 * n1 + c1) * n2;
+      int lo = R2 < 0 ? 0 : ci2 - R2, hi = R2 < 0 ? n2 - 1 : ci2 + R2;
+      bool reach = true;
+      if (rect) {
+        const T g0 = gap(c0 - ci0, n0, fc0) * cw0, g1 = gap(c1 - ci1, n1, fc1) * cw1;
+        const T left = reach2 - g0 * g0 - g1 * g1;
+        reach = left >= T(0);
+        if (reach) {
+          const T dz = sqrt(left) / cw2;
+          const int zl = ci2 + (int)floor(fc2 - dz), zh = ci2 + (int)floor(fc2 + dz);
+          if (zh - zl + 1 >= n2) { lo = 0; hi = n2 - 1; }
+          else { lo = zl; hi = zh; }
         }
+      }
+      if (reach) {
+        if (hi < 0) { lo += n2; hi += n2; }
+        if (lo >= n2) { lo -= n2; hi -= n2; }
+        if (lo < 0) {
+          b1 = st[0]; l1 = st[hi + 1] - b1;
+          lo += n2; hi = n2 - 1;
+        } else if (hi >= n2) {
+          b1 = st[0]; l1 = st[hi - n2 + 1] - b1;
+          hi = n2 - 1;
+        }
+        b0 = st[lo]; l0 = st[hi + 1] - b0;
+      }
+    }
+    for (unsigned todo = __ballot_sync(0xffffffffu, l0 + l1 > 0); todo; todo &= todo - 1) {
+      const int k = __ffs(todo) - 1;
+      const int f0 = __shfl_sync(0xffffffffu, b0, k), m0 = __shfl_sync(0xffffffffu, l0, k);
+      const int f1 = __shfl_sync(0xffffffffu, b1, k), tot = m0 + __shfl_sync(0xffffffffu, l1, k);
+      for (int t0 = 0; t0 < tot; t0 += 32) {
+        const int u = t0 + lane, t = u < m0 ? f0 + u : f1 + u - m0;
+        bool keep = false;
+        if (u < tot) {
+          const v4<T> pj = a.spos[t];
+          if (pj.w != pi.w) {
+            T x = pi.x - pj.x, y = pi.y - pj.y, z = pi.z - pj.z;
+            min_image_scan(x, y, z, H, id);
+            keep = x * x + y * y + z * z < rl2;
+          }
+        }
+        unsigned bal = __ballot_sync(0xffffffffu, keep);
+        if (keep) {
+          int slot = count + __popc(bal & ((1u << lane) - 1u));
+          if (slot < a.cc) out[slot] = a.cell_atoms[t];
+        }
+        count += __popc(bal);
       }
     }
   }
   if (lane == 0) {
     a.ncand[i] = count;
-    a.pos_ref[i] = pi;
+    a.pos_ref[i] = a.pos4[i];
     if (count > a.cc) atomicOr(&a.status[s], 0x10u);
   }
 }
@@ -441,22 +499,6 @@ __device__ __forceinline__ T group_sum(T v, unsigned m) {
     for (int o = LPA / 2; o > 0; o >>= 1) v += __shfl_xor_sync(m, v, o);
     return v;
   }
-}
-
-// FP32 sequential minimum image (the mixed-precision row build's candidate loop).  Rounding to the
-// nearest integer by adding and subtracting 1.5 2^23 (wrapped positions: |argument| < 2): two
-// additions, where rintf is a conversion at a quarter of their rate.
-__device__ __forceinline__ float nearest_f(float x) { return __fadd_rn(__fadd_rn(x, 12582912.f), -12582912.f); }
-__device__ __forceinline__ void min_image_scan(double &x, double &y, double &z, const double *H, const double *id) {
-  min_image_fast(x, y, z, H, id);
-}
-__device__ __forceinline__ void min_image_scan(float &x, float &y, float &z, const float *H, const float *id) {
-  float n = nearest_f(z * id[2]);
-  x -= n * H[6]; y -= n * H[7]; z -= n * H[8];
-  n = nearest_f(y * id[1]);
-  x -= n * H[3]; y -= n * H[4];
-  n = nearest_f(x * id[0]);
-  x -= n * H[0];
 }
 
 // The row scan of atom i by its warp: the molecule partners (special = true), then the

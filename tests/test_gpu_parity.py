@@ -425,6 +425,34 @@ def test_field_on_the_workload_meshes(grid, prec):
     assert np.abs(got - ref).max() <= tol * np.abs(ref).max(), np.abs(got - ref).max() / np.abs(ref).max()
 
 
+@pytest.mark.parametrize("edges", [(1.25, 1.25, 1.25), (1.4, 2.1, 3.3), (2.9, 2.5, 1.9), (4.4, 1.3, 2.2)])
+@pytest.mark.parametrize("prec", ["double", "mixed"])
+def test_candidate_list_of_rectangular_boxes_is_complete(edges, prec):
+    """The engine's candidate list against rows of every pair within the cutoff given by the caller, on rectangular
+    boxes with few and many cells per axis, a third of the atoms on cell faces, positions outside the box: the
+    same pairs (exact counts), the same forces."""
+    from pgm_jax_b200.forcefield import MDSettings, PGMForceField
+    from pgm_jax_b200.systems import Molecule, System
+
+    rng = np.random.default_rng(23)
+    n, cutoff, L = 420, 0.6, np.array(edges)
+    pos = rng.uniform(0, 1, size=(n, 3)) * L
+    cells = np.floor(L / (0.5 * cutoff))
+    pos[: n // 3] = np.round(pos[: n // 3] / L * cells) / cells * L
+    pos += rng.normal(scale=1e-9, size=pos.shape)
+    s = System([Molecule("X", ["O"], [q], [0.05], [1e-3]) for q in rng.normal(size=n)])
+    ff = PGMForceField(s, np.diag(L), MDSettings(precision=prec, elec="q", cutoff=cutoff, ewald_beta=6.0, pme_grid=(24, 24, 24)),
+                       row_capacity=416)
+    ff.set_list_capacity(512)
+    given = ff.compute(pos, np.diag(L), ff.rows_for(pos, np.diag(L)))
+    pairs = int(ff._lib.pgm_row_pairs(ff._h))
+    for shift in (0, 1):  # the second call rebuilds the list at positions a lattice vector away
+        own = ff.compute(pos + shift * L, np.diag(L))
+        assert int(ff._lib.pgm_row_pairs(ff._h)) == pairs
+        assert not bool(own.overflow.any())
+        assert rms_rel(own.forces.cpu().numpy(), given.forces.cpu().numpy()) <= (1e-10 if prec == "double" else 1e-5)
+
+
 @pytest.mark.parametrize("prec,beta", [("double", b) for b in (1.0, 4.0, 8.0, 14.0)] + [("mixed", b) for b in (1.0, 4.0, 8.0)])
 def test_pair_kernels_over_their_ranges(prec, beta):
     """The field of charges and dipoles of single atoms at all distances from 0.02 nm (both arguments of the
