@@ -230,7 +230,8 @@ struct Engine : EngineBase {
   // lanes per atom of the learned guess's channel pass (32: a warp per atom; 16, 8: two, four atoms per warp)
   static constexpr int CHAN_LPA = 32;
   float nn_sigma = 2e-4f, nn_rg = 0.5f;  // until pgm_set_nn_model
-  int *h_any = nullptr;
+  int *h_any = nullptr;  // pinned: the solve's flag after the last two iterations
+  cudaEvent_t ev_any[2] = {nullptr, nullptr};
   const double *last_pos = nullptr;
   cudaStream_t side = nullptr, aux = nullptr, aux_b = nullptr, nn_st = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_fork_b = nullptr, ev_join_b = nullptr, ev_nn_fork = nullptr,
@@ -244,6 +245,8 @@ struct Engine : EngineBase {
 
   ~Engine() {
     if (h_any) cudaFreeHost(h_any);
+    for (auto &e : ev_any)
+      if (e) cudaEventDestroy(e);
     if (side) cudaStreamDestroy(side);
     if (aux) cudaStreamDestroy(aux);
     if (aux_b) cudaStreamDestroy(aux_b);
@@ -608,7 +611,8 @@ struct Engine : EngineBase {
       CK(cudaMemset(sh_n.p, 0, sizeof(int) * nt));
     }
     CK(cudaMemset(nn_valid.p, 0, sizeof(int)));
-    CK(cudaMallocHost(&h_any, sizeof(int)));
+    CK(cudaMallocHost(&h_any, 2 * sizeof(int)));
+    for (auto &e : ev_any) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     CK(cudaStreamCreateWithFlags(&aux, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&aux_b, cudaStreamNonBlocking));
     CK(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
@@ -1182,10 +1186,24 @@ struct Engine : EngineBase {
   // must not set it for the predicted starts that follow (3 to 8).
   int unroll_count() const { return std::max(0, std::min({last_iters - 2, 3, set.max_iter})); }
 
-  bool any_active(cudaStream_t st) {
-    CK(cudaMemcpyAsync(h_any, dany.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    return *h_any != 0;
+  // The CG loop driven from the host: iteration k + 1 is enqueued before the flag that iteration k left is
+  // read, so that the GPU does not idle for the round trip (12 us a turn); the one enqueued after the last
+  // finds every system converged and returns at once.  Returns the iterations until convergence.
+  int host_loop(cudaStream_t st, pgm::Dev<T> &a) {
+    auto post = [&](int k) {  // the flag after k iterations
+      CK(cudaMemcpyAsync(h_any + (k & 1), dany.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+      CK(cudaEventRecord(ev_any[k & 1], st));
+    };
+    post(0);
+    for (int k = 0; k < set.max_iter; ++k) {
+      const long long l0 = launches;
+      iteration(st, a, 0, 0);
+      per_iter = launches - l0;
+      post(k + 1);
+      CK(cudaEventSynchronize(ev_any[k & 1]));
+      if (!h_any[k & 1]) return k;
+    }
+    return set.max_iter;
   }
 
   // The induced-dipole solve (forcefield.py:1917-2008 and 1714-1821).  mode 0: predictor start
@@ -1293,14 +1311,7 @@ struct Engine : EngineBase {
         per_iter = launches - l0;
       });
     } else {
-      int it = 0;
-      for (; it < set.max_iter; ++it) {
-        if (!any_active(st)) break;
-        long long l0 = launches;
-        iteration(st, a, 0, 0);
-        per_iter = launches - l0;
-      }
-      last_iters = it;
+      last_iters = host_loop(st, a);
     }
     const int push = mode == 0 ? 1 : 0;
     launch_pdl(pgm::k_cg_finish<T>, grid1(nt), 256, 0, st, a, mu_out, push ? ind->hist : nullptr, push,
@@ -1375,14 +1386,7 @@ struct Engine : EngineBase {
         per_iter = launches - l0;
       });
     } else {
-      int it = 0;
-      for (; it < set.max_iter; ++it) {
-        if (!any_active(st)) break;
-        long long l0 = launches;
-        iteration(st, a, 0, 0);
-        per_iter = launches - l0;
-      }
-      last_iters = it;
+      last_iters = host_loop(st, a);
     }
     launch_pdl(pgm::k_iel_finish<T>, grid1(nt), 256, 0, st, a, mu_out, ind->hist, ind->xl, iel_co);
     launch_pdl(pgm::k_cg_state_out, grid1(nsys, 64), 64, 0, st, (const pgm::CGSys *)d_cg.p, nsys,
