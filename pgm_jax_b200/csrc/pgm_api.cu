@@ -244,9 +244,12 @@ struct Engine : EngineBase {
   long long per_iter = 0;
 
   ~Engine() {
-    if (h_any) cudaFreeHost(h_any);
     for (auto &e : ev_any)
-      if (e) cudaEventDestroy(e);
+      if (e) {
+        cudaEventSynchronize(e);  // the copy of the flag that ran ahead has landed
+        cudaEventDestroy(e);
+      }
+    if (h_any) cudaFreeHost(h_any);
     if (side) cudaStreamDestroy(side);
     if (aux) cudaStreamDestroy(aux);
     if (aux_b) cudaStreamDestroy(aux_b);

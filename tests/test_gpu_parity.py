@@ -428,9 +428,10 @@ def test_field_on_the_workload_meshes(grid, prec):
 @pytest.mark.parametrize("edges", [(1.25, 1.25, 1.25), (1.4, 2.1, 3.3), (2.9, 2.5, 1.9), (4.4, 1.3, 2.2)])
 @pytest.mark.parametrize("prec", ["double", "mixed"])
 def test_candidate_list_of_rectangular_boxes_is_complete(edges, prec):
-    """The engine's candidate list against rows of every pair within the cutoff given by the caller, on rectangular
-    boxes with few and many cells per axis, a third of the atoms on cell faces, positions outside the box: the
-    same pairs (exact counts), the same forces."""
+    """The engine's candidate list against candidate rows of all other atoms given by the caller (the cutoff is tested in
+    the engine either way: a third of the atoms sit on cell faces, many pairs at the cutoff to rounding), on
+    rectangular boxes with few and many cells per axis, positions outside the box: the same pairs (exact
+    counts), the same forces."""
     from pgm_jax_b200.forcefield import MDSettings, PGMForceField
     from pgm_jax_b200.systems import Molecule, System
 
@@ -444,7 +445,8 @@ def test_candidate_list_of_rectangular_boxes_is_complete(edges, prec):
     ff = PGMForceField(s, np.diag(L), MDSettings(precision=prec, elec="q", cutoff=cutoff, ewald_beta=6.0, pme_grid=(24, 24, 24)),
                        row_capacity=416)
     ff.set_list_capacity(512)
-    given = ff.compute(pos, np.diag(L), ff.rows_for(pos, np.diag(L)))
+    others = (np.arange(n)[:, None] + np.arange(1, n)) % n
+    given = ff.compute(pos, np.diag(L), others.astype(np.int32))
     pairs = int(ff._lib.pgm_row_pairs(ff._h))
     for shift in (0, 1):  # the second call rebuilds the list at positions a lattice vector away
         own = ff.compute(pos + shift * L, np.diag(L))
