@@ -1043,7 +1043,8 @@ struct Engine : EngineBase {
     }
     launch_pdl(pgm::k_rows<T>, nwblk, 256, 0, st, a);
     if (nn_hist) nn_fork(st, a, nn_hist);
-    launch_pdl(pgm::k_influence<T>, (int)std::min<long long>(8 * nsm, (cgrid + 255) / 256), 256, 0, st, a, (long long)cgrid);
+    launch_pdl(pgm::k_influence<T>, (int)std::min<long long>(8 * nsm, std::max<long long>((cgrid + 255) / 256, grid1(2 * nt))), 256, 0, st, a,
+               (long long)cgrid);
   }
 
   void set_list_capacity(int c) override {
