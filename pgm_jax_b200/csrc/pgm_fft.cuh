@@ -12,6 +12,8 @@
 // What bounds a pass: the meshes sit in L2 and a pass reads and writes them once, so it is latency:
 // loads in flight per SM, and the barriers between phases.  A staged shared-memory Stockham plan
 // (radix 8, 4, 2, 3, 5; one barrier and one shared round trip per radix) had 4 to 6 barriers a line.
+// Chains of a convolution, FP32, that plan -> this: 192^3 122 -> 73 us, 96^3 20.3 -> 15.6; a length that the plan
+// had at run time only, 108^3: 68 -> 20.
 #pragma once
 #include "pgm_device.cuh"
 

@@ -202,7 +202,9 @@ __device__ __forceinline__ void box_setup(Dev<T> &a, int s, const double *H, Box
 // (pme.py:269-304), permanent dipoles (forcefield.py:1032-1042), the list's displacement test, and, on the
 // thread of a molecule's first atom, the offsets of its atoms from its centre of mass (the molecule made
 // whole from its first atom), for the molecular virial.  A non-finite position is marked in base.w (the
-// status word is being started by another block) and reported by the force pass.
+// status word is being started by another block) and reported by the force pass.  Small kernels are bound by
+// their launch: this and the merges of the start, finish and energy kernels took an MD step of 512 waters from 256 to
+// 249 us, 24 boxes of 216 to 1,000 waters 2 % down.
 template <typename T>
 __global__ void k_prep(Dev<T> a, const double *boxes) {
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
@@ -365,7 +367,9 @@ __device__ __forceinline__ void min_image_scan(float &x, float &y, float &z, con
 // the positions of the build are kept for the displacement test (the reference's neighbour list,
 // md/neighbors.py:169-304, rebuilt when an atom moved more than skin / 2).  The lanes look up the
 // ranges of 32 cell columns at once (a column's range is a load that its atoms' loads wait for); mixed
-// precision tests FP32 displacements against a radius 1e-5 wider (they are good to 1e-6 nm).
+// precision tests FP32 displacements against a radius 1e-5 wider (they are good to 1e-6 nm).  A rectangular
+// box trims the columns and their ranges to the sphere.  Latency of dependent loads bounds it: a rebuild took 1724 us
+// at 98,304 atoms and 239 at 12,288 with a column at a time in FP64 over the cube of cells, 525 and 77 so.
 template <typename T>
 __global__ void __launch_bounds__(256) k_cand(Dev<T> a) {
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
@@ -482,6 +486,9 @@ __global__ void __launch_bounds__(256) k_cand(Dev<T> a) {
 // the warp in shared memory; whenever 32 are waiting the warp evaluates their radial kernels
 // (pair_kernels), every lane busy, and writes k, x, y, z, G0..G3 with them, contiguous over the lanes,
 // and the local preconditioner's short entries and the learned guess's graph edges.
+// Bound by the latency of the candidates' gathers and by issue: the scan alone takes 137 of 232 us at 59,049
+// atoms (FP32; 305 with rows in eight arrays and a round that waited for its loads; 378 of 494 at 98,304, 57 of
+// 78 at 12,288; FP64 127 of 147).  3 or 5 blocks per SM are slower (309, 296 against 272 at the time).
 
 // An atom's group of LPA lanes (32: the warp; 16, 8: a half, a quarter warp): its shuffle mask, and the sum over
 // it (the warp's own reduction for a whole warp).
@@ -764,7 +771,8 @@ __global__ void k_influence(Dev<T> a, long long total) {
 // two points), one lane each: the vectors of a row sit side by side, so a warp's request touches 16 rows in whole
 // sectors, and a lane's k3 weights stay in registers for all rows.  What bounds them is latency and the L1's line
 // rate: with one point or vector per lane and the k3 weights read from shared memory for every
-// point, a row cost three times the instructions.
+// point, a row cost three times the instructions.  At 98,304 atoms, 192^3: gather 59.5 -> 37.0 us, spread
+// 43.2 -> 38.9; at 59,049 atoms 31.0 -> 22.6 and 25.5 -> 24.7 (the spread keeps its vector atomics, which L2 bounds).
 constexpr int QL = 8, ATOMS_PER_BLOCK = 32;
 template <typename T, int VW> struct VecOf;
 template <> struct VecOf<float, 4> { using type = float4; };
@@ -916,7 +924,9 @@ __global__ void __launch_bounds__(ATOMS_PER_BLOCK * QL) k_spread(Dev<T> a, const
 // (32: a warp per atom; 16 or 8: two or four atoms per warp, each row split over fewer lanes, more
 // rows in flight per warp), 8 atoms per block of 8 LPR threads either way -- the autotuner's choice
 // (Engine::autotune).  The lane partial sums are combined by a butterfly within each LPR group,
-// so the variants differ only in the order of the row's additions.
+// so the variants differ only in the order of the row's additions.  Bound by HBM: 24 bytes a pair, 111.8 us
+// at 30.2 M pairs = 0.99 of the measured copy bandwidth (116.8 with the arrays apart); cached instead of evict-first
+// loads lose 4 to 10 % of a step (they push the grids out of L2).
 template <typename T, bool WITH_Q, int ACT, int LPR = 32>
 __global__ void __launch_bounds__(8 * LPR) k_rowfield(Dev<T> a, const v4<T> *__restrict__ D, v4<T> *__restrict__ F, int nvb) {
   static_assert(LPR == 32 || LPR == 16 || LPR == 8, "lanes per row");
@@ -2167,6 +2177,8 @@ __global__ void k_iel_finish(Dev<T> a, double *mu, double *hist, double *xl, Iel
 // atoms with the block preconditioner, the i-side delta scaled by a.iel_keep = 1 - 1/omega); their
 // position gradients at fixed delta go to the forces, not to the virial (the fixed-mu strain
 // derivative); the sums of |delta|^2 and |delta|^2 / (2 alpha) go to the energy accumulators.
+// Bound by the row stream (40 bytes a pair) and the partners' gathers.  The stencil comes first and its sums wait in
+// shared memory, so that registers serve one part at a time: 303 -> 238 us at 98,304 atoms, 197 -> 157 at 59,049.
 template <typename T, int P, int MINB = 3, bool SHADOW = false>
 __global__ void __launch_bounds__(ATOMS_PER_BLOCK * QL, MINB) k_forces(Dev<T> a, const double *mu) {
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
