@@ -240,6 +240,28 @@ __device__ __forceinline__ void pair_kernels(T w2, T beta, T r2, T G[4]) {  // w
   for (int n = 0; n < 4; ++n) G[n] -= U[n];
 }
 
+// The cells lo .. hi of a periodic axis of n cells that come within z cell widths of an atom at fraction f of its
+// cell ci (about [0, 1]): -n < lo <= hi < 2 n, fewer than n.  All n cells wherever that does not follow from the
+// numbers -- a non-finite position or box, a cell without width --, so that no index leaves the axis.
+template <typename T>
+__host__ __device__ __forceinline__ void cells_within(T f, T z, int ci, int n, int &lo, int &hi) {
+  const T a = floor(f - z), b = floor(f + z);
+  const bool part = a <= b && b - a + T(1) < T(n) && a > T(-n) && b < T(n);  // false for NaN
+  lo = part ? ci + (int)a : 0;
+  hi = part ? ci + (int)b : n - 1;
+}
+// Cells lo .. hi (-n < lo <= hi < 2 n, at most n of them) of a periodic axis in cell order: lo .. hi and 0 .. hi2 (-1: none).
+struct CellRange {
+  int lo, hi, hi2;
+};
+__host__ __device__ __forceinline__ CellRange wrapped_cells(int lo, int hi, int n) {
+  if (hi < 0) { lo += n; hi += n; }
+  if (lo >= n) { lo -= n; hi -= n; }
+  if (lo < 0) return CellRange{lo + n, n - 1, hi};
+  if (hi >= n) return CellRange{lo, n - 1, hi - n};
+  return CellRange{lo, hi, -1};
+}
+
 // Cardinal B-spline weights of order P at offset f, with first and second derivatives: the
 // recursion of pgm_jax/md/pme.py:81-103 (theta[k] = M_P(f + P - 1 - k)).
 template <typename T, int P, bool SECOND>

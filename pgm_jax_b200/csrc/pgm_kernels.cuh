@@ -428,24 +428,12 @@ __global__ void __launch_bounds__(256) k_cand(Dev<T> a) {
         const T g0 = gap(c0 - ci0, n0, fc0) * cw0, g1 = gap(c1 - ci1, n1, fc1) * cw1;
         const T left = reach2 - g0 * g0 - g1 * g1;
         reach = left >= T(0);
-        if (reach) {
-          const T dz = sqrt(left) / cw2;
-          const int zl = ci2 + (int)floor(fc2 - dz), zh = ci2 + (int)floor(fc2 + dz);
-          if (zh - zl + 1 >= n2) { lo = 0; hi = n2 - 1; }
-          else { lo = zl; hi = zh; }
-        }
+        if (reach) cells_within(fc2, T(sqrt(left) / cw2), ci2, n2, lo, hi);
       }
       if (reach) {
-        if (hi < 0) { lo += n2; hi += n2; }
-        if (lo >= n2) { lo -= n2; hi -= n2; }
-        if (lo < 0) {
-          b1 = st[0]; l1 = st[hi + 1] - b1;
-          lo += n2; hi = n2 - 1;
-        } else if (hi >= n2) {
-          b1 = st[0]; l1 = st[hi - n2 + 1] - b1;
-          hi = n2 - 1;
-        }
-        b0 = st[lo]; l0 = st[hi + 1] - b0;
+        const CellRange z = wrapped_cells(lo, hi, n2);
+        if (z.hi2 >= 0) { b1 = st[0]; l1 = st[z.hi2 + 1] - b1; }
+        b0 = st[z.lo]; l0 = st[z.hi + 1] - b0;
       }
     }
     for (unsigned todo = __ballot_sync(0xffffffffu, l0 + l1 > 0); todo; todo &= todo - 1) {

@@ -455,6 +455,28 @@ def test_candidate_list_of_rectangular_boxes_is_complete(edges, prec):
         assert rms_rel(own.forces.cpu().numpy(), given.forces.cpu().numpy()) <= (1e-10 if prec == "double" else 1e-5)
 
 
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("skew", [0.0, 0.3])
+@pytest.mark.parametrize("prec", ["double", "mixed"])
+def test_non_finite_position_is_a_status_not_a_fault(prec, skew, value):
+    """A coordinate that is not a number ends the call with the status bit, in rectangular and triclinic boxes with
+    several cells per axis; the next call with finite positions gives what a new handle gives."""
+    from pgm_jax_b200 import _lib
+    from pgm_jax_b200.systems import water_box
+
+    s, pos, H = water_box(6, 1.8624, seed=2)
+    H = H + np.array([[0, 0, 0], [skew, 0, 0], [0, skew, 0]])
+    kw = dict(cutoff=0.5, pme_grid=(24, 24, 24), dipole_tol=1e-8 if prec == "double" else 1e-6)
+    ff = ff_for(s, H, prec, **kw)
+    for atom, axis in ((0, 2), (s.n - 1, 0), (s.n // 2, 1)):
+        x = pos.copy()
+        x[atom, axis] = value
+        assert int(ff.compute(x, H).status[0]) & _lib.STATUS_NONFINITE
+    got, ref = ff.compute(pos, H), ff_for(s, H, prec, **kw).compute(pos, H)
+    assert not int(got.status[0]) & _lib.STATUS_NONFINITE
+    assert rms_rel(got.forces.cpu().numpy(), ref.forces.cpu().numpy()) <= (1e-10 if prec == "double" else 2e-6)
+
+
 @pytest.mark.parametrize("prec,beta", [("double", b) for b in (1.0, 4.0, 8.0, 14.0)] + [("mixed", b) for b in (1.0, 4.0, 8.0)])
 def test_pair_kernels_over_their_ranges(prec, beta):
     """The field of charges and dipoles of single atoms at all distances from 0.02 nm (both arguments of the
