@@ -180,9 +180,9 @@ __device__ __forceinline__ void box_setup(Dev<T> &a, int s, const double *H, Box
     // plane height h_a = 1 / |column a of H^-1|
     double c0 = Hi[0 * 3 + ax], c1 = Hi[1 * 3 + ax], c2v = Hi[2 * 3 + ax];
     B.h[ax] = 1.0 / sqrt(c0 * c0 + c1 * c1 + c2v * c2v);
-    int nc = S.nc[ax];
-    int R = (int)ceil((a.cutoff + a.skin) * nc / B.h[ax] - 1e-12);
-    B.R[ax] = (2 * R + 1 >= nc) ? -1 : R;
+    const int nc = S.nc[ax];
+    const double R = ceil((a.cutoff + a.skin) * nc / B.h[ax] - 1e-12);
+    B.R[ax] = R >= 0.0 && 2.0 * R + 1.0 < nc ? (int)R : -1;  // -1: all cells (a degenerate box: R infinite or NaN)
   }
   int changed = 0;
   for (int k = 0; k < 9; ++k) changed |= (a.box[s].H[k] != H[k]);

@@ -477,6 +477,26 @@ def test_non_finite_position_is_a_status_not_a_fault(prec, skew, value):
     assert rms_rel(got.forces.cpu().numpy(), ref.forces.cpu().numpy()) <= (1e-10 if prec == "double" else 2e-6)
 
 
+@pytest.mark.parametrize("prec", ["double", "mixed"])
+def test_degenerate_box_is_a_status_not_a_fault(prec):
+    """Boxes without volume, with a negative edge or with entries that are not finite end the call with a
+    status bit (box or non-finite energy); the next call with a good box gives what a new handle gives."""
+    from pgm_jax_b200 import _lib
+    from pgm_jax_b200.systems import water_box
+
+    s, pos, H = water_box(6, 1.8624, seed=2)
+    kw = dict(cutoff=0.5, pme_grid=(24, 24, 24), dipole_tol=1e-8 if prec == "double" else 1e-6, max_iter=40)
+    ff = ff_for(s, H, prec, **kw)
+    bad = [np.zeros((3, 3)), -H, np.diag([1.8624, 1.8624, 0.0]), np.diag([1.8624, -1.8624, 1.8624]), np.full((3, 3), np.nan)]
+    bad += [np.diag([1.8624, 1.8624, v]) for v in (np.nan, np.inf)]
+    bad.append(H + np.array([[0, 0, 0], [0.3, 0, 0], [0, np.nan, 0]]))
+    for box in bad:
+        assert int(ff.compute(pos, box).status[0]) & (_lib.STATUS_BAD_BOX | _lib.STATUS_NONFINITE), box
+    got, ref = ff.compute(pos, H), ff_for(s, H, prec, **kw).compute(pos, H)
+    assert not int(got.status[0]) & (_lib.STATUS_BAD_BOX | _lib.STATUS_NONFINITE)
+    assert rms_rel(got.forces.cpu().numpy(), ref.forces.cpu().numpy()) <= (1e-10 if prec == "double" else 2e-6)
+
+
 @pytest.mark.parametrize("prec,beta", [("double", b) for b in (1.0, 4.0, 8.0, 14.0)] + [("mixed", b) for b in (1.0, 4.0, 8.0)])
 def test_pair_kernels_over_their_ranges(prec, beta):
     """The field of charges and dipoles of single atoms at all distances from 0.02 nm (both arguments of the
