@@ -1385,7 +1385,7 @@ __device__ __forceinline__ void cg_begin(const BeginArgs &b, int which) {
     CGSys &G = b.cg[s];
     const bool mine = which == 2 || (which == 0 && G.fused) || (which == 1 && !G.fused) || (which == 3 && G.fallback);
     if (mine) {
-      if (!G.fused) G.norm = G.acc_abs / G.n3 + 1e-300;
+      if (!G.fused && which != 3) G.norm = G.acc_abs / G.n3 + 1e-300;  // a fallback keeps the norm of its solve's b
       G.rz = G.acc_rz;
       G.err = __longlong_as_double((long long)G.acc_max) / G.norm;
       G.beta = 0.0;

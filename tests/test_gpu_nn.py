@@ -98,13 +98,13 @@ def _same_positions(md, steps, ffs, captured=False):
     return {k: np.array(v) for k, v in its.items()}
 
 
-def _learned_md(prec="mixed", tol=1e-6):
+def _learned_md(prec="mixed", tol=1e-6, **more):
     from pgm_jax_b200.forcefield import MDSettings, PGMForceField
     from pgm_jax_b200.md import RigidMD
     from pgm_jax_b200.systems import water_box
 
     s, pos, H = water_box(5, 1.55, seed=6)
-    kw = dict(precision=prec, cutoff=0.7, ewald_beta=5.0, pme_grid=(32, 32, 32), dipole_tol=tol, max_iter=100)
+    kw = dict(precision=prec, cutoff=0.7, ewald_beta=5.0, pme_grid=(32, 32, 32), dipole_tol=tol, max_iter=100, **more)
     ff = PGMForceField(s, H, MDSettings(predictor="nn", **kw))
     md = RigidMD(ff, pos, H, temperature=300.0, dt_fs=1.0, gamma_ps=5.0, seed=2)
     others = {p: PGMForceField(s, H, MDSettings(predictor=p, **kw)) for p in ("mu4", "mu1")}
@@ -162,3 +162,34 @@ def test_bad_model_falls_back_to_mu4(prec):
     ff.set_nn_fallback(0.0)  # without the check the bad guess costs iterations
     its_off = _same_positions(md, 4, {"mu4": others["mu4"]}, captured=True)
     assert its_off["md"].mean() > its_off["mu4"].mean() + 1, its_off
+
+
+@pytest.mark.parametrize("more", [{"fused": False}, {"fused": False, "local_niter": 1}, {"norm_refresh": 2},
+                                  {"norm_refresh": 2, "local_niter": 1}])
+@pytest.mark.parametrize("captured", [False, True])
+def test_fallback_of_a_plain_start_keeps_the_norm(more, captured):
+    """A bad model on starts that evaluate b and its norm (every step without the fused start, every second one with
+    norm_refresh 2): the fallback's residual is measured against that norm, so the solve meets the tolerance
+    in at most one iteration more than mu4's, and the stored norm is that of mu4's solve at the same positions."""
+    from pgm_jax_b200.learned import N_HID, N_OUT, GuessModel, init_weights
+
+    s, H, ff, md, others = _learned_md("double", 1e-7, **more)
+    for _ in range(12):
+        md.step()
+    md.stream.synchronize()
+    w = init_weights(0)
+    w[-(N_HID * N_OUT + N_OUT):] = np.random.default_rng(9).normal(scale=0.5, size=N_HID * N_OUT + N_OUT)  # output layer
+    GuessModel(w).install(ff)
+    for k in range(4):
+        mu4 = others["mu4"]
+        state = md.ind.clone()
+        if captured and k == 0:
+            md.capture()
+        md.run(1) if captured else md.step()
+        md.stream.synchronize()
+        r = mu4.compute(md.pos.clone(), H, None, state)
+        assert int(ff.nn_fallback_stats()["fallbacks"][0]) == k + 1
+        assert not int(md.result.status[0]) & 0x2 and float(md.result.residual[0]) <= ff.s.dipole_tol
+        assert int(md.result.iterations[0]) <= int(r.iterations[0]) + 1
+        # the two solves' b differ by nothing but rounding (FP64 sums of 375 atoms)
+        assert abs(float(md.ind.norm[0]) - float(r.induction.norm[0])) <= 1e-12 * float(r.induction.norm[0])
