@@ -367,7 +367,7 @@ __device__ __forceinline__ void min_image_scan(float &x, float &y, float &z, con
 // the positions of the build are kept for the displacement test (the reference's neighbour list,
 // md/neighbors.py:169-304, rebuilt when an atom moved more than skin / 2).  The lanes look up the
 // ranges of 32 cell columns at once (a column's range is a load that its atoms' loads wait for); mixed
-// precision tests FP32 displacements against a radius 1e-5 wider (they are good to 1e-6 nm).  A rectangular
+// precision tests FP32 displacements against a radius wider by their error, which grows with the box.  A rectangular
 // box trims the columns and their ranges to the sphere.  Latency of dependent loads bounds it: a rebuild took 1724 us
 // at 98,304 atoms and 239 at 12,288 with a column at a time in FP64 over the cube of cells, 525 and 77 so.
 template <typename T>
@@ -387,7 +387,11 @@ __global__ void __launch_bounds__(256) k_cand(Dev<T> a) {
   v4<T> pi;
   if constexpr (sizeof(T) == 4) pi = a.pos4f[i];
   else pi = a.pos4[i];
-  const double rl = (a.cutoff + a.skin) * (sizeof(T) == 4 ? 1.00001 : 1.0);
+  // W: the largest coordinate of a wrapped position.  A displacement of two of them in FP32 is off by less than
+  // 12 W 2^-24 a component (both positions, three lattice vectors and the subtractions), 1.3e-6 W in length; the
+  // square's rounding is below 1e-6 of it.
+  const double W = fmax(fabs(B.H[0]) + fabs(B.H[3]) + fabs(B.H[6]), fmax(fabs(B.H[4]) + fabs(B.H[7]), fabs(B.H[8])));
+  const double rl = sizeof(T) == 4 ? (a.cutoff + a.skin) * (1.0 + 1e-6) + 1.3e-6 * W : a.cutoff + a.skin;
   const T rl2 = T(rl * rl);
   int *out = a.cand + (size_t)i * a.cc;
   int count = 0;
@@ -402,7 +406,7 @@ __global__ void __launch_bounds__(256) k_cand(Dev<T> a) {
   // leaves of the radius (a quarter of the cube of cells that the index ranges span); cw: cell widths, fc: the
   // atom in its cell; reach: the radius with room for the rounding of these
   const bool rect = B.H[3] == 0.0 && B.H[6] == 0.0 && B.H[7] == 0.0;
-  const T reach2 = T((rl + 1e-4) * (rl + 1e-4));
+  const T reach2 = T((rl + 1e-4 + 1e-6 * W) * (rl + 1e-4 + 1e-6 * W));  // a place along an axis: 2.4e-7 W in FP32
   auto in_cell = [](T u, int n, int ci) {
     const T f = (u - floor(u)) * T(n) - T(ci);
     return f < T(-0.5) ? f + T(n) : f > T(1.5) ? f - T(n) : f;

@@ -455,6 +455,39 @@ def test_candidate_list_of_rectangular_boxes_is_complete(edges, prec):
         assert rms_rel(own.forces.cpu().numpy(), given.forces.cpu().numpy()) <= (1e-10 if prec == "double" else 1e-5)
 
 
+@pytest.mark.parametrize("edge", [4.0, 60.0, 1000.0])
+@pytest.mark.parametrize("skew", [0.0, 0.3])
+@pytest.mark.parametrize("prec", ["double", "mixed"])
+def test_candidate_list_of_large_boxes_is_complete(edge, skew, prec):
+    """Pairs a hair closer than cutoff + skin when the list is built, then moved together by a hair less than the
+    skin, so that the list must still hold every one: the same pairs as from the caller's rows of all other
+    atoms (the cutoff is tested in the engine either way), in boxes whose FP32 coordinates are good to 2e-7 to
+    6e-5 nm."""
+    from pgm_jax_b200.forcefield import MDSettings, PGMForceField
+    from pgm_jax_b200.systems import Molecule, System
+
+    rng = np.random.default_rng(31)
+    n, cutoff, skin = 400, 0.6, 0.1
+    H = np.diag([edge] * 3) + edge * np.array([[0, 0, 0], [skew, 0, 0], [-skew, skew, 0]])
+    u = rng.normal(size=(n, 3))
+    u /= np.linalg.norm(u, axis=1)[:, None]
+    a = rng.uniform(0, 1, size=(n, 3)) @ H
+    b = a + u * (cutoff + skin - rng.uniform(0, 2e-8 * edge, size=(n, 1)))
+    move = 0.5 * skin * (1 - 1e-9) * u
+    start, end = np.concatenate([a, b]), np.concatenate([a + move, b - move])
+    s = System([Molecule("X", ["O"], [q], [0.05], [1e-3]) for q in rng.normal(size=2 * n)])
+    st = MDSettings(precision=prec, elec="q", cutoff=cutoff, skin=skin, ewald_beta=6.0, pme_grid=(24, 24, 24))
+    own, given = (PGMForceField(s, H, st, row_capacity=128) for _ in range(2))
+    own.set_list_capacity(256)
+    own.compute(start, H)
+    built = own.list_rebuilds()
+    own.compute(end, H)
+    assert own.list_rebuilds() == built
+    others = (np.arange(2 * n)[:, None] + np.arange(1, 2 * n)) % (2 * n)
+    given.compute(end, H, others.astype(np.int32))
+    assert int(own._lib.pgm_row_pairs(own._h)) == int(given._lib.pgm_row_pairs(given._h))
+
+
 @pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
 @pytest.mark.parametrize("skew", [0.0, 0.3])
 @pytest.mark.parametrize("prec", ["double", "mixed"])
