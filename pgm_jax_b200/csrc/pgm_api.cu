@@ -167,6 +167,7 @@ struct Engine : EngineBase {
   long long rgrid = 0, cgrid = 0;
   std::vector<std::unique_ptr<FftGroup>> gx, gy, gz, gp;  // k3, k2, k1 passes; plane passes (k3 + k2)
   int nwblk = 0, nqblk = 0, ntblk = 0;
+  int nbig = 0;  // atoms of molecules with more than FEW partners each (k_influence)
   std::vector<int> natoms;
 
   DBuf<pgm::SysInfo> d_sys;
@@ -175,7 +176,7 @@ struct Engine : EngineBase {
   DBuf<pgm::EnergyAcc> d_eacc;
   DBuf<unsigned> d_status;
   DBuf<int4> wb, qb, tb;
-  DBuf<int> sysid, molid, molfirst, molend, mol_start, cov_start, cov_j, cov_i_flat, cov_j_flat;
+  DBuf<int> big, sysid, molid, molfirst, molend, mol_start, cov_start, cov_j, cov_i_flat, cov_j_flat;
   DBuf<T> q, radius, alpha, ialpha, rminh, seps;
   DBuf<pgm::c2<T>> ljp;
   DBuf<double> mass, cov_c, cov_c_flat, bmod;
@@ -314,7 +315,7 @@ struct Engine : EngineBase {
     set = *s;
     nsys = n;
     hsys.resize(n);
-    std::vector<int> h_sysid, h_molid, h_molfirst, h_molend, h_molstart, h_covstart, h_covj, h_covi_flat, h_covj_flat;
+    std::vector<int> h_big, h_sysid, h_molid, h_molfirst, h_molend, h_molstart, h_covstart, h_covj, h_covi_flat, h_covj_flat;
     std::vector<T> h_q, h_rad, h_al, h_ial, h_rh, h_se;
     std::vector<double> h_mass, h_covc, h_covc_flat, h_bmod;
     std::vector<pgm::c2<T>> h_tw;
@@ -397,6 +398,7 @@ struct Engine : EngineBase {
       S.sum_q = sq; S.sum_q2 = sq2;
       for (int m = 0; m < d.n_mol; ++m) {
         int a0 = d.mol_start[m], a1 = d.mol_start[m + 1];
+        for (int i = a0; i < a1 && a1 - a0 - 1 > pgm::FEW; ++i) h_big.push_back(atom0 + i);
         h_molstart.push_back(atom0 + a0);
         for (int i = a0; i < a1; ++i) {
           h_molid.push_back(mol0 + m);
@@ -547,7 +549,7 @@ struct Engine : EngineBase {
     d_cg.upload(hcg);
     d_eacc.alloc(n);
     d_status.alloc(n);
-    sysid.upload(h_sysid); molid.upload(h_molid); molfirst.upload(h_molfirst); molend.upload(h_molend);
+    big.upload(h_big); sysid.upload(h_sysid); molid.upload(h_molid); molfirst.upload(h_molfirst); molend.upload(h_molend);
     mol_start.upload(h_molstart); cov_start.upload(h_covstart); cov_j.upload(h_covj);
     cov_i_flat.upload(h_covi_flat); cov_j_flat.upload(h_covj_flat);
     q.upload(h_q); radius.upload(h_rad); alpha.upload(h_al); ialpha.upload(h_ial); rminh.upload(h_rh); seps.upload(h_se);
@@ -1043,8 +1045,9 @@ struct Engine : EngineBase {
     }
     launch_pdl(pgm::k_rows<T>, nwblk, 256, 0, st, a);
     if (nn_hist) nn_fork(st, a, nn_hist);
-    launch_pdl(pgm::k_influence<T>, (int)std::min<long long>(8 * nsm, std::max<long long>((cgrid + 255) / 256, grid1(2 * nt))), 256, 0, st, a,
-               (long long)cgrid);
+    const long long threads = std::max<long long>(cgrid, sizeof(T) == 4 ? 2ll * nt + 32ll * nbig : 1);
+    launch_pdl(pgm::k_influence<T>, (int)std::min<long long>(8 * nsm, (threads + 255) / 256), 256, 0, st, a, (long long)cgrid,
+               (const int *)big.p, nbig);
   }
 
   void set_list_capacity(int c) override {

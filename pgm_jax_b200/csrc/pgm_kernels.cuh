@@ -701,22 +701,32 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_rows(Dev<T> a) 
 // G(m) = exp(-pi^2 |m*|^2 / beta^2) / (2 pi V |m*|^2) / (b1 b2 b3), 0 at m = 0 (pme.py:243-267),
 // on the half spectrum, computed in FP64, stored in T; recomputed only when the box changed.
 // Two closing jobs of the row build ride in the launch: a rebuild of the candidate list is counted and its flag
-// lowered, and in mixed precision the molecule partners' kernels (two threads per atom) are evaluated again in
-// FP64 and rounded once.  Their pairs carry most of the energy at distances that a rigid molecule never changes,
-// so a rounding error of theirs is a bias: the energy of a water box at zero induced dipoles is 7.2 to 8.2e-8 off
-// with all kernels in FP32, 4.8 to 5.4e-8 with this.  Cost: 4 us at 12,288 atoms, none seen at 59,049; in
-// the row build, where a warp would run it for a few lanes, 12 us of 57 and 58 us of 230.
+// lowered, and in mixed precision the molecule partners' kernels are evaluated again in FP64 and rounded once.  Their
+// pairs carry most of the energy at distances that a rigid molecule never changes, so a rounding error of theirs is a
+// bias: the energy of a water box at zero induced dipoles is 7.2 to 8.2e-8 off with all kernels in FP32, 4.7 to 5.4e-8
+// with this, and 4.8e-8 is what the FP32 rounding of the charges and widths alone makes.  Cost: 4 us at 12,288
+// atoms of water, none seen at 59,049; in the row build, where a warp would run it for a few lanes, 12 us of 57 and
+// 58 us of 230.
+// An atom's partners go to two threads up to FEW of them (a water has two), to 32 threads above: an evaluation is
+// 0.5 us of dependent FP64 arithmetic.  A call at given dipoles on 1,536 atoms in molecules of 256: 221 us with two
+// threads for every atom, 155 so; one molecule of 201 atoms in 98,304 atoms of water: 924 with two, 980 with 32 for
+// every atom, 910 so.  big: the nbig atoms of molecules large enough for more than FEW.
+constexpr int FEW = 8;
 template <typename T>
-__global__ void k_influence(Dev<T> a, long long total) {
+__global__ void k_influence(Dev<T> a, long long total, const int *big, int nbig) {
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
   if (blockIdx.x == 0 && threadIdx.x == 0 && !a.idx && *a.nb_flag) { *a.nb_flag = 0; *a.nb_builds += 1; }
   if constexpr (sizeof(T) == 4) {
     using C = RowChunk<T>;
-    for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < 2 * a.nt; u += gridDim.x * blockDim.x) {
-      const int i = u >> 1, n = min(a.rnsp[i], a.mce);
+    const long long many = 32ll * nbig;
+    for (long long u = blockIdx.x * blockDim.x + threadIdx.x; u < many + 2ll * a.nt; u += gridDim.x * blockDim.x) {
+      const bool wide = u < many;
+      const int i = wide ? big[u >> 5] : (int)((u - many) >> 1), step = wide ? 32 : 2;
+      const int n = min(a.rnsp[i], a.mce);
+      if ((n > FEW) != wide) continue;  // the other part's
       unsigned char *row = row_of(a, i);
       const T Ri = a.radius[i];
-      for (int t = u & 1; t < n; t += 2) {
+      for (int t = (int)(wide ? u : u - many) & (step - 1); t < n; t += step) {
         unsigned char *c = row_entry<T>(row, t);
         const T Rk = a.radius[entry_k<T>(c, t)], x = entry_v<T, C::X>(c, t), y = entry_v<T, C::Y>(c, t), z = entry_v<T, C::Z>(c, t);
         double g[4];

@@ -555,6 +555,31 @@ def test_pair_kernels_over_their_ranges(prec, beta):
     assert np.abs(got - ref).max() <= tol * np.abs(ref).max(), np.abs(got - ref).max() / np.abs(ref).max()
 
 
+@pytest.mark.parametrize("size", [1, 8, 9, 10, 33, 70])
+@pytest.mark.parametrize("prec", ["double", "mixed"])
+def test_molecules_of_many_sizes(prec, size):
+    """One rigid molecule of `size` atoms (no partners, up to the partners that two threads share, one above, more
+    than a chunk of 32 and than two) among waters, in a box where some of its atoms are beyond the cutoff of
+    others: energy, forces and virial of charges and permanent dipoles against the oracle.  Tolerances as for the small
+    box."""
+    from pgm_jax_b200.systems import Molecule, System, pgm3p25_water, water_box
+
+    s, pos, H = water_box(5, 1.552, seed=8)
+    rng = np.random.default_rng(size)
+    q = rng.normal(scale=0.3, size=size)
+    big = Molecule("B", ["C"] * size, q, rng.uniform(0.05, 0.07, size), np.full(size, 1e-3), [], np.full(size, 0.15), np.full(size, 0.4))
+    first = 3 * -(-size // 3)  # the molecule takes the places of the first waters' atoms
+    sy = System([big] + [pgm3p25_water()] * ((s.n - first) // 3))
+    x = np.concatenate([pos[:size], pos[first:]])
+    kw = dict(cutoff=0.5, pme_grid=(30, 30, 30), elec="qp")
+    r = O.Oracle(sy, dict(SMALL_BOX_SETTINGS, **kw)).compute(x, H)
+    g = ff_for(sy, H, prec, **kw).compute(x, H)
+    e, f, w = (1e-9, 1e-8, 1e-7) if prec == "double" else (1e-6, 1e-5, 1e-4)
+    assert abs(float(g.energy["elec"][0]) - r["energy"]["elec"]) <= e * abs(r["energy"]["elec"])
+    assert rms_rel(g.forces.cpu().numpy(), r["forces"]) <= f
+    assert np.abs(g.virial[0].cpu().numpy() - r["virial"]).max() <= w * np.abs(r["virial"]).max()
+
+
 MESH_LENGTHS = [K for K in range(8, 257, 2) if 2**8 * 3**5 * 5**3 % K == 0]
 
 
