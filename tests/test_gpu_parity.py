@@ -602,6 +602,32 @@ def test_field_on_every_mesh_length(L, prec):
         assert np.abs(got - ref).max() <= tol * np.abs(ref).max(), (grid, np.abs(got - ref).max() / np.abs(ref).max())
 
 
+@pytest.mark.parametrize("L", MESH_LENGTHS)
+@pytest.mark.parametrize("prec", ["double", "mixed"])
+def test_energy_and_virial_on_every_mesh_length(L, prec):
+    """The energy form of the k1 pass (its block reductions, the weights of the half spectrum and the influence
+    part of the virial) for every mesh length along k1 and along k3, on charges and permanent dipoles,
+    against the oracle.  Tolerances as for the molecules of many sizes.  On the k1 Nyquist plane m1 has one sign in
+    the engine's half spectrum (as in the reference's rfft), while its products with m2 and m3 cancel in the oracle's
+    full one: the xy and xz elements are compared where that plane's exp(-(pi m1 / beta L)^2) is
+    below 2e-8 (lengths from 20)."""
+    from pgm_jax_b200.forcefield import MDSettings, PGMForceField
+    from pgm_jax_b200.systems import water_box
+
+    s, pos, H = water_box(4, 1.2416, seed=3)
+    e, f, w = (1e-9, 1e-8, 1e-7) if prec == "double" else (1e-6, 1e-5, 1e-4)
+    for grid in [(L, 24, 20), (20, 24, L)]:
+        st = dict(cutoff=0.6, ewald_beta=6.0, pme_grid=grid, pme_order=4, elec="qp")
+        r = O.Oracle(s, st).compute(pos, H)
+        g = PGMForceField(s, H, MDSettings(precision=prec, **st)).compute(pos, H)
+        assert abs(float(g.energy["elec"][0]) - r["energy"]["elec"]) <= e * abs(r["energy"]["elec"]), grid
+        assert rms_rel(g.forces.cpu().numpy(), r["forces"]) <= f, grid
+        dW = np.abs(g.virial[0].cpu().numpy() - r["virial"])
+        if grid[0] < 20:
+            dW[0, 1:] = dW[1:, 0] = 0.0
+        assert dW.max() <= w * np.abs(r["virial"]).max(), grid
+
+
 def test_water4096_frame_matches_oracle():
     """The 4,096-water benchmark frame (12,288 atoms, 4.966 nm box, PME 96^3, cutoff 0.9 nm,
     Ewald 4.0/nm) as a single point at tol 1e-8: the FP64 engine against the oracle (energy 1e-9,
