@@ -308,10 +308,4 @@ __device__ __forceinline__ void atomic_max_nonneg(unsigned long long *a, double 
   atomicMax(a, (unsigned long long)__double_as_longlong(v));
 }
 
-// Block of the batch -> (system, first atom of the block); blocks never straddle systems.
-struct BlockMap {
-  const int *sys;    // system of every block
-  const int *atom0;  // first atom (global) of every block
-};
-
 }  // namespace pgm

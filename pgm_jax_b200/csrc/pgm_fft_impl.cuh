@@ -408,8 +408,6 @@ __global__ void __launch_bounds__(YShape<T, N>::THREADS, min_blocks<T>(YShape<T,
   }
   if constexpr (ENERGY) {
     __shared__ double red[(Y::THREADS + 31) / 32][7];
-    const unsigned m = __activemask();
-    (void)m;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int LAST = Y::THREADS % 32;  // threads of a last, partial warp (0: none)
     const unsigned mask = (LAST && warp == Y::THREADS / 32) ? (1u << LAST) - 1u : 0xffffffffu;

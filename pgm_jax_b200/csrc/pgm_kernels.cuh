@@ -871,7 +871,7 @@ __global__ void __launch_bounds__(ATOMS_PER_BLOCK * QL) k_spread(Dev<T> a, const
   // the loads go out before the test of the system's flag
   const int4 b = a.base[i];
   const v4<T> f = a.frac[i];
-  const v4<T> z = UPDATE_P ? a.Z[i] : vin[i], p = a.P[i];
+  const v4<T> z = UPDATE_P ? a.Z[i] : vin[i], p = UPDATE_P ? a.P[i] : z;
   const Mesh M = mesh_of(a, s);
   if (!solve_active(a, s, ACT)) return;
   v4<T> d;
@@ -1146,9 +1146,8 @@ __global__ void __launch_bounds__(8 * LPA, 8 * 32 / LPA) k_nn_chan(Dev<T> a, con
   const int warp = threadIdx.x / LPA, lane = threadIdx.x % LPA;  // the atom's group of LPA lanes
   const unsigned gm = group_mask<LPA>();
   const Where at = where(a, a.wb, blockIdx.x, WARPS_PER_BLOCK, warp);
-  const int s = at.s, i = at.i;
+  const int i = at.i;
   if (i >= at.end) return;
-  const SysInfo &S = a.sys[s];
   (void)rg;  // the graph radius is a.nn_rg2 here
   float f0 = 0.f, f1 = 0.f, f2 = 0.f;
   const float2 *G = a.nn_g + (size_t)i * a.nn_emax;
@@ -1258,9 +1257,8 @@ __global__ void __launch_bounds__(256, 4) k_nn_features(Dev<T> a, const float *c
   int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (valid && blockIdx.x == 0 && threadIdx.x == 0) *valid = 1;  // read by the previous kernel only
   const Where at = where(a, a.wb, blockIdx.x, WARPS_PER_BLOCK, warp);
-  const int s = at.s, i = at.i;
+  const int i = at.i;
   if (i >= at.end) return;
-  const SysInfo &S = a.sys[s];
   float *V = vec + (size_t)i * pgmnn::NN_CH * 3;
   float *F = inv + (size_t)i * pgmnn::NN_IN;
   const float is = 1.f / sigma, is2 = is * is;
@@ -1298,21 +1296,6 @@ __global__ void __launch_bounds__(256, 4) k_nn_features(Dev<T> a, const float *c
     }
   }
   if (slot >= 0) F[slot] = ash ? asinhf(arg) : arg;
-}
-
-template <typename T>
-__global__ void k_copy_vec(int n, const v4<T> *src, v4<T> *dst) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dst[i] = src[i];
-}
-
-template <typename T>
-__global__ void k_vec_from_f64(int n, const double *src, v4<T> *dst) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  v4<T> d;
-  d.x = T(src[3 * i]); d.y = T(src[3 * i + 1]); d.z = T(src[3 * i + 2]); d.w = T(0);
-  dst[i] = d;
 }
 
 // ------------------------------------------------------------------ CG
