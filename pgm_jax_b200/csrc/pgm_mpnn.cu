@@ -348,16 +348,22 @@ __global__ void __launch_bounds__(32 * AGG_WARPS, 4) k_aggregate(const __nv_bflo
   cp_async_wait<0>();
 }
 
+// Multiprocessors of the current device.
+inline int sm_count() {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return std::max(1, sms);
+}
+
 // Grid of the edge-sum kernels: enough warps for every SM to hold its share at full occupancy,
 // each warp walking atoms at the grid's stride.
 inline int agg_blocks(int n) {
   static int resident = 0;  // blocks of k_aggregate that fit on the device at once
   if (!resident) {
-    int dev = 0, sms = 0, per = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int per = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_aggregate, 32 * AGG_WARPS, 0);
-    resident = std::max(1, sms) * std::max(1, per);
+    resident = sm_count() * std::max(1, per);
   }
   return std::max(1, std::min((n + AGG_WARPS - 1) / AGG_WARPS, resident));
 }
@@ -394,12 +400,11 @@ __global__ void __launch_bounds__(256) k_aggregate_t(const float *__restrict__ d
   }
 }
 
-// The filter weights' gradient: dWf[f, r] += sum_i da_i[f] s_i[r, f] (da: columns 64..79 of dZ);
-// thread r F + f of a 128-thread block, atoms in a grid-stride loop, one atomic add per block.
-// Four groups of R F threads take rows in turn, eight rows a time in flight, and the block adds its sum once:
-// 148 atomics per weight instead of 1184 (62 us of 505 in a training step at 12,288 atoms went into the
-// two launches; they were serial at the weights' addresses).
-constexpr int WF_GROUPS = 4, WF_BLOCKS = 148;
+// The filter weights' gradient: dWf[f, r] += sum_i da_i[f] s_i[r, f] (da: columns 64..79 of dZ); thread r F + f of
+// four groups of R F threads, which take rows in turn, eight rows a time in flight, and the block adds its sum once.
+// One block per multiprocessor: 148 atomics per weight (with 128-thread blocks and 1184 of them, 62 us of 505 in a
+// training step at 12,288 atoms went into the two launches; the adds were serial at the weights' addresses).
+constexpr int WF_GROUPS = 4;
 __global__ void __launch_bounds__(R * F * WF_GROUPS) k_wf_grad(const float *__restrict__ dZ, int ldd, const float *__restrict__ S, int n,
                                                                float *__restrict__ dWf) {
   __shared__ float part[WF_GROUPS][R * F];
@@ -498,8 +503,9 @@ __global__ void k_to_bf16(const float *__restrict__ x, int total, __nv_bfloat16 
 // Weight gradients on the CUDA cores: dW[o, k] += sum_m dY[m, o] X[m, k] (X BF16, the first K of
 // rows of ldx), db[o] += sum_m dY[m, o]; rows in chunks of 32 staged in shared memory, FP32 sums
 // per thread, one atomic add per output and block.
-// A thread keeps a TO x TK tile of dW in registers (one shared load per three to four products, where one output
-// at a time took two loads a product), and the next 32 rows load while the current ones are multiplied.
+// A thread keeps a TO x TK tile of dW in registers, and the next 32 rows load while the current ones are multiplied:
+// 4 x 4 and 4 x 5 outputs (64 x 64, 64 x 80) take at most 8 and 9 shared loads for 16 and 20 products, 2 x 2
+// (16 x 64, 64 x 16) 4 for 4, where one output at a time took two loads a product.
 template <int NO, int KI>
 __global__ void __launch_bounds__(256) k_wgrad(const float *__restrict__ dY, int ldy, const __nv_bfloat16 *__restrict__ X, int ldx,
                                                int M, float *__restrict__ dW, float *__restrict__ db) {
@@ -948,7 +954,7 @@ cudaError_t backward(const float *flat, Work &w, const float *inv, const float *
   View v = view(flat);
   GView g = gview(grad);
   WB b = wb_view(w.wb);
-  const int wgb = std::min(blocks(n, 64), 148);  // two chunks of rows a block and more: a block ends with an atomic per weight
+  const int sms = sm_count(), wgb = std::min(blocks(n, 64), sms);  // two chunks of rows a block and more: a block ends with an atomic per weight
   k_loss<<<blocks(n), 256, 0, st>>>(w.Cc, vec, target, n, sigma, scale, loss, w.dC, w.dCb);
   k_wgrad<COEF, HID><<<wgb, 256, 0, st>>>(w.dC, COEF, w.HZ[2], ZW, n, g.Wo, g.bo);
   MPCK((gemm<COEF, HID, ACT_NONE, float>(w.dCb, COEF, n, b.WoT, nullptr, w.dh, HID, w.err, st)));
@@ -960,7 +966,7 @@ cudaError_t backward(const float *flat, Work &w, const float *inv, const float *
     k_dsilu<<<blocks((long long)n * HID), 256, 0, st>>>(w.dU, w.zu[l], n * HID, w.dzu, w.dzub);
     k_wgrad<HID, ZW><<<wgb, 256, 0, st>>>(w.dzu, HID, w.HZ[l], ZW, n, g.Wa[l], g.ba[l]);
     MPCK((gemm<HID, ZW, ACT_NONE, float>(w.dzub, HID, n, b.WaT[l], nullptr, w.dZ, ZW, w.err, st)));
-    k_wf_grad<<<std::min(n, WF_BLOCKS), R * F * WF_GROUPS, 0, st>>>(w.dZ, ZW, w.Sk[l], n, g.Wf[l]);
+    k_wf_grad<<<std::min(n, sms), R * F * WF_GROUPS, 0, st>>>(w.dZ, ZW, w.Sk[l], n, g.Wf[l]);
     k_aggregate_t<<<blocks((long long)n * 32), 256, 0, st>>>(w.dZ, ZW, edges, ecount, emax, n, rg, v.Wf[l], w.dG, w.dGb);
     k_wgrad<F, HID><<<wgb, 256, 0, st>>>(w.dG, F, w.HZ[l], ZW, n, g.Wg[l], nullptr);
     MPCK((gemm<F, HID, ACT_NONE, float>(w.dGb, F, n, b.WgT[l], nullptr, w.dGh, HID, w.err, st)));
