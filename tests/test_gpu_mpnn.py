@@ -66,6 +66,34 @@ def test_mpnn_forward_and_gradient_match_numpy():
     assert np.linalg.norm(g - g_ex) <= 8e-2 * np.linalg.norm(g_ex)  # BF16 is the only approximation
 
 
+@pytest.mark.parametrize("n", [14, 32, 33, 64, 65, 4737, 9500])
+def test_weight_gradients_at_the_edges_of_their_blocks(n):
+    """Every weight's gradient with fewer rows than a chunk of 32, whole chunks and one row more, one row more
+    than a pass of the filter gradient's blocks, and several chunks per block, against the NumPy restatement.  As a whole
+    within the tolerance of the test above, each layer within half of what all roundings together are allowed there."""
+    from pgm_jax_b200.learned import GRAPH_CUTOFF, MPNN_SHAPES, SIGMA, MPNNModel
+
+    rng = np.random.default_rng(n)
+    edges, counts, src, dst, dist = _graph(n, 6, rng)
+    w = rng.normal(scale=0.15, size=N.mpnn_nparam()).astype(np.float32)
+    inv = rng.normal(size=(n, N.N_IN)).astype(np.float32)
+    vec = rng.normal(scale=0.02, size=(n, N.N_CH, 3)).astype(np.float32)
+    tgt = rng.normal(scale=2e-4, size=(n, 3)).astype(np.float32)
+    t = lambda a: torch.tensor(a, device="cuda")  # noqa: E731
+    m = MPNNModel(w)
+    scale = 1.0 / (n * SIGMA**2)
+    m.loss_grad({"inv": t(inv), "vec": t(vec), "target": t(tgt), "edges": t(edges), "counts": t(counts)}, scale)
+    g = m.g.cpu().numpy()
+    _, ref = N.mpnn_loss_grad(w, inv, vec, src, dst, N.radial(dist, GRAPH_CUTOFF), tgt, SIGMA, scale)
+    assert np.linalg.norm(g - ref) <= 1e-2 * np.linalg.norm(ref)
+    at = 0
+    for shape in MPNN_SHAPES:
+        k = int(np.prod(shape))
+        assert np.linalg.norm(g[at:at + k] - ref[at:at + k]) <= 4e-2 * np.linalg.norm(ref[at:at + k]), shape
+        at += k
+    assert at == len(g)
+
+
 def test_trained_mpnn_saves_iterations_over_mu4_and_mu1():
     """Plain-solver MD writes frames (features, graph, mu* - mu4 guess); GPU Adam steps on the
     project's forward and backward kernels train the message-passing model; on held-out frames its
