@@ -2294,7 +2294,9 @@ __global__ void __launch_bounds__(ATOMS_PER_BLOCK * QL, MINB) k_forces(Dev<T> a,
       T didk = di.x * dk.x + di.y * dk.y + di.z * dk.z;
       const T qq = qi * qk, pp = dix * dkx;
       const T tt = qi * dkx - qk * dix;
-      ee += qq * G0 + tt * G1 - G2 * pp + G1 * didk;
+      // not qq G0: the rounding of a charge product is the same for every pair of its kind, a bias (2.2e-8 of a water
+      // box's energy in FP32)
+      ee += qi * (qk * G0) + tt * G1 - G2 * pp + G1 * didk;
       const T radial = -qq * G1 - tt * G2 + G3 * pp - G2 * didk;
       // the gradient is radial x + u1 dk - u2 di, the field of (q_k, d_k) G1 dk - u2 x
       const T u1 = qi * G1 - G2 * dix, u2 = qk * G1 + G2 * dkx;
