@@ -9,8 +9,10 @@
 // directions with two exchanges.  The inverse transform is the forward one on swapped real and
 // imaginary parts.
 //
-// What bounds a pass: the meshes sit in L2 and a pass reads and writes them once, so it is latency:
-// loads in flight per SM, and the barriers between phases.  A staged shared-memory Stockham plan
+// What bounds a pass: the meshes sit in L2 and a pass reads and writes them once.  By the counters: the plane passes
+// (96^3) by their barriers and by having 96 CTAs for 148 SMs, issue 30 % of the slots; at 192^3 the k3 passes by L1
+// throughput (71 to 75 %), the k2 and k1 passes by load latency and barriers (issue 42 to 50 %).  A staged
+// shared-memory Stockham plan
 // (radix 8, 4, 2, 3, 5; one barrier and one shared round trip per radix) had 4 to 6 barriers a line.
 // Chains of a convolution, FP32, that plan -> this: 192^3 122 -> 73 us, 96^3 20.3 -> 15.6; a length that the plan
 // had at run time only, 108^3: 68 -> 20.

@@ -150,8 +150,9 @@ __device__ __forceinline__ void step1(c2<T> (&v)[n1_of(N)], int n2, const c2<T> 
 
 template <int N>
 constexpr int N1R = n1_of(N) > 18 ? 96 : 64;  // registers asked for (FP32)
-// Blocks per SM that the compiler leaves registers for: FP32 64 a thread (k2, k3 passes) or 80 (the
-// convolution), FP64 twice that, where the transform's points fit.
+// Blocks per SM that the compiler leaves registers for: FP32 64 a thread (k2, k3 passes), 80 (the convolution) or
+// 96 (its energy form), 96 to 128 where N1 > 18, FP64 twice that.  Not every transform fits: 192 spills 76 bytes in the
+// convolution, 128 180, 256 356 (136 in the k2 pass), most lengths below 144 none.
 template <typename T>
 constexpr int min_blocks(int threads, int regs32) {
   const int b = 65536 / (threads * (sizeof(T) == 4 ? regs32 : 2 * regs32));

@@ -478,9 +478,10 @@ __global__ void __launch_bounds__(256) k_cand(Dev<T> a) {
 // the warp in shared memory; whenever 32 are waiting the warp evaluates their radial kernels
 // (pair_kernels), every lane busy, and writes k, x, y, z, G0..G3 with them, contiguous over the lanes,
 // and the local preconditioner's short entries and the learned guess's graph edges.
-// Bound by the latency of the candidates' gathers and by issue: the scan alone takes 137 of 232 us at 59,049
-// atoms (FP32; 305 with rows in eight arrays and a round that waited for its loads; 378 of 494 at 98,304, 57 of
-// 78 at 12,288; FP64 127 of 147).  3 or 5 blocks per SM are slower (309, 296 against 272 at the time).
+// Bound by issue (77 % of the slots at 12,288 atoms; DRAM 20 %, L1 52 %, a warp waits for a load 1.2 of its 9.0 cycles
+// an instruction): the scan alone takes 137 of 232 us at 59,049 atoms (FP32; 305 with rows in eight arrays and a
+// round that waited for its loads; 378 of 494 at 98,304, 57 of 78 at 12,288; FP64 127 of 147).  3 or 5 blocks per SM
+// are slower (309, 296 against 272 at the time); four leave 64 registers, 64 bytes of spills.
 
 // An atom's group of LPA lanes (32: the warp; 16, 8: a half, a quarter warp): its shuffle mask, and the sum over
 // it (the warp's own reduction for a whole warp).
@@ -703,10 +704,10 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_rows(Dev<T> a) 
 // Two closing jobs of the row build ride in the launch: a rebuild of the candidate list is counted and its flag
 // lowered, and in mixed precision the molecule partners' kernels are evaluated again in FP64 and rounded once.  Their
 // pairs carry most of the energy at distances that a rigid molecule never changes, so a rounding error of theirs is a
-// bias: the energy of a water box at zero induced dipoles is 7.2 to 8.2e-8 off with all kernels in FP32, 4.7 to 5.4e-8
-// with this, and 4.8e-8 is what the FP32 rounding of the charges and widths alone makes.  Cost: 4 us at 12,288
-// atoms of water, none seen at 59,049; in the row build, where a warp would run it for a few lanes, 12 us of 57 and
-// 58 us of 230.
+// bias: the energy of a water box at zero induced dipoles was 7.2 to 8.2e-8 off with all kernels in FP32, 4.9e-8 with
+// this (3.1e-8 now, without the rounded charge products of the force pass; 2.6e-8 is the rounding of the parameters
+// to FP32).  Cost: 4 us at 12,288 atoms of water, none seen at 59,049; in the row build, where a warp would run it
+// for a few lanes, 12 us of 57 and 58 us of 230.
 // An atom's partners go to two threads up to FEW of them (a water has two), to 32 threads above: an evaluation is
 // 0.5 us of dependent FP64 arithmetic.  A call at given dipoles on 1,536 atoms in molecules of 256: 221 us with two
 // threads for every atom, 155 so; one molecule of 201 atoms in 98,304 atoms of water: 924 with two, 980 with 32 for
@@ -771,10 +772,11 @@ __global__ void k_influence(Dev<T> a, long long total, const int *big, int nbig)
 // The PME kernels give an atom QL = 8 lanes (four atoms per warp, 32 per block).  The P x P stencil rows along
 // k3 are taken SLOTS at a time, a row's points as GPL aligned vectors of VW (16 bytes where K3 allows it, else
 // two points), one lane each: the vectors of a row sit side by side, so a warp's request touches 16 rows in whole
-// sectors, and a lane's k3 weights stay in registers for all rows.  What bounds them is latency and the L1's line
-// rate: with one point or vector per lane and the k3 weights read from shared memory for every
-// point, a row cost three times the instructions.  At 98,304 atoms, 192^3: gather 59.5 -> 37.0 us, spread
-// 43.2 -> 38.9; at 59,049 atoms 31.0 -> 22.6 and 25.5 -> 24.7 (the spread keeps its vector atomics, which L2 bounds).
+// sectors, and a lane's k3 weights stay in registers for all rows.  What bounds them is load latency (8 of a gather's 14
+// cycles an instruction, 6 of a spread's 14, at 30 % of the warps) and then L1 (44 and 55 %): with one point or vector
+// per lane and the k3 weights read from shared memory for every point, a row cost three times the instructions.
+// At 98,304 atoms, 192^3: gather 59.5 -> 37.0 us, spread 43.2 -> 38.9; at 59,049 atoms 31.0 -> 22.6 and 25.5 -> 24.7
+// (the spread keeps its vector atomics; L2 takes them in 20 % of its cycles).
 constexpr int QL = 8, ATOMS_PER_BLOCK = 32;
 template <typename T, int VW> struct VecOf;
 template <> struct VecOf<float, 4> { using type = float4; };
@@ -2162,7 +2164,8 @@ __global__ void k_iel_finish(Dev<T> a, double *mu, double *hist, double *xl, Iel
 // atoms with the block preconditioner, the i-side delta scaled by a.iel_keep = 1 - 1/omega); their
 // position gradients at fixed delta go to the forces, not to the virial (the fixed-mu strain
 // derivative); the sums of |delta|^2 and |delta|^2 / (2 alpha) go to the energy accumulators.
-// Bound by the row stream (40 bytes a pair) and the partners' gathers.  The stencil comes first and its sums wait in
+// Bound by the latency of the row stream (40 bytes a pair) and of the partners' gathers (7 of 12 cycles an instruction;
+// DRAM 31 %, L1 52 %, issue 42 %, at 12,288 atoms and four blocks per SM).  The stencil comes first and its sums wait in
 // shared memory, so that registers serve one part at a time: 303 -> 238 us at 98,304 atoms, 197 -> 157 at 59,049.
 template <typename T, int P, int MINB = 3, bool SHADOW = false>
 __global__ void __launch_bounds__(ATOMS_PER_BLOCK * QL, MINB) k_forces(Dev<T> a, const double *mu) {

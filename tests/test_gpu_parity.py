@@ -55,8 +55,8 @@ def test_field_of_charges_and_dipoles(box, prec):
 @pytest.mark.parametrize("prec", ["double", "mixed"])
 def test_field_through_every_fft_route(box, grid, prec):
     """The field sweep on meshes that take each route of the reciprocal-space chain: the plane
-    passes (K2 = K3 with a compiled plan: 32^3 and 36 x 48^2), separate k3 and k2 passes with compiled
-    plans (32 x 32 x 48), and the runtime-length passes (30 x 36 x 32), against the oracle.  The
+    passes (K2 = K3: 32^3 and 36 x 48^2) and separate k3 and k2 passes (32 x 32 x 48, 30 x 36 x 32),
+    against the oracle.  The
     oracle transforms the full spectrum, the engine (as pme.py:370-376) the rfft half: on this
     triclinic box the influence function is not mirror-symmetric on the Nyquist planes, which
     separates the two by up to ~2e-10 of the field on the coarse 30 x 36 x 32 mesh (white-noise

@@ -1,7 +1,7 @@
 """The autotuner's kernel variants (GPU): every choice of lanes per row in the CG matvec's row
 stream, of blocks per SM in the force pass, of the order of the CG sweep's concurrent parts (the
 row field of p, or of z combined with the previous direction's) and of the row field's grid beside
-the FFT chain (all SMs, or 1 or 2 blocks per SM at the highest priority) computes the same step (FP64: only
+the FFT chain (all SMs, or 4 or 8 blocks per SM at the highest priority) computes the same step (FP64: only
 the order of additions changes), and the first direct step of a handle times them and keeps the
 fastest."""
 
