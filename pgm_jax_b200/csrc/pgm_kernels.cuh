@@ -389,9 +389,10 @@ __global__ void __launch_bounds__(256) k_cand(Dev<T> a) {
   else pi = a.pos4[i];
   // W: the largest coordinate of a wrapped position.  A displacement of two of them in FP32 is off by less than
   // 12 W 2^-24 a component (both positions, three lattice vectors and the subtractions), 1.3e-6 W in length; the
-  // square's rounding is below 1e-6 of it.
+  // square's rounding is below 1e-6 of it.  At most a tenth of the radius: above 8e4 nm FP32 positions resolve less
+  // than that, and the list must not outgrow its capacity for them.
   const double W = fmax(fabs(B.H[0]) + fabs(B.H[3]) + fabs(B.H[6]), fmax(fabs(B.H[4]) + fabs(B.H[7]), fabs(B.H[8])));
-  const double rl = sizeof(T) == 4 ? (a.cutoff + a.skin) * (1.0 + 1e-6) + 1.3e-6 * W : a.cutoff + a.skin;
+  const double r0 = a.cutoff + a.skin, rl = sizeof(T) == 4 ? r0 * (1.0 + 1e-6) + fmin(1.3e-6 * W, 0.1 * r0) : r0;
   const T rl2 = T(rl * rl);
   int *out = a.cand + (size_t)i * a.cc;
   int count = 0;
