@@ -2167,7 +2167,7 @@ __global__ void k_iel_finish(Dev<T> a, double *mu, double *hist, double *xl, Iel
 // derivative); the sums of |delta|^2 and |delta|^2 / (2 alpha) go to the energy accumulators.
 // Bound by the latency of the row stream (40 bytes a pair) and of the partners' gathers (7 of 12 cycles an instruction;
 // DRAM 31 %, L1 52 %, issue 42 %, at 12,288 atoms and four blocks per SM).  The stencil comes first and its sums wait in
-// shared memory, so that registers serve one part at a time: 303 -> 238 us at 98,304 atoms, 197 -> 157 at 59,049.
+// shared memory, so that registers serve one part at a time: 303 -> 257 us at 98,304 atoms, 198 -> 169 at 59,049.
 template <typename T, int P, int MINB = 3, bool SHADOW = false>
 __global__ void __launch_bounds__(ATOMS_PER_BLOCK * QL, MINB) k_forces(Dev<T> a, const double *mu) {
   pdl_enter();  // launched as a programmatic dependent of the previous kernel
